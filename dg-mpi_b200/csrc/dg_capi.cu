@@ -16,6 +16,7 @@
 #include "../host/case.h"
 #include "../host/partition.h"
 #include "dg_ctx.cuh"
+#include "dg_column.cuh"
 #include "dg_tc.cuh"
 
 using dgk::GeoDev;
@@ -171,6 +172,7 @@ void stage_args(const dg_ctx* c, int mode, const double* Us, const double* U0, d
     a.geo_class = c->d_geo_class;
     a.geo = c->d_geo;
     a.cmap = c->d_cmap;
+    a.cmapn = c->d_cmapn;
     a.gjd = c->d_gjd;
     a.gnrm = c->d_gnrm;
     a.gimm = c->d_gimm;
@@ -192,6 +194,14 @@ void stage_args(const dg_ctx* c, int mode, const double* Us, const double* U0, d
     dgk::stage_variants(c->p, &vs);
     // the tensor-core kernel bulk-copies each face's fluxes: a 16-byte multiple per face
     if (vs[c->variant].flags & dgk::kTC) a.fstride = dgk::tc_face_stride(c->p);
+    if (vs[c->variant].flags & dgk::kCF) {
+        // the face kernel stores lifted fluxes; the residual output takes the plain tables
+        a.fstride = 5 * (c->p + 1) * (c->p + 1);
+        if (mode == dgk::kModeResidual) {
+            std::memcpy(a.tab.MB, a.tab.B, sizeof(a.tab.MB));
+            std::memcpy(a.tab.MD, a.tab.D, sizeof(a.tab.MD));
+        }
+    }
 }
 
 int launch_stage(dg_ctx* c, int mode, const double* Us, const double* U0, double* out, double dt, int e_begin, int e_end)
@@ -919,6 +929,19 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
     for (size_t i = 0; i < c->tab.B.size(); ++i) c->stage_tab.Bf[i] = static_cast<float>(c->tab.B[i]);
     for (size_t i = 0; i < c->tab.D.size(); ++i) c->stage_tab.Df[i] = static_cast<float>(c->tab.D[i]);
     for (size_t i = 0; i < c->tab.wq.size(); ++i) c->stage_tab.Wf[i] = static_cast<float>(c->tab.wq[i]);
+    {   // the 1D inverse mass folded into the contraction tables: MB[q][b] = sum_k B[q][k] Minv[b][k]
+        const int n = c->p + 1;
+        for (int q = 0; q < c->p + 2; ++q)
+            for (int b = 0; b < n; ++b) {
+                long double sb = 0.0L, sd = 0.0L;
+                for (int k = 0; k < n; ++k) {
+                    sb += static_cast<long double>(c->tab.B[q * n + k]) * c->tab.Minv[b * n + k];
+                    sd += static_cast<long double>(c->tab.D[q * n + k]) * c->tab.Minv[b * n + k];
+                }
+                c->stage_tab.MB[q * n + b] = static_cast<double>(sb);
+                c->stage_tab.MD[q * n + b] = static_cast<double>(sd);
+            }
+    }
     {   // nodal derivative of the 1D basis: Dn[i*n + j] = l_j'(xi_i) at the equidistant nodes
         const int n = c->p + 1;
         const std::vector<double> xn = dgh::equidistant_nodes(n);
@@ -1021,7 +1044,7 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
         {(void**)&c->d_frec, static_cast<size_t>(std::max(1, c->ne)) * 6 * sizeof(dgk::FaceRec)},
         {(void**)&c->d_geo_class, static_cast<size_t>(c->ne_alloc) * sizeof(int)},
         {(void**)&c->d_geo, ncls * (sizeof(GeoDev) + 9 * sizeof(double))},
-        {(void**)&c->d_cmap, std::max<size_t>(1, c->pm.cmap.size())},
+        {(void**)&c->d_cmap, std::max<size_t>(1, c->pm.cmap.size() + c->pm.cmapn.size())},
         {(void**)&c->d_X0, static_cast<size_t>(c->ne_alloc) * 3 * sizeof(double)},
         {(void**)&c->d_halo_send, std::max<size_t>(1, c->nslices) * sizeof(int2)},
         {(void**)&c->d_halo_recv, std::max<size_t>(1, c->nslices) * sizeof(int2)},
@@ -1040,6 +1063,10 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
             return bail(DG_ERR_NOMEM);
         }
     }
+    // the face-point permutations, then the face-node ones
+    c->d_cmapn = c->d_cmap + c->pm.cmap.size();
+    std::vector<uint8_t> cmaps(c->pm.cmap);
+    cmaps.insert(cmaps.end(), c->pm.cmapn.begin(), c->pm.cmapn.end());
     std::vector<int2> conn(static_cast<size_t>(c->ne_alloc) * 6);
     for (size_t i = 0; i < conn.size(); ++i) conn[i] = make_int2(c->pm.conn[i * 2], c->pm.conn[i * 2 + 1]);
     // the face records of the owned elements (see dgk::FaceRec)
@@ -1142,7 +1169,7 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
         }
         // the default variant again, now that face-kernel variants may match
         for (int v = 0; v < nv; ++v)
-            if (variant_matches(c, v)) {
+            if (variant_matches(c, v) && c->ne >= vs[v].min_per_sm * dev_sms) {
                 c->variant = v;
                 break;
             }
@@ -1158,7 +1185,7 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
               cudaMemcpy(c->d_halo_send, hs.data(), hs.size() * sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(c->d_halo_recv, hr.data(), hr.size() * sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(c->d_X0, c->pm.X0.data(), c->pm.X0.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&
-              (c->pm.cmap.empty() || cudaMemcpy(c->d_cmap, c->pm.cmap.data(), c->pm.cmap.size(), cudaMemcpyHostToDevice) == cudaSuccess) &&
+              (cmaps.empty() || cudaMemcpy(c->d_cmap, cmaps.data(), cmaps.size(), cudaMemcpyHostToDevice) == cudaSuccess) &&
               (!c->pm.general ||
                (cudaMemcpy(c->d_gjd, c->pm.gjd.data(), c->pm.gjd.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&
                 cudaMemcpy(c->d_gnrm, gnrm.data(), gnrm.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&

@@ -1,0 +1,701 @@
+// dg_column.cuh -- the column form of the DG stage (affine elements, orders 1..5):
+// face_lift_kernel and column_kernel, one launch each per RK stage.
+//
+// Same scheme as dg_stage.cuh's face kernel and stage kernel, with the work cut
+// so that little of it goes through shared memory:
+//
+//   face_lift_kernel  every interior face's numerical flux once, and its 2D
+//       lift once: [face][5][(p+1)^2] lifted values in the listed side's order
+//       (the other side reads them through the face-node permutation, which
+//       commutes with the lift: nodes and points are symmetric on the face).
+//   column_kernel     per batch of E elements: x and y interpolation through
+//       shared memory, then one thread per (x, y) quadrature column does the z
+//       interpolation, the Euler flux and the z contraction in registers
+//       (holding the p+2 point states and contravariant velocities of its
+//       column, variable by variable for the accumulators), then the y
+//       contraction, and the x contraction fused with the face lifts and the
+//       stage update.  A row of p+1 coefficients along x is one task's from
+//       global memory to global memory, so the state, the step-start state and
+//       the accumulator go straight between global memory and registers, the
+//       next batch's prefetched into L2.
+//
+// FP64: the 1D inverse mass matrix is folded into the contraction tables
+// (MB = B Minv, MD = D Minv per direction) and a face's lift is spread along its
+// normal by the inverse mass's end columns, so no separate inverse-mass passes
+// run.  The FP32 residual keeps its FP64 inverse mass as three passes after the
+// contraction and the stage kernel's FP32 operations in their order (the same
+// bits on meshes whose face orders agree).
+//
+// Why: the stage kernel writes and reads every intermediate through shared
+// memory between up to nine block barriers per element, and waits on them
+// (40^3, p = 3, FP64: 5140 warp instructions and 1640 shared wavefronts per
+// element, FP64 pipe 40 %, `barrier` the first stall).  Here a warp owns its
+// elements (no block barriers up to p = 3), 2610 instructions per element, the
+// column phase keeping 27 of the point array's 45 words in registers.  RK stage
+// (both kernels), stage kernel -> column form, GDOF/s: FP64 11.7 -> 20.5 (72^3,
+// p = 1), 24.5 -> 31.5 (60^3, p = 2), 31.9 -> 38.5 (48^3, p = 3), 30.2 -> 37.3
+// (40^3, p = 4), 31.9 -> 37.7 (32^3, p = 5); mixed 19.4 -> 26.3, 33.0 -> 37.7,
+// 39.7 -> 42.2, 44.0 -> 45.9, 41.8 -> 43.7.
+#pragma once
+#include "dg_stage.cuh"
+
+namespace dgk {
+
+// launch option: the column form (needs the face kernel's fluxes lifted)
+constexpr int kCF = 8192;
+
+// Shared-memory layout of a batch element.  The point array has 15 rows (v, d)
+// of [bz][qy][qx] with plane stride PS and row stride AS; the x-interpolated
+// block [v][bz][by][qx] (stride X1S) sits in its rows 5.. .  Strides and task
+// orders (see TaskOrd for their coding) minimise the wavefronts of the passes'
+// addresses (FP64 served per half-warp on 16 bank pairs, FP32 per warp on 32).
+template <int P, typename T>
+struct ColLay {
+    static constexpr bool W8 = sizeof(T) == 8;
+    static constexpr int N = P + 1, M = P + 2, NB = N * N * N, NF = M * M, N2 = N * N;
+    static constexpr int PS = NF + (W8 ? (P == 1 ? 6 : P == 2 ? 4 : P == 3 ? 3 : P == 4 ? 5 : 6)
+                                       : (P == 1 ? 6 : P == 2 ? 5 : P == 3 ? 0 : P == 4 ? 5 : 0));
+    static constexpr int AS = W8 ? (P == 1 ? 33 : P == 2 ? 63 : P == 3 ? 111 : P == 4 ? 207 : 335)
+                                 : (P == 1 ? 31 : P == 2 ? 74 : P == 3 ? 119 : P == 4 ? 207 : 301);
+    static constexpr int X1S = N * N * M + (W8 ? (P == 2 || P == 3 ? 1 : 0) : (P == 2 ? 1 : P == 4 ? 3 : 0));
+    // (v, qx, bz) orders of the y interpolation and the y contraction
+    static constexpr int oy = W8 ? (P == 1 ? 21 : P == 2 ? 7 : P == 3 ? 11 : P == 4 ? 19 : 7)
+                                 : (P == 1 ? 21 : P == 2 ? 21 : P == 3 ? 7 : P == 4 ? 11 : 19);
+    static constexpr int oyc = W8 ? (P == 3 || P == 4 ? 11 : 21) : (P == 1 ? 21 : P == 2 ? 15 : P == 4 ? 11 : 19);
+    static_assert(PS >= NF && AS >= (N - 1) * PS + NF && 10 * AS >= 5 * X1S, "point-array rows overlap");
+    static constexpr int W = 15 * AS;                     // point array, T
+    static constexpr int VS = odd(NB);                    // FP32 path: residual block stride, FP64
+    static constexpr int RES = W8 ? 0 : 5 * VS;           // FP64 residual of the FP32 path
+    static constexpr int LF = 30 * N2;                    // the six faces' lifts, T
+    static constexpr size_t f64_words(int E) { return static_cast<size_t>(E) * RES + 2 * N; }
+    static constexpr size_t t_words(int E) { return static_cast<size_t>(E) * (W + LF + 6); }
+    static constexpr size_t bytes(int E) { return f64_words(E) * 8 + t_words(E) * sizeof(T) + E * sizeof(int); }
+};
+
+template <int NT>
+__device__ __forceinline__ void cta_sync()
+{
+    if constexpr (NT == 32) __syncwarp();
+    else __syncthreads();
+}
+
+// a row of N consecutive doubles (16-byte aligned when N is even)
+template <int N>
+__device__ __forceinline__ void load_row(const double* p, double (&x)[N])
+{
+    if constexpr (N % 2 == 0) {
+#pragma unroll
+        for (int k = 0; k < N; k += 2) {
+            const double2 t = *reinterpret_cast<const double2*>(p + k);
+            x[k] = t.x;
+            x[k + 1] = t.y;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; ++k) x[k] = p[k];
+    }
+}
+template <int N>
+__device__ __forceinline__ void store_row(double* p, const double (&x)[N])
+{
+    if constexpr (N % 2 == 0) {
+#pragma unroll
+        for (int k = 0; k < N; k += 2) *reinterpret_cast<double2*>(p + k) = make_double2(x[k], x[k + 1]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; ++k) p[k] = x[k];
+    }
+}
+
+// starts fetching n doubles at p into L2 (whole 16-byte pieces of them)
+__device__ __forceinline__ void prefetch_l2(const double* p, int n)
+{
+    const unsigned long long g = __cvta_generic_to_global(p);
+    const unsigned bytes = (static_cast<unsigned>(n) * 8u) & ~15u;
+    if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(g & ~15ull), "r"(bytes) : "memory");
+}
+
+// contraction tables: with the inverse mass folded in (FP64), or the plain ones
+template <typename T> struct ColTab;
+template <> struct ColTab<double> {
+    static __device__ __forceinline__ const double* B(const StageTables& t) { return t.MB; }
+    static __device__ __forceinline__ const double* D(const StageTables& t) { return t.MD; }
+};
+template <> struct ColTab<float> {
+    static __device__ __forceinline__ const float* B(const StageTables& t) { return t.Bf; }
+    static __device__ __forceinline__ const float* D(const StageTables& t) { return t.Df; }
+};
+
+// entry (q, b) of a table of M x N values that is (anti)symmetric under the
+// reversal of both indices: only its first half is read
+template <int MN, typename T>
+__device__ __forceinline__ T sym(const T* t, int k) { return k < MN / 2 ? t[k] : t[MN - 1 - k]; }
+template <int MN, typename T>
+__device__ __forceinline__ T asym(const T* t, int k) { return k < MN / 2 ? t[k] : -t[MN - 1 - k]; }
+
+// c + (d x + b y): in FP64 two fused operations, in FP32 rounded as the stage
+// kernel's passes round it
+__device__ __forceinline__ double add_two(double c, double d, double x, double b, double y) { return fma(d, x, fma(b, y, c)); }
+__device__ __forceinline__ float add_two(float c, float d, float x, float b, float y)
+{
+    return __fadd_rn(c, __fmaf_rn(d, x, __fmul_rn(b, y)));
+}
+
+template <int P, int E, int NT, typename T, int MB>
+__global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ StageArgs a)
+{
+    using L = ColLay<P, T>;
+    constexpr int N = L::N, M = L::M, NB = L::NB, NF = L::NF, N2 = L::N2;
+    constexpr int PS = L::PS, AS = L::AS, X1S = L::X1S, W = L::W, VS = L::VS;
+    constexpr bool F64 = sizeof(T) == 8;
+    constexpr bool kShift = !F64;
+    constexpr int ROWS = E * 5 * N2;                   // coefficient rows along x of a batch
+    extern __shared__ double csm[];
+    double* sRes = csm;                                // [E][5][VS] (FP32 path)
+    double* sM = sRes + E * L::RES;                    // [2][N] end columns of the 1D inverse mass
+    T* sW = reinterpret_cast<T*>(sM + 2 * N);          // [E][W]
+    T* sL = sW + E * W;                                // [E][6][5][N2] lifts in this element's node order
+    T* sSgn = sL + E * L::LF;                          // [E][6] -1 on the left side, +1 on the right
+    int* sCls = reinterpret_cast<int*>(sSgn + E * 6);  // [E]
+    const T* __restrict__ Bt = TabSel<T>::B(a.tab);
+    const T* __restrict__ Wt = TabSel<T>::W(a.tab);
+    const T* __restrict__ Ct = ColTab<T>::B(a.tab);
+    const T* __restrict__ Dt = ColTab<T>::D(a.tab);
+    const double* __restrict__ Mi = a.tab.Minv;
+    const int tid = threadIdx.x;
+    const T gamma = T(a.gamma);
+    const int mode = a.mode;
+    const bool need_u0 = mode >= kModeRK1, need_acc = mode == kModeRK2 || mode == kModeRK3 || mode == kModeRK4;
+    unsigned status = 0;
+    // spread of a face's lift along its normal: the end columns of the 1D inverse
+    // mass, or of the identity for the residual output
+    if (tid < 2 * N) {
+        const int b = tid % N, end = tid < N ? 0 : N - 1;
+        sM[tid] = mode == kModeResidual ? (b == end ? 1.0 : 0.0) : Mi[b * N + end];
+    }
+
+    const int stride = gridDim.x * E;
+    for (int e0 = a.e_begin + blockIdx.x * E; e0 < a.ne; e0 += stride) {
+        // the next batch's rows and RK operands on their way into L2
+        if (tid < 3 && e0 + stride < a.ne && (tid == 0 || (tid == 1 ? need_u0 && a.U0 != a.Us : need_acc)))
+            prefetch_l2((tid == 0 ? a.Us : tid == 1 ? a.U0 : a.acc) + (size_t)(e0 + stride) * 5 * NB,
+                        min(E, a.ne - e0 - stride) * 5 * NB);
+        // ---- this batch's face lifts stream in (used by the last pass) ----
+        {
+            const T* gL = reinterpret_cast<const T*>(a.fflux);
+#pragma unroll 1
+            for (int i = tid; i < E * 6 * N2; i += NT) {
+                const int c = i % N2, f = (i / N2) % 6, e = i / (6 * N2);
+                // the second half of the face record: neighbour, info, class, listed face
+                const int4 fr = *(reinterpret_cast<const int4*>(a.frec + (size_t)min(e0 + e, a.ne - 1) * 6 + f) + 2);
+                const int pc = ((fr.w >> 30) & 1) ? c : a.cmapn[(fr.y >> 4) * N2 + c];
+                const T* src = gL + (size_t)(fr.w & 0x3fffffff) * a.fstride + pc;
+                T* dst = sL + e * L::LF + f * 5 * N2 + c;
+#pragma unroll
+                for (int v = 0; v < 5; ++v) cp_async_t(dst + v * N2, src + v * N2);
+                if (c == 0) sSgn[e * 6 + f] = ((fr.y >> 3) & 1) ? T(-1) : T(1);
+                if (c == 0 && f == 0) sCls[e] = fr.z;
+            }
+            cp_async_commit();
+        }
+        // ---- x interpolation ----
+#pragma unroll 1
+        for (int i = tid; i < ROWS; i += NT) {
+            const int e = i / (5 * N2), row = i - e * (5 * N2), v = row / N2, byz = row - v * N2;
+            const int ge = min(e0 + e, a.ne - 1);
+            double ur[N];
+            load_row<N>(a.Us + ((size_t)ge * 5 * N2 + row) * N, ur);
+            const double sh = kShift && v == 4 ? a.geo[a.geo_class[ge]].eref : 0.0;
+            T u[N];
+#pragma unroll
+            for (int b = 0; b < N; ++b) u[b] = kShift ? T(ur[b] - sh) : T(ur[b]);
+            T* o = sW + e * W + 5 * AS + v * X1S + byz * M;
+#pragma unroll
+            for (int q = 0; q < M; ++q) {
+                T s = T(0);
+#pragma unroll
+                for (int b = 0; b < N; ++b) s += sym<M * N>(Bt, q * N + b) * u[b];
+                o[q] = s;
+            }
+        }
+        cta_sync<NT>();
+        // ---- y interpolation ----
+#pragma unroll 1
+        for (int i = tid; i < E * 5 * N * M; i += NT) {
+            const int e = i / (5 * N * M);
+            int v, qx, bz;
+            task3<L::oy, 5, M, N>(i - e * (5 * N * M), v, qx, bz);
+            const T* x1 = sW + e * W + 5 * AS + v * X1S + bz * N * M + qx;
+            T col[N];
+#pragma unroll
+            for (int b = 0; b < N; ++b) col[b] = x1[b * M];
+            T* o = sW + e * W + v * AS + bz * PS + qx;
+#pragma unroll
+            for (int q = 0; q < M; ++q) {
+                T s = T(0);
+#pragma unroll
+                for (int b = 0; b < N; ++b) s += sym<M * N>(Bt, q * N + b) * col[b];
+                o[q * M] = s;
+            }
+        }
+        cta_sync<NT>();
+        // ---- columns: z interpolation, flux, z contraction in registers ----
+#pragma unroll 1
+        for (int i = tid; i < E * NF; i += NT) {
+            const int e = i / NF, qxy = i - e * NF;
+            T* col = sW + e * W + qxy;
+            T S[5][M];  // rho, momenta, energy (then enthalpy rE + P) at the column's points
+#pragma unroll
+            for (int v = 0; v < 5; ++v) {
+                T x[N];
+#pragma unroll
+                for (int b = 0; b < N; ++b) x[b] = col[v * AS + b * PS];
+#pragma unroll
+                for (int q = 0; q < M; ++q) {
+                    T s = T(0);
+#pragma unroll
+                    for (int b = 0; b < N; ++b) s += sym<M * N>(Bt, q * N + b) * x[b];
+                    S[v][q] = s;
+                }
+            }
+            const GeoDev* geo = a.geo + sCls[e];
+            const T hr = kShift ? T(a.gamma * geo->eref) : T(0);
+            const T pref = kShift ? T((a.gamma - 1.0) * geo->eref) : T(0);
+            T vel[3][M], p[M];
+#pragma unroll
+            for (int q = 0; q < M; ++q) {
+                // P = (gamma-1) (rE - |m|^2 / (2 rho)), as dgp::interior_flux_r1
+                const T r1 = T(1.) / S[0][q];
+                p[q] = (gamma - T(1.0)) * (S[4][q] - T(0.5) * ((S[1][q] * S[1][q] + S[2][q] * S[2][q] + S[3][q] * S[3][q]) * r1));
+#pragma unroll
+                for (int d = 0; d < 3; ++d) vel[d][q] = S[1 + d][q] * r1;
+                if (!(S[0][q] > T(0))) status |= kStatusRho;
+                if (!(p[q] + pref > T(0))) status |= kStatusPressure;
+                if (S[0][q] != S[0][q] || p[q] != p[q]) status |= kStatusNaN;
+                S[4][q] = kShift ? S[4][q] + p[q] + hr : S[4][q] + p[q];
+            }
+            T JD[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) JD[k] = T(geo->JD[k]);
+            const T wxy = Wt[qxy % M] * Wt[qxy / M];
+            // contract the components g_d(v, q) of each variable along z
+            auto contract = [&](auto&& component) {
+#pragma unroll
+                for (int v = 0; v < 5; ++v) {
+                    T a0[N], a1[N], a2[N];
+#pragma unroll
+                    for (int b = 0; b < N; ++b) { a0[b] = T(0); a1[b] = T(0); a2[b] = T(0); }
+#pragma unroll
+                    for (int q = 0; q < M; ++q) {
+                        T g[3];
+                        component(v, q, g);
+#pragma unroll
+                        for (int b = 0; b < N; ++b) {
+                            a0[b] += sym<M * N>(Ct, q * N + b) * g[0];
+                            a1[b] += sym<M * N>(Ct, q * N + b) * g[1];
+                            a2[b] += asym<M * N>(Dt, q * N + b) * g[2];
+                        }
+                    }
+#pragma unroll
+                    for (int b = 0; b < N; ++b) {
+                        col[(3 * v + 0) * AS + b * PS] = a0[b];
+                        col[(3 * v + 1) * AS + b * PS] = a1[b];
+                        col[(3 * v + 2) * AS + b * PS] = a2[b];
+                    }
+                }
+            };
+            if constexpr (F64) {
+                // S[v] V_d (+ P JD[d][v-1] for a momentum) with the weighted
+                // contravariant velocities V_d = w JD[d] . u
+#pragma unroll
+                for (int q = 0; q < M; ++q) {
+                    const T wq = wxy * Wt[q], u = vel[0][q], v = vel[1][q], w = vel[2][q];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                        vel[d][q] = (u * JD[d * 3 + 0] + v * JD[d * 3 + 1] + w * JD[d * 3 + 2]) * wq;
+                    p[q] *= wq;
+                }
+                contract([&](int v, int q, T (&g)[3]) {
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        g[d] = S[v][q] * vel[d][q];
+                        if (v >= 1 && v <= 3) g[d] += p[q] * JD[d * 3 + v - 1];
+                    }
+                });
+            } else {
+                // the stage kernel's operations in its order (the same bits):
+                // (F_0 JD[d][0] + F_1 JD[d][1] + F_2 JD[d][2]) w
+                auto flux = [&](int v, int q, T (&F)[3]) {
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                        F[d] = v == 0 ? S[1 + d][q] : (v == 1 + d ? S[v][q] * vel[d][q] + p[q] : S[v][q] * vel[d][q]);
+                };
+                if (JD[1] == T(0) && JD[2] == T(0) && JD[3] == T(0) && JD[5] == T(0) && JD[6] == T(0) && JD[7] == T(0))
+                    contract([&](int v, int q, T (&g)[3]) {  // axis-parallel element: the other products are zeros
+                        T F[3];
+                        flux(v, q, F);
+                        const T wq = wxy * Wt[q];
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) g[d] = (F[d] * JD[d * 4]) * wq;
+                    });
+                else
+                    contract([&](int v, int q, T (&g)[3]) {
+                        T F[3];
+                        flux(v, q, F);
+                        const T wq = wxy * Wt[q];
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) g[d] = (F[0] * JD[d * 3 + 0] + F[1] * JD[d * 3 + 1] + F[2] * JD[d * 3 + 2]) * wq;
+                    });
+            }
+        }
+        cta_sync<NT>();
+        // ---- y contraction: By^T A0 over row 3v, Dy^T A1 + By^T A2 over row 3v+1 ----
+#pragma unroll 1
+        for (int i = tid; i < E * 5 * N * M; i += NT) {
+            const int e = i / (5 * N * M);
+            int v, qx, bz;
+            task3<L::oyc, 5, M, N>(i - e * (5 * N * M), v, qx, bz);
+            T* A0 = sW + e * W + (3 * v) * AS + bz * PS + qx;
+            T c0[N], c12[N];
+#pragma unroll
+            for (int b = 0; b < N; ++b) { c0[b] = T(0); c12[b] = T(0); }
+#pragma unroll
+            for (int q = 0; q < M; ++q) {
+                const T x0 = A0[q * M], x1 = A0[AS + q * M], x2 = A0[2 * AS + q * M];
+#pragma unroll
+                for (int b = 0; b < N; ++b) {
+                    c0[b] += sym<M * N>(Ct, q * N + b) * x0;
+                    c12[b] = add_two(c12[b], asym<M * N>(Dt, q * N + b), x1, sym<M * N>(Ct, q * N + b), x2);
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < N; ++b) {
+                A0[b * M] = c0[b];
+                A0[AS + b * M] = c12[b];
+            }
+        }
+        cp_async_wait_group<0>();  // the lifts have landed
+        cta_sync<NT>();
+        // ---- x contraction, face lifts; FP64: the stage update ----
+#pragma unroll 1
+        for (int i = tid; i < ROWS; i += NT) {
+            const int e = i / (5 * N2), row = i - e * (5 * N2), v = row / N2, byz = row - v * N2;
+            const int by = byz % N, bz = byz / N;
+            const size_t g = ((size_t)min(e0 + e, a.ne - 1) * 5 * N2 + row) * N;
+            double u0[N], ac[N];
+            if constexpr (F64) {
+                if (need_u0) load_row<N>(a.U0 + g, u0);
+                if (need_acc) load_row<N>(a.acc + g, ac);
+            }
+            const T* C0 = sW + e * W + (3 * v) * AS + bz * PS + by * M;
+            T x[N];
+#pragma unroll
+            for (int b = 0; b < N; ++b) x[b] = T(0);
+#pragma unroll
+            for (int q = 0; q < M; ++q) {
+                const T c0 = C0[q], c12 = C0[AS + q];
+#pragma unroll
+                for (int b = 0; b < N; ++b) x[b] = add_two(x[b], asym<M * N>(Dt, q * N + b), c0, sym<M * N>(Ct, q * N + b), c12);
+            }
+            // lifts: faces 4 / 2 at the row's ends, 1 / 3 and 0 / 5 along it
+            const T* Lv = sL + e * L::LF + v * N2;
+            const T* sg = sSgn + e * 6;
+            if constexpr (F64) {
+                const double l4 = sg[4] * Lv[4 * 5 * N2 + byz], l2 = sg[2] * Lv[2 * 5 * N2 + byz];
+                const double c1 = sg[1] * sM[by], c3 = sg[3] * sM[N + by], c0 = sg[0] * sM[bz], c5 = sg[5] * sM[N + bz];
+                const double* L1 = Lv + 1 * 5 * N2 + bz * N;
+                const double* L3 = Lv + 3 * 5 * N2 + bz * N;
+                const double* L0 = Lv + by * N;
+                const double* L5 = Lv + 5 * 5 * N2 + by * N;
+                const double scale = mode == kModeResidual ? 1.0 : a.dt * a.geo[sCls[e]].dtf * a.geo[sCls[e]].inv_djac;
+                double k[N];
+#pragma unroll
+                for (int b = 0; b < N; ++b) {
+                    double s = x[b];
+                    s += sM[b] * l4;
+                    s += sM[N + b] * l2;
+                    s += c1 * L1[b];
+                    s += c3 * L3[b];
+                    s += c0 * L0[b];
+                    s += c5 * L5[b];
+                    k[b] = scale * s;
+                }
+                if (e0 + e >= a.ne) continue;
+                double o[N], ao[N];
+                switch (mode) {
+                    case kModeRK1:
+#pragma unroll
+                        for (int b = 0; b < N; ++b) { ao[b] = k[b]; o[b] = 0.5 * k[b] + u0[b]; }
+                        break;
+                    case kModeRK2:
+#pragma unroll
+                        for (int b = 0; b < N; ++b) { ao[b] = ac[b] + 2.0 * k[b]; o[b] = 0.5 * k[b] + u0[b]; }
+                        break;
+                    case kModeRK3:
+#pragma unroll
+                        for (int b = 0; b < N; ++b) { ao[b] = ac[b] + 2.0 * k[b]; o[b] = 1.0 * k[b] + u0[b]; }
+                        break;
+                    case kModeRK4:
+#pragma unroll
+                        for (int b = 0; b < N; ++b) o[b] = u0[b] + (1.0 / 6.0) * (ac[b] + k[b]);
+                        break;
+                    case kModeFE:
+#pragma unroll
+                        for (int b = 0; b < N; ++b) o[b] = u0[b] + 1.0 * k[b];
+                        break;
+                    default:  // residual, mass-inverse residual
+#pragma unroll
+                        for (int b = 0; b < N; ++b) o[b] = k[b];
+                        break;
+                }
+                if (mode == kModeRK1 || mode == kModeRK2 || mode == kModeRK3) store_row<N>(a.acc + g, ao);
+                store_row<N>(a.out + g, o);
+            } else {
+                double t[N];
+#pragma unroll
+                for (int b = 0; b < N; ++b) {
+                    double s = 0.0;  // the node's faces, in face order
+                    if (bz == 0) s += double(sg[0] * Lv[by * N + b]);
+                    if (by == 0) s += double(sg[1] * Lv[1 * 5 * N2 + bz * N + b]);
+                    if (b == N - 1) s += double(sg[2] * Lv[2 * 5 * N2 + byz]);
+                    if (by == N - 1) s += double(sg[3] * Lv[3 * 5 * N2 + bz * N + b]);
+                    if (b == 0) s += double(sg[4] * Lv[4 * 5 * N2 + byz]);
+                    if (bz == N - 1) s += double(sg[5] * Lv[5 * 5 * N2 + by * N + b]);
+                    t[b] = double(x[b]) + s;
+                }
+                if (mode == kModeResidual) {
+                    if (e0 + e < a.ne) store_row<N>(a.out + ((size_t)(e0 + e) * 5 * N2 + row) * N, t);
+                    continue;
+                }
+                double* res = sRes + e * L::RES + v * VS;
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                    double s = 0.0;
+#pragma unroll
+                    for (int k = 0; k < N; ++k) s += Mi[j * N + k] * t[k];
+                    res[Lay<P, 1>::cw(j, by, bz)] = s;
+                }
+            }
+        }
+        if constexpr (!F64) {
+            if (mode != kModeResidual) {
+                // ---- FP64 inverse mass along y, then z fused with the update ----
+                cta_sync<NT>();
+#pragma unroll 1
+                for (int i = tid; i < ROWS; i += NT) {
+                    const int e = i / (5 * N2);
+                    int v, bx, bz;
+                    task3<TaskOrd<P, 4>::minvy, 5, N, N>(i - e * (5 * N2), v, bx, bz);
+                    double* res = sRes + e * L::RES + v * VS;
+                    double t[N];
+#pragma unroll
+                    for (int k = 0; k < N; ++k) t[k] = res[Lay<P, 1>::cw(bx, k, bz)];
+#pragma unroll
+                    for (int j = 0; j < N; ++j) {
+                        double s = 0.0;
+#pragma unroll
+                        for (int k = 0; k < N; ++k) s += Mi[j * N + k] * t[k];
+                        res[Lay<P, 1>::cw(bx, j, bz)] = s;
+                    }
+                }
+                cta_sync<NT>();
+#pragma unroll 1
+                for (int i = tid; i < ROWS; i += NT) {
+                    const int e = i / (5 * N2), row = i - e * (5 * N2), v = row / N2, bxy = row - v * N2;
+                    if (e0 + e >= a.ne) continue;
+                    const size_t g0 = ((size_t)(e0 + e) * 5 + v) * NB + bxy;
+                    double u0[N], ac[N];
+#pragma unroll
+                    for (int k = 0; k < N; ++k) {
+                        if (need_u0) u0[k] = a.U0[g0 + k * N2];
+                        if (need_acc) ac[k] = a.acc[g0 + k * N2];
+                    }
+                    const int bx = bxy % N, by = bxy / N;
+                    const GeoDev& gg = a.geo[sCls[e]];
+                    const double scale = a.dt * gg.dtf * gg.inv_djac;
+                    const double* res = sRes + e * L::RES + v * VS;
+                    double t[N];
+#pragma unroll
+                    for (int k = 0; k < N; ++k) t[k] = res[Lay<P, 1>::cw(bx, by, k)];
+#pragma unroll
+                    for (int j = 0; j < N; ++j) {
+                        double s = 0.0;
+#pragma unroll
+                        for (int k = 0; k < N; ++k) s += Mi[j * N + k] * t[k];
+                        const double kk = scale * s;
+                        const size_t g = g0 + (size_t)j * N2;
+                        switch (mode) {
+                            case kModeMassInv: a.out[g] = kk; break;
+                            case kModeRK1: a.acc[g] = kk; a.out[g] = 0.5 * kk + u0[j]; break;
+                            case kModeRK2: a.acc[g] = ac[j] + 2.0 * kk; a.out[g] = 0.5 * kk + u0[j]; break;
+                            case kModeRK3: a.acc[g] = ac[j] + 2.0 * kk; a.out[g] = 1.0 * kk + u0[j]; break;
+                            case kModeRK4: a.out[g] = u0[j] + (1.0 / 6.0) * (ac[j] + kk); break;
+                            default: a.out[g] = u0[j] + 1.0 * kk; break;
+                        }
+                    }
+                }
+            }
+        }
+        cta_sync<NT>();  // the point array and the lifts are the next batch's
+    }
+    if (status) atomicOr(a.status, status);
+}
+
+// ---------------------------------------------------------------------------
+// the face kernel with the lift: batches of FB faces as face_flux_body, then
+// L[b1][b0] = sum_t1 C[t1][b1] sum_t0 C[t0][b0] F[t1][t0] (C = B Minv in FP64,
+// B in FP32), one task per (face, variable, output column)
+template <int P, typename T, int FB, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant__ StageArgs a)
+{
+    using L = Lay<P, 1, T>;
+    constexpr int N = L::N, M = L::M, NB = L::NB, NF = L::NF, N2 = L::N2, FS = L::FS;
+    constexpr bool kShift = sizeof(T) == 4;
+    extern __shared__ double fsm[];
+    T* sTr = reinterpret_cast<T*>(fsm);                                             // [FB][2][5][FS]
+    unsigned char* tail = reinterpret_cast<unsigned char*>(sTr) + ((sizeof(T) * FB * 10 * FS + 15) / 16) * 16;
+    FaceRec* sRecBuf = reinterpret_cast<FaceRec*>(tail);                            // [2][FB] listed side's records
+    int* sELBuf = reinterpret_cast<int*>(sRecBuf + 2 * FB);                         // [2][FB] listed elements
+    int* sFLBuf = sELBuf + 2 * FB;                                                  // [2][FB] listed faces
+    const T* __restrict__ Bt = TabSel<T>::B(a.tab);
+    const T* __restrict__ Wt = TabSel<T>::W(a.tab);
+    const T* __restrict__ Ct = ColTab<T>::B(a.tab);
+    T* out = reinterpret_cast<T*>(a.fflux);
+    const int tid = threadIdx.x;
+    unsigned status = 0;
+    auto fetch_records = [&](int f, int rb, int2 fe) {
+        if (tid < FB && f < a.nface) {
+            sELBuf[rb * FB + tid] = fe.x;
+            sFLBuf[rb * FB + tid] = fe.y;
+            const double* src = reinterpret_cast<const double*>(a.frec + (size_t)fe.x * 6 + fe.y);
+            double* dst = reinterpret_cast<double*>(sRecBuf + rb * FB + tid);
+#pragma unroll
+            for (int w = 0; w < 6; ++w) cp_async8(dst + w, src + w);
+        }
+        cp_async_commit();
+    };
+    const int f_first = a.face_begin + blockIdx.x * FB, fstep = gridDim.x * FB;
+    if (f_first < a.nface)
+        fetch_records(f_first, 0, tid < FB ? a.faces[min(f_first + tid, a.nface - 1)] : make_int2(0, 0));
+    int it = 0;
+    for (int f0 = f_first; f0 < a.nface; f0 += fstep, ++it) {
+        const int rb = it & 1;
+        FaceRec* sRecL = sRecBuf + rb * FB;
+        const int* sEL = sELBuf + rb * FB;
+        const int* sFL = sFLBuf + rb * FB;
+        cp_async_wait_all();
+        __syncthreads();
+        const int fn = f0 + fstep;
+        const int2 fe_next = tid < FB && fn < a.nface ? a.faces[min(fn + tid, a.nface - 1)] : make_int2(0, 0);
+        for (int t = tid; t < FB * 10; t += NT) {
+            const int v = t % 5, sj = t / 5, j = sj / 2, side = sj % 2;
+            const FaceRec& rec = sRecL[j];
+            const int el = side == 0 ? sEL[j] : rec.nbr;
+            const int fc = side == 0 ? sFL[j] : (rec.info & 7);
+            const int ax = face_axis(fc), sidx = face_side(fc) ? N - 1 : 0;
+            const int o0 = ax == 0 ? sidx : (ax == 1 ? sidx * N : sidx * N2);
+            const int s0 = ax == 0 ? N : 1, s1 = ax == 2 ? N : N2;
+            const double* src = a.Us + ((size_t)el * 5 + v) * NB + o0;
+            const double sh = kShift && v == 4 ? a.geo[rec.cls].eref : 0.0;
+            double x[N][N];
+#pragma unroll
+            for (int b1 = 0; b1 < N; ++b1)
+#pragma unroll
+                for (int b0 = 0; b0 < N; ++b0) x[b1][b0] = __ldg(src + b0 * s0 + b1 * s1);
+            T sl[N][N];
+#pragma unroll
+            for (int b1 = 0; b1 < N; ++b1)
+#pragma unroll
+                for (int b0 = 0; b0 < N; ++b0) sl[b1][b0] = kShift ? T(x[b1][b0] - sh) : T(x[b1][b0]);
+            interp2d<N, M, T>(Bt, sl, sTr + (sj * 5 + v) * FS);
+        }
+        fetch_records(fn, rb ^ 1, fe_next);
+        __syncthreads();
+        // the flux at the listed side's face points, over that side's trace
+        for (int i = tid; i < FB * NF; i += NT) {
+            const int c = i % NF, j = i / NF;
+            if (f0 + j >= a.nface) continue;
+            const FaceRec& rec = sRecL[j];
+            const int cn = a.cmap[(rec.info >> 4) * NF + c];
+            const int isL = (rec.info >> 3) & 1;
+            T* To = sTr + (j * 2) * 5 * FS;
+            const T* Tn = To + 5 * FS;
+            T UL[5], UR[5], Fo[5];
+#pragma unroll
+            for (int v = 0; v < 5; ++v) {
+                const T uo = To[v * FS + c], un = Tn[v * FS + cn];
+                UL[v] = isL ? uo : un;
+                UR[v] = isL ? un : uo;
+            }
+            const T nd[4] = {T(rec.n[0]), T(rec.n[1]), T(rec.n[2]), T(rec.nmag)};
+            const double eref = kShift ? a.geo[rec.cls].eref : 0.0;
+            numerical_flux<T, kShift>(a.flux, a.gamma, UL, UR, nd, eref, Fo, status);
+            const T w = Wt[c % M] * Wt[c / M];
+#pragma unroll
+            for (int v = 0; v < 5; ++v) To[v * FS + c] = Fo[v] * w;
+        }
+        __syncthreads();
+        for (int t = tid; t < FB * 5 * N; t += NT) {
+            const int b0 = t % N, jv = t / N, v = jv % 5, j = jv / 5;
+            if (f0 + j >= a.nface) continue;
+            const T* F = sTr + (j * 2) * 5 * FS + v * FS;
+            T r[M];
+#pragma unroll
+            for (int t1 = 0; t1 < M; ++t1) {
+                T s = T(0);
+#pragma unroll
+                for (int t0 = 0; t0 < M; ++t0) s += Ct[t0 * N + b0] * F[t1 * M + t0];
+                r[t1] = s;
+            }
+            T* o = out + (size_t)(f0 + j) * a.fstride + v * N2 + b0;
+#pragma unroll
+            for (int b1 = 0; b1 < N; ++b1) {
+                T s = T(0);
+#pragma unroll
+                for (int t1 = 0; t1 < M; ++t1) s += Ct[t1 * N + b1] * r[t1];
+                o[b1 * N] = s;
+            }
+        }
+    }
+    cp_async_wait_all();
+    if (status) atomicOr(a.status, status);
+}
+
+template <int P, typename T, int FB>
+constexpr size_t face_lift_smem_bytes()
+{
+    return ((sizeof(T) * FB * 10 * Lay<P, 1, T>::FS + 15) / 16) * 16 + 2 * FB * sizeof(FaceRec) + 4 * FB * sizeof(int);
+}
+
+template <int P, int E, int NT, typename T, int MB>
+cudaError_t launch_column(const StageArgs& a, int grid, cudaStream_t s)
+{
+    column_kernel<P, E, NT, T, MB><<<grid, NT, ColLay<P, T>::bytes(E), s>>>(a);
+    return cudaGetLastError();
+}
+template <int P, typename T, int FB, int NT, int MB>
+cudaError_t launch_face_lift(const StageArgs& a, int grid, cudaStream_t s)
+{
+    face_lift_kernel<P, T, FB, NT, MB><<<grid, NT, face_lift_smem_bytes<P, T, FB>(), s>>>(a);
+    return cudaGetLastError();
+}
+
+// E elements and NT threads per CTA, at least MB resident CTAs per SM asked of the
+// compiler; the default from min_per_sm elements per SM on (below, the stage
+// kernel's many threads per element finish sooner than one warp per element)
+template <int P, int E, int NT, typename T, int MB>
+StageVariant make_column_variant(int min_per_sm)
+{
+    static_assert(ColLay<P, T>::bytes(E) <= 227 * 1024, "column kernel shared memory exceeds 227 KB");
+    constexpr int FB = face_batch<P, T>(), FNT = face_threads<P, T>(), FMB = 1;
+    StageVariant v{E, NT, 1, sizeof(T) == 4 ? 1 : 0, kSB | kFX | kCF, ColLay<P, T>::bytes(E),
+                   (const void*)column_kernel<P, E, NT, T, MB>, launch_column<P, E, NT, T, MB>, nullptr, 0, 0, nullptr, 0, min_per_sm};
+    v.face_func = (const void*)face_lift_kernel<P, T, FB, FNT, FMB>;
+    v.face_smem = face_lift_smem_bytes<P, T, FB>();
+    v.face_threads = FNT;
+    v.face_launch = launch_face_lift<P, T, FB, FNT, FMB>;
+    v.face_batch = FB;
+    return v;
+}
+
+}  // namespace dgk

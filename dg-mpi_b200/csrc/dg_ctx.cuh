@@ -43,6 +43,7 @@ struct dg_ctx {
     int* d_geo_class = nullptr;
     dgk::GeoDev* d_geo = nullptr;
     uint8_t* d_cmap = nullptr;
+    uint8_t* d_cmapn = nullptr;  // inside d_cmap's allocation
     double* d_X0 = nullptr;
     // general (trilinear) geometry (pm.general): the stage kernel's per-point
     // tables (see dgk::StageArgs) and the element nodes [ne][8][3]

@@ -55,6 +55,10 @@ struct StageTables {
     // derivative of the 1D Lagrange basis at its own equidistant nodes,
     // Dn[i*N + j] = l_j'(xi_i) (the tensor-core kernel's nodal derivative)
     float Dn[(kMaxP + 1) * (kMaxP + 1)];
+    // contraction tables of the column form in FP64: B and D times the inverse
+    // 1D mass matrix (or B and D themselves for the residual output)
+    double MB[kTabB];
+    double MD[kTabB];
 };
 
 template <typename T> struct TabSel;
@@ -123,6 +127,7 @@ struct StageArgs {
     const int* geo_class;   // [ne]
     const GeoDev* geo;      // [nclasses]
     const uint8_t* cmap;    // [ncodes][m*m]
+    const uint8_t* cmapn;   // [ncodes][n*n], the same permutation of the face nodes
     // general (trilinear) geometry, launch option GE: per element ijac * djac
     // at the volume points [ne][9][(p+2)^3], the face normal data at the own
     // face points [ne][6][4][(p+2)^2] (n as for FaceRec, then |N|), and the
@@ -362,6 +367,8 @@ __device__ __forceinline__ void cp_async4(float* smem_dst, const float* gmem_src
 __device__ __forceinline__ void cp_async_t(double* d, const double* g) { cp_async8(d, g); }
 __device__ __forceinline__ void cp_async_t(float* d, const float* g) { cp_async4(d, g); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int G>
+__device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;\n" ::"n"(G) : "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 // all but the most recent group complete
 __device__ __forceinline__ void cp_async_wait_older() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
@@ -1518,6 +1525,7 @@ struct StageVariant {
     int face_threads;
     cudaError_t (*face_launch)(const StageArgs&, int grid, cudaStream_t);
     int face_batch;      // faces per CTA batch of the face kernel
+    int min_per_sm;      // elements per SM from which the variant may be the untuned default
 };
 
 template <int P, typename T, bool GEO>
@@ -1557,7 +1565,7 @@ StageVariant make_variant()
     if constexpr (MB > 0) func = (const void*)stage_kernel_mb<P, E, NT, G, T, FL, MB>;
     else func = (const void*)stage_kernel<P, E, NT, G, T, FL>;
     StageVariant v{E, NT, G, sizeof(T) == 4 ? 1 : 0, FL | (MB << 8), stage_smem_bytes<P, E, G, T, FL>(),
-                   func, launch_stage_variant<P, E, NT, G, T, FL, MB>, nullptr, 0, 0, nullptr, 0};
+                   func, launch_stage_variant<P, E, NT, G, T, FL, MB>, nullptr, 0, 0, nullptr, 0, 0};
     if constexpr ((FL & 64) != 0) {
         static_assert(face_smem_bytes<P, T>() <= 227 * 1024, "face kernel shared memory exceeds 227 KB");
         constexpr bool geo = (FL & 32) != 0;

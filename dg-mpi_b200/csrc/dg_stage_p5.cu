@@ -7,10 +7,12 @@
 // general-geometry (kGE) entries only, the others never do.  The
 // first variant of each precision is the default (the measured best); dg_tune_stage may pick another.
 #include "dg_stage.cuh"
+#include "dg_column.cuh"
 
 namespace dgk {
 
 static const StageVariant kVariants5[] = {
+    make_column_variant<5, 1, 64, double, 4>(3),
     make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kFX | kMG, 2>(),
     make_variant<5, 1, 192, 1, double, kUF | kRS | kSB | kFX | kMG>(),
     make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kFX, 2>(),
@@ -19,6 +21,7 @@ static const StageVariant kVariants5[] = {
     make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kK1, 2>(),
     make_variant<5, 1, 128, 1, double, kUF | kRS | kSB | kK1>(),
     make_variant<5, 1, 128, 3, double>(),
+    make_column_variant<5, 1, 64, float, 6>(6),
     make_variant<5, 1, 256, 1, float, kUF | kSB | kFX | kMG, 3>(),
     make_variant<5, 1, 256, 1, float, kUF | kRS | kSB | kFX | kMG, 3>(),
     make_variant<5, 1, 256, 1, float, kUF | kRS | kSB | kFX, 3>(),

@@ -443,6 +443,19 @@ std::string prepare_mesh(const MeshView& mv, int m, PreparedMesh& out)
         order_inv[o].assign(m * m, -1);
         for (int q = 0; q < m * m; ++q) order_inv[o][order[o][q]] = q;
     }
+    // the same maps of the (m-1) x (m-1) face nodes
+    const int n1 = m - 1, n2 = n1 * n1;
+    std::vector<int> ncanon[6], ncanon_inv[6], norder[8], norder_inv[8];
+    for (int f = 0; f < 6; ++f) {
+        face_canonical_map(n1, f, ncanon[f]);
+        ncanon_inv[f].assign(n2, -1);
+        for (int q = 0; q < n2; ++q) ncanon_inv[f][ncanon[f][q]] = q;
+    }
+    for (int o = 0; o < 8; ++o) {
+        face_orientation_order(o, n2, norder[o]);
+        norder_inv[o].assign(n2, -1);
+        for (int q = 0; q < n2; ++q) norder_inv[o][norder[o][q]] = q;
+    }
     out.conn.assign(static_cast<size_t>(ne) * 12, -1);
     std::map<std::array<int, 4>, int> code_of;
     auto add_side = [&](int e, int f, int en, int fn, int ox, int oy, int isL) -> std::string {
@@ -460,6 +473,8 @@ std::string prepare_mesh(const MeshView& mv, int m, PreparedMesh& out)
                 const int b = order[oy][q];           // neighbour's face point
                 out.cmap.push_back(static_cast<uint8_t>(canon[fn][b]));
             }
+            for (int c = 0; c < n2; ++c)
+                out.cmapn.push_back(static_cast<uint8_t>(ncanon[fn][norder[oy][norder_inv[ox][ncanon_inv[f][c]]]]));
         } else {
             code = it->second;
         }

@@ -55,6 +55,7 @@ struct PreparedMesh {
     std::vector<int> geo_class;        // [ne]
     std::vector<GeoClass> classes;
     std::vector<int> conn;             // [ne][6][2]: neighbour element, packed (fn | isL<<3 | code<<4)
+    std::vector<uint8_t> cmapn;        // [ncodes][n*n]: the same for the face nodes, n = m - 1
     std::vector<uint8_t> cmap;         // [ncodes][m*m]: own canonical face point -> neighbour's
     int ncodes = 0;
     std::vector<double> X0;            // [ne][3] coordinates of local node 0
