@@ -336,75 +336,148 @@ struct ReduceArgs {
     double data[16];
 };
 
-template <int P>
-__global__ void __launch_bounds__(256) reduce_kernel(ReduceArgs a)
+// Points per direction (the error's rule of 2 max(p,1) + 2, the kinetic
+// energy's volume rule), elements and threads per CTA: one thread per (x, y)
+// point column of an element, whole elements to a CTA of about 128 threads.
+template <int P, int KIND>
+struct ReduceCfg {
+    static constexpr int N = P + 1, NB = N * N * N, ME = KIND == 0 ? (P > 1 ? 2 * P + 2 : 4) : P + 2;
+    static constexpr int NV = KIND == 0 ? 5 : 4;  // the kinetic energy needs no energy
+    static constexpr int E = ME * ME >= 128 ? 1 : 128 / (ME * ME), NT = (E * ME * ME + 31) / 32 * 32;
+    static constexpr size_t smem = sizeof(double) * E * NV * (NB + N * N * ME + N * ME * ME);
+};
+
+// Interpolation by three 1D passes (x and y through shared memory, z in the
+// column's thread); the dense sum over the (p+1)^3 basis functions per point
+// that this replaces was bound by its 5 (N^3 + N^2 + N) multiply-adds and its
+// divergent constant-memory indices.  Calls, 48^3, p = 4: kinetic energy 4.04 -> 0.47 ms, x-y vortex
+// error 18.1 -> 2.7 ms; 32^3, p = 3: error 9.37 -> 0.37 ms.  Each interpolated
+// value is the same sum in the same order.
+template <int P, int KIND>
+__global__ void __launch_bounds__(ReduceCfg<P, KIND>::NT) reduce_kernel(ReduceArgs a)
 {
-    constexpr int N = P + 1, NB = N * N * N;
-    __shared__ double sU[5 * NB];
-    __shared__ double red[5][256];
-    const int me = a.kind == 0 ? (P > 1 ? 2 * P + 2 : 4) : P + 2;
-    const double* Bq = a.kind == 0 ? cBe[P] : cVB[P];
-    const double* Wq = a.kind == 0 ? cWe[P] : cVW[P];
-    const double* Xq = a.kind == 0 ? cXe[P] : cXq[P];
+    using C = ReduceCfg<P, KIND>;
+    constexpr int N = C::N, NB = C::NB, N2 = N * N, ME = C::ME, M2 = ME * ME, E = C::E, NT = C::NT, NV = C::NV;
+    extern __shared__ double rsm[];
+    double* sU = rsm;                   // [E][NV][bz][by][bx]
+    double* s1 = sU + E * NV * NB;      // [E][NV][bz][by][i]
+    double* s2 = s1 + E * NV * N2 * ME; // [E][NV][bz][j][i]
+    const double* Bq = KIND == 0 ? cBe[P] : cVB[P];
+    const double* Wq = KIND == 0 ? cWe[P] : cVW[P];
+    const double* Xq = KIND == 0 ? cXe[P] : cXq[P];
+    const int tid = threadIdx.x;
     double acc[5] = {0, 0, 0, 0, 0};
-    for (int e = blockIdx.x; e < a.ne; e += gridDim.x) {
+    for (int e0 = blockIdx.x * E; e0 < a.ne; e0 += gridDim.x * E) {
+        const int en = min(E, a.ne - e0);
+        for (int i = tid; i < en * NV * NB; i += NT) {
+            const int e = i / (NV * NB), r = i - e * (NV * NB);
+            sU[i] = a.U[(size_t)(e0 + e) * 5 * NB + r];
+        }
         __syncthreads();
-        for (int i = threadIdx.x; i < 5 * NB; i += blockDim.x) sU[i] = a.U[(size_t)e * 5 * NB + i];
+        for (int t = tid; t < en * NV * N2; t += NT) {  // x: rows (e, v, bz, by)
+            double u[N];
+#pragma unroll
+            for (int b = 0; b < N; ++b) u[b] = sU[t * N + b];
+#pragma unroll
+            for (int i = 0; i < ME; ++i) {
+                double s = 0.0;
+#pragma unroll
+                for (int b = 0; b < N; ++b) s += Bq[i * N + b] * u[b];
+                s1[t * ME + i] = s;
+            }
+        }
         __syncthreads();
-        const int cls = a.geo_class[e];
-        const double* J = a.J + cls * 9;
-        const double djac = 1.0 / a.geo[cls].inv_djac;
-        for (int q = threadIdx.x; q < me * me * me; q += blockDim.x) {
-            const int i = q % me, j = (q / me) % me, k = q / (me * me);
-            double Uq[5];
+        for (int t = tid; t < en * NV * N * ME; t += NT) {  // y: (e, v, bz, i)
+            const int i = t % ME, evz = t / ME;
+            double u[N];
 #pragma unroll
-            for (int v = 0; v < 5; ++v) {
-                double sz = 0.0;
-                for (int bz = 0; bz < N; ++bz) {
-                    double sy = 0.0;
-                    for (int by = 0; by < N; ++by) {
-                        double sx = 0.0;
+            for (int b = 0; b < N; ++b) u[b] = s1[(evz * N + b) * ME + i];
 #pragma unroll
-                        for (int bx = 0; bx < N; ++bx) sx += Bq[i * N + bx] * sU[v * NB + (bz * N + by) * N + bx];
-                        sy += Bq[j * N + by] * sx;
+            for (int j = 0; j < ME; ++j) {
+                double s = 0.0;
+#pragma unroll
+                for (int b = 0; b < N; ++b) s += Bq[j * N + b] * u[b];
+                s2[(evz * ME + j) * ME + i] = s;
+            }
+        }
+        __syncthreads();
+        if (tid < en * M2) {  // z and the integrand, column (i, j) of element e
+            const int e = tid / M2, ij = tid - e * M2, i = ij % ME, j = ij / ME, ge = e0 + e;
+            double u[NV][N];
+#pragma unroll
+            for (int v = 0; v < NV; ++v)
+#pragma unroll
+                for (int b = 0; b < N; ++b) u[v][b] = s2[((e * NV + v) * N + b) * M2 + ij];
+            const int cls = a.geo_class[ge];
+            const double* J = a.J + cls * 9;
+            const double djac = 1.0 / a.geo[cls].inv_djac;
+            // the x-y vortex does not change along a column that runs along z
+            const bool same = KIND == 0 && a.ic_type == DG_IC_VORTEX_XY && !a.gnodes && J[2] == 0.0 && J[5] == 0.0;
+            double Ue[5];
+#pragma unroll 1
+            for (int k = 0; k < ME; ++k) {
+                double Uq[NV];
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    double s = 0.0;
+#pragma unroll
+                    for (int b = 0; b < N; ++b) s += Bq[k * N + b] * u[v][b];
+                    Uq[v] = s;
+                }
+                double x[3], dj = djac;
+                if (a.gnodes) {
+                    const double xr[3] = {Xq[i], Xq[j], Xq[k]};
+                    trilinear_point(a.gnodes + (size_t)ge * 24, xr, x, &dj);
+                } else if (KIND == 0) {
+                    const double xi[3] = {Xq[i] + 1.0, Xq[j] + 1.0, Xq[k] + 1.0};
+                    for (int d = 0; d < 3; ++d)
+                        x[d] = a.X0[(size_t)ge * 3 + d] + J[d * 3 + 0] * xi[0] + J[d * 3 + 1] * xi[1] + J[d * 3 + 2] * xi[2];
+                }
+                const double w = (Wq[i] * Wq[j]) * Wq[k] * dj;
+                if constexpr (KIND == 0) {
+                    if (k == 0 || !same) dgp::initial_state(a.ic_type, a.data, a.gamma, a.R, x, a.t, Ue);
+#pragma unroll
+                    for (int v = 0; v < 5; ++v) {
+                        const double d = Uq[v] - Ue[v];
+                        acc[v] += d * d * w;
                     }
-                    sz += Bq[k * N + bz] * sy;
+                } else {
+                    acc[0] += 0.5 * (Uq[1] * Uq[1] + Uq[2] * Uq[2] + Uq[3] * Uq[3]) / Uq[0] * w;
                 }
-                Uq[v] = sz;
-            }
-            double x[3], dj = djac;
-            if (a.gnodes) {
-                const double xr[3] = {Xq[i], Xq[j], Xq[k]};
-                trilinear_point(a.gnodes + (size_t)e * 24, xr, x, &dj);
-            } else {
-                const double xi[3] = {Xq[i] + 1.0, Xq[j] + 1.0, Xq[k] + 1.0};
-                for (int d = 0; d < 3; ++d)
-                    x[d] = a.X0[(size_t)e * 3 + d] + J[d * 3 + 0] * xi[0] + J[d * 3 + 1] * xi[1] + J[d * 3 + 2] * xi[2];
-            }
-            const double w = (Wq[i] * Wq[j]) * Wq[k] * dj;
-            if (a.kind == 0) {
-                double Ue[5];
-                dgp::initial_state(a.ic_type, a.data, a.gamma, a.R, x, a.t, Ue);
-#pragma unroll
-                for (int v = 0; v < 5; ++v) {
-                    const double d = Uq[v] - Ue[v];
-                    acc[v] += d * d * w;
-                }
-            } else {
-                acc[0] += 0.5 * (Uq[1] * Uq[1] + Uq[2] * Uq[2] + Uq[3] * Uq[3]) / Uq[0] * w;
             }
         }
     }
-    __syncthreads();
-    for (int v = 0; v < 5; ++v) red[v][threadIdx.x] = acc[v];
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s)
-            for (int v = 0; v < 5; ++v) red[v][threadIdx.x] += red[v][threadIdx.x + s];
-        __syncthreads();
+    // the block's sums: warps by shuffles, then their results in warp order
+    __shared__ double red[5][NT / 32];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+        double s = acc[v];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (tid % 32 == 0) red[v][tid / 32] = s;
     }
-    if (threadIdx.x == 0)
-        for (int v = 0; v < 5; ++v) a.partials[blockIdx.x * 5 + v] = red[v][0];
+    __syncthreads();
+    if (tid < 5) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < NT / 32; ++w) s += red[tid][w];
+        a.partials[blockIdx.x * 5 + tid] = s;
+    }
+}
+
+// launches the reduction of ne elements on at most c->red_grid CTAs; *grid gets their number
+template <int P, int KIND>
+cudaError_t launch_reduce(const dg_ctx* c, const ReduceArgs& a, int* grid)
+{
+    using C = ReduceCfg<P, KIND>;
+    if (C::smem > 48 * 1024) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(reduce_kernel<P, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem);
+        if (e != cudaSuccess) return e;
+    }
+    *grid = std::max(1, std::min(c->red_grid, (a.ne + C::E - 1) / C::E));
+    reduce_kernel<P, KIND><<<*grid, C::NT, C::smem, c->stream>>>(a);
+    return cudaGetLastError();
 }
 
 int run_reduce(dg_ctx* c, int kind, int ic_type, const double* data, int ndata, double t, double* out5, int e0, int ne,
@@ -426,21 +499,29 @@ int run_reduce(dg_ctx* c, int kind, int ic_type, const double* data, int ndata, 
     for (int i = 0; i < ndata && i < 16; ++i) a.data[i] = data[i];
     // per-class Jacobians, kept on the device after the classes
     a.J = reinterpret_cast<const double*>(c->d_geo + c->pm.classes.size());
-    switch (c->p) {
-        case 0: reduce_kernel<0><<<c->red_grid, 256, 0, c->stream>>>(a); break;
-        case 1: reduce_kernel<1><<<c->red_grid, 256, 0, c->stream>>>(a); break;
-        case 2: reduce_kernel<2><<<c->red_grid, 256, 0, c->stream>>>(a); break;
-        case 3: reduce_kernel<3><<<c->red_grid, 256, 0, c->stream>>>(a); break;
-        case 4: reduce_kernel<4><<<c->red_grid, 256, 0, c->stream>>>(a); break;
-        case 5: reduce_kernel<5><<<c->red_grid, 256, 0, c->stream>>>(a); break;
+    int grid = 0;
+    cudaError_t le = cudaErrorInvalidValue;
+    switch (c->p * 2 + (kind ? 1 : 0)) {
+        case 0: le = launch_reduce<0, 0>(c, a, &grid); break;
+        case 1: le = launch_reduce<0, 1>(c, a, &grid); break;
+        case 2: le = launch_reduce<1, 0>(c, a, &grid); break;
+        case 3: le = launch_reduce<1, 1>(c, a, &grid); break;
+        case 4: le = launch_reduce<2, 0>(c, a, &grid); break;
+        case 5: le = launch_reduce<2, 1>(c, a, &grid); break;
+        case 6: le = launch_reduce<3, 0>(c, a, &grid); break;
+        case 7: le = launch_reduce<3, 1>(c, a, &grid); break;
+        case 8: le = launch_reduce<4, 0>(c, a, &grid); break;
+        case 9: le = launch_reduce<4, 1>(c, a, &grid); break;
+        case 10: le = launch_reduce<5, 0>(c, a, &grid); break;
+        case 11: le = launch_reduce<5, 1>(c, a, &grid); break;
         default: return fail(c, DG_ERR_UNSUPPORTED, "order out of range");
     }
-    DG_CUDA(c, cudaGetLastError());
-    std::vector<double> part(static_cast<size_t>(c->red_grid) * 5);
+    DG_CUDA(c, le);
+    std::vector<double> part(static_cast<size_t>(grid) * 5);
     DG_CUDA(c, cudaMemcpyAsync(part.data(), c->d_partials, part.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     DG_CUDA(c, cudaStreamSynchronize(c->stream));
     for (int v = 0; v < 5; ++v) out5[v] = 0.0;
-    for (int b = 0; b < c->red_grid; ++b)
+    for (int b = 0; b < grid; ++b)
         for (int v = 0; v < 5; ++v) out5[v] += part[static_cast<size_t>(b) * 5 + v];
     return DG_OK;
 }
@@ -1033,7 +1114,7 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
     const size_t ncls = c->pm.classes.size();
     int dev_sms = 0;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device);
-    c->red_grid = std::max(1, std::min(c->ne, 4 * dev_sms));
+    c->red_grid = std::max(1, std::min(c->ne, 8 * dev_sms));
     struct Alloc { void** p; size_t bytes; } allocs[] = {
         {(void**)&c->d_U0, nstate * sizeof(double)},
         {(void**)&c->d_Ua, nstate * sizeof(double)},
