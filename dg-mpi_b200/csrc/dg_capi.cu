@@ -178,6 +178,7 @@ void stage_args(const dg_ctx* c, int mode, const double* Us, const double* U0, d
     a.gimm = c->d_gimm;
     a.gfsd = c->d_gfsd;
     a.faces = c->d_faces;
+    a.fdesc = c->d_fdesc;
     a.nface = c->nface;
     a.fflux = c->d_fflux;
     a.fstride = 5 * (c->p + 2) * (c->p + 2);
@@ -290,6 +291,33 @@ __global__ void halo_unpack_kernel(double* __restrict__ U, const int2* __restric
         const int2 ef = list[s];
         U[((size_t)ef.x * 5 + v) * nb + slice_index_rt(n, ef.y, b % n, b / n)] = in[i];
     }
+}
+
+// ---------------------------------------------------------------------------
+// the face list's descriptors (see dgk::FaceDesc) from the face records
+
+__global__ void face_desc_kernel(const dgk::FaceRec* __restrict__ frec, const int2* __restrict__ faces, int nface, int n,
+                                 dgk::FaceDesc* __restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nface) return;
+    const int2 ef = faces[i];
+    const dgk::FaceRec r = frec[(size_t)ef.x * 6 + ef.y];
+    dgk::FaceDesc d;
+    for (int k = 0; k < 3; ++k) d.n[k] = r.n[k];
+    d.nmag = r.nmag;
+    d.strides = 0;
+    for (int side = 0; side < 2; ++side) {
+        const long long el = side == 0 ? ef.x : r.nbr;
+        const int f = side == 0 ? ef.y : (r.info & 7), ax = dgk::face_axis(f);
+        d.base[side] = el * 5 * n * n * n + slice_index_rt(n, f, 0, 0);
+        const unsigned s0 = ax == 0 ? n : 1, s1 = ax == 2 ? n : n * n;
+        d.strides |= (s0 | s1 << 8) << (16 * side);
+    }
+    d.info = r.info;
+    d.cls = r.cls;
+    d.pad = 0;
+    out[i] = d;
 }
 
 // ---------------------------------------------------------------------------
@@ -915,7 +943,7 @@ void release(dg_ctx* c)
     cudaFree(c->d_conn); cudaFree(c->d_frec); cudaFree(c->d_geo_class); cudaFree(c->d_geo); cudaFree(c->d_cmap);
     cudaFree(c->d_X0); cudaFree(c->d_partials); cudaFree(c->d_status);
     cudaFree(c->d_gjd); cudaFree(c->d_gnrm); cudaFree(c->d_gimm); cudaFree(c->d_gnodes); cudaFree(c->d_gfsd);
-    cudaFree(c->d_faces); cudaFree(c->d_fflux); cudaFree(c->d_tcop);
+    cudaFree(c->d_faces); cudaFree(c->d_fdesc); cudaFree(c->d_fflux); cudaFree(c->d_tcop);
     cudaFree(c->d_halo_send); cudaFree(c->d_halo_recv);
     for (cudaEvent_t e : c->chunk_ev) cudaEventDestroy(e);
     c->chunk_ev.clear();
@@ -1226,12 +1254,15 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
         const size_t nflux = static_cast<size_t>(c->nface) * 5 * (c->p + 2) * (c->p + 2);
         if (has_fx && c->nface > 0) {
             if (cudaMalloc((void**)&c->d_faces, faces.size() * sizeof(int2)) != cudaSuccess ||
+                cudaMalloc((void**)&c->d_fdesc, faces.size() * sizeof(dgk::FaceDesc)) != cudaSuccess ||
                 cudaMalloc((void**)&c->d_fflux, nflux * sizeof(double)) != cudaSuccess ||
                 cudaMemcpy(c->d_faces, faces.data(), faces.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess) {
                 cudaGetLastError();
                 cudaFree(c->d_faces);
+                cudaFree(c->d_fdesc);
                 cudaFree(c->d_fflux);
                 c->d_faces = nullptr;
+                c->d_fdesc = nullptr;
                 c->d_fflux = nullptr;
             }
         }
@@ -1278,6 +1309,13 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
     if (!ok) {
         c->err = std::string("table upload failed: ") + cudaGetErrorString(cudaGetLastError());
         return bail(DG_ERR_CUDA);
+    }
+    if (c->d_fdesc) {
+        face_desc_kernel<<<(c->nface + 255) / 256, 256, 0, c->stream>>>(c->d_frec, c->d_faces, c->nface, c->p + 1, c->d_fdesc);
+        if (cudaGetLastError() != cudaSuccess) {
+            c->err = "face descriptor kernel failed";
+            return bail(DG_ERR_CUDA);
+        }
     }
     c->class_dtf.assign(ncls, 1.0);
     c->class_eref.assign(ncls, 0.0);

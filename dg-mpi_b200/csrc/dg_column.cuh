@@ -79,6 +79,12 @@ __device__ __forceinline__ void cta_sync()
     else __syncthreads();
 }
 
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
+{
+    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem_src) : "memory");
+}
+
 // a row of N consecutive doubles (16-byte aligned when N is even)
 template <int N>
 __device__ __forceinline__ void load_row(const double* p, double (&x)[N])
@@ -542,82 +548,128 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
 }
 
 // ---------------------------------------------------------------------------
-// the face kernel with the lift: batches of FB faces as face_flux_body, then
-// L[b1][b0] = sum_t1 C[t1][b1] sum_t0 C[t0][b0] F[t1][t0] (C = B Minv in FP64,
-// B in FP32), one task per (face, variable, output column)
+// the face kernel with the lift, per batch of FB faces:
+//   gather   both sides' boundary slices by cp.async into shared memory, one lane
+//            per slice entry (a warp takes whole sides, so neighbouring lanes read
+//            neighbouring coefficients), while the batch before computes its
+//            fluxes and lifts;
+//   traces   one task per slice (2D interpolation in registers);
+//   flux     one task per point of the listed side's face grid, in the
+//            reference's L/R convention, weighted, over that side's trace;
+//   lift     L[b1][b0] = sum_t1 C[t1][b1] sum_t0 C[t0][b0] F[t1][t0] (C = B Minv
+//            in FP64, B in FP32), one task per (face, variable, output column).
+// Three buffers of face descriptors: the batch's, the next one's (for its
+// gather) and the one after that in flight.
+//
+// Bound by its FP64 chains at 16-18 warps per SM (FP64 pipe 39 %, `wait` the first
+// stall). One thread per slice used to read its 16 strided coefficients, 32
+// cache lines to a load (79 % of the load pipe): 40^3, p = 3, FP64 0.207 -> 0.172
+// ms with the cooperative gather; descriptors, three square roots and one-warp
+// CTAs bring the RK stage of 48^3 from 0.845 to 0.821 ms.
+template <int P, typename T, int FB>
+struct FaceLay {
+    // the cooperative gather pays from p = 3 on; a slice of 4 or 9 coefficients
+    // is read by its trace task itself (p = 1, 72^3, FP64: stage 0.727 against
+    // 0.781 ms; p = 2, 60^3, mixed: 0.774 against 0.835 ms)
+    static constexpr bool COOP = P >= 3;
+    static constexpr int N = P + 1, M = P + 2, NF = M * M, N2 = N * N;
+    static constexpr int FS = odd(NF), NS = odd(N2);       // trace and slice strides
+    static constexpr size_t tr_bytes = (sizeof(T) * FB * 10 * FS + 15) / 16 * 16;
+    static constexpr size_t sl_bytes = COOP ? (sizeof(double) * FB * 10 * NS + 15) / 16 * 16 : 0;
+    static constexpr size_t bytes = tr_bytes + sl_bytes + 3 * FB * sizeof(FaceDesc);
+};
+
 template <int P, typename T, int FB, int NT, int MB>
 __global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant__ StageArgs a)
 {
-    using L = Lay<P, 1, T>;
-    constexpr int N = L::N, M = L::M, NB = L::NB, NF = L::NF, N2 = L::N2, FS = L::FS;
+    using L = FaceLay<P, T, FB>;
+    constexpr int N = L::N, M = L::M, NB = N * N * N, NF = L::NF, N2 = L::N2, FS = L::FS, NS = L::NS;
     constexpr bool kShift = sizeof(T) == 4;
-    extern __shared__ double fsm[];
-    T* sTr = reinterpret_cast<T*>(fsm);                                             // [FB][2][5][FS]
-    unsigned char* tail = reinterpret_cast<unsigned char*>(sTr) + ((sizeof(T) * FB * 10 * FS + 15) / 16) * 16;
-    FaceRec* sRecBuf = reinterpret_cast<FaceRec*>(tail);                            // [2][FB] listed side's records
-    int* sELBuf = reinterpret_cast<int*>(sRecBuf + 2 * FB);                         // [2][FB] listed elements
-    int* sFLBuf = sELBuf + 2 * FB;                                                  // [2][FB] listed faces
+    extern __shared__ __align__(16) unsigned char fraw[];
+    T* sTr = reinterpret_cast<T*>(fraw);                              // [FB][2][5][FS]
+    double* sSl = reinterpret_cast<double*>(fraw + L::tr_bytes);      // [FB][2][5][NS]
+    FaceDesc* sDesc = reinterpret_cast<FaceDesc*>(fraw + L::tr_bytes + L::sl_bytes);  // [3][FB]
     const T* __restrict__ Bt = TabSel<T>::B(a.tab);
     const T* __restrict__ Wt = TabSel<T>::W(a.tab);
     const T* __restrict__ Ct = ColTab<T>::B(a.tab);
     T* out = reinterpret_cast<T*>(a.fflux);
     const int tid = threadIdx.x;
     unsigned status = 0;
-    auto fetch_records = [&](int f, int rb, int2 fe) {
-        if (tid < FB && f < a.nface) {
-            sELBuf[rb * FB + tid] = fe.x;
-            sFLBuf[rb * FB + tid] = fe.y;
-            const double* src = reinterpret_cast<const double*>(a.frec + (size_t)fe.x * 6 + fe.y);
-            double* dst = reinterpret_cast<double*>(sRecBuf + rb * FB + tid);
-#pragma unroll
-            for (int w = 0; w < 6; ++w) cp_async8(dst + w, src + w);
-        }
-        cp_async_commit();
+    const int fstep = gridDim.x * FB;
+    // the descriptors of batch f (the last face repeated past the end)
+    auto fetch = [&](int f, int slot) {
+        if (f < a.nface)
+            for (int i = tid; i < FB * 4; i += NT) {
+                const int j = i / 4, w = i % 4;
+                cp_async16(reinterpret_cast<char*>(sDesc + slot * FB + j) + 16 * w,
+                           reinterpret_cast<const char*>(a.fdesc + min(f + j, a.nface - 1)) + 16 * w);
+            }
     };
-    const int f_first = a.face_begin + blockIdx.x * FB, fstep = gridDim.x * FB;
-    if (f_first < a.nface)
-        fetch_records(f_first, 0, tid < FB ? a.faces[min(f_first + tid, a.nface - 1)] : make_int2(0, 0));
-    int it = 0;
-    for (int f0 = f_first; f0 < a.nface; f0 += fstep, ++it) {
-        const int rb = it & 1;
-        FaceRec* sRecL = sRecBuf + rb * FB;
-        const int* sEL = sELBuf + rb * FB;
-        const int* sFL = sFLBuf + rb * FB;
+    // the slices of batch f, whose descriptors have landed in slot
+    auto gather = [&](int f, int slot) {
+        if (!L::COOP || f >= a.nface) return;
+        for (int sj = tid / 32; sj < 2 * FB; sj += NT / 32) {
+            const FaceDesc& fd = sDesc[slot * FB + sj / 2];
+            const int st = fd.strides >> (16 * (sj % 2)), s0 = st & 255, s1 = (st >> 8) & 255;
+            const double* src = a.Us + fd.base[sj % 2];
+            double* dst = sSl + sj * 5 * NS;
+#pragma unroll
+            for (int r = 0; r < (5 * N2 + 31) / 32; ++r) {
+                const int i = tid % 32 + 32 * r, v = i / N2, c = i - v * N2;
+                if (i < 5 * N2) cp_async8(dst + v * NS + c, src + v * NB + (c % N) * s0 + (c / N) * s1);
+            }
+        }
+    };
+    int f0 = a.face_begin + blockIdx.x * FB;
+    if (f0 < a.nface) {
+        fetch(f0, 0);
+        fetch(f0 + fstep, 1);
+        cp_async_commit();
         cp_async_wait_all();
-        __syncthreads();
-        const int fn = f0 + fstep;
-        const int2 fe_next = tid < FB && fn < a.nface ? a.faces[min(fn + tid, a.nface - 1)] : make_int2(0, 0);
+        cta_sync<NT>();
+        gather(f0, 0);
+        cp_async_commit();
+    }
+    int slot = 0;
+    for (; f0 < a.nface; f0 += fstep) {
+        const FaceDesc* sD = sDesc + slot * FB;
+        const int next = slot == 2 ? 0 : slot + 1, after = next == 2 ? 0 : next + 1;
+        cp_async_wait_all();  // this batch's slices, the next one's descriptors
+        cta_sync<NT>();
+        fetch(f0 + 2 * fstep, after);
+        // traces, both sides in the listed side's energy frame
         for (int t = tid; t < FB * 10; t += NT) {
-            const int v = t % 5, sj = t / 5, j = sj / 2, side = sj % 2;
-            const FaceRec& rec = sRecL[j];
-            const int el = side == 0 ? sEL[j] : rec.nbr;
-            const int fc = side == 0 ? sFL[j] : (rec.info & 7);
-            const int ax = face_axis(fc), sidx = face_side(fc) ? N - 1 : 0;
-            const int o0 = ax == 0 ? sidx : (ax == 1 ? sidx * N : sidx * N2);
-            const int s0 = ax == 0 ? N : 1, s1 = ax == 2 ? N : N2;
-            const double* src = a.Us + ((size_t)el * 5 + v) * NB + o0;
-            const double sh = kShift && v == 4 ? a.geo[rec.cls].eref : 0.0;
+            const FaceDesc& fd = sD[t / 10];
+            const double sh = kShift && t % 5 == 4 ? a.geo[fd.cls].eref : 0.0;
+            const double* s = sSl + t * NS;
+            int s0 = 1, s1 = N;
+            if constexpr (!L::COOP) {
+                const int side = (t / 5) % 2, st = fd.strides >> (16 * side);
+                s = a.Us + fd.base[side] + (t % 5) * NB;
+                s0 = st & 255;
+                s1 = (st >> 8) & 255;
+            }
             double x[N][N];
 #pragma unroll
             for (int b1 = 0; b1 < N; ++b1)
 #pragma unroll
-                for (int b0 = 0; b0 < N; ++b0) x[b1][b0] = __ldg(src + b0 * s0 + b1 * s1);
+                for (int b0 = 0; b0 < N; ++b0) x[b1][b0] = s[b0 * s0 + b1 * s1];
             T sl[N][N];
 #pragma unroll
             for (int b1 = 0; b1 < N; ++b1)
 #pragma unroll
                 for (int b0 = 0; b0 < N; ++b0) sl[b1][b0] = kShift ? T(x[b1][b0] - sh) : T(x[b1][b0]);
-            interp2d<N, M, T>(Bt, sl, sTr + (sj * 5 + v) * FS);
+            interp2d<N, M, T>(Bt, sl, sTr + t * FS);
         }
-        fetch_records(fn, rb ^ 1, fe_next);
-        __syncthreads();
-        // the flux at the listed side's face points, over that side's trace
+        cta_sync<NT>();
+        gather(f0 + fstep, next);
+        cp_async_commit();
         for (int i = tid; i < FB * NF; i += NT) {
             const int c = i % NF, j = i / NF;
             if (f0 + j >= a.nface) continue;
-            const FaceRec& rec = sRecL[j];
-            const int cn = a.cmap[(rec.info >> 4) * NF + c];
-            const int isL = (rec.info >> 3) & 1;
+            const FaceDesc& fd = sD[j];
+            const int cn = a.cmap[(fd.info >> 4) * NF + c];
+            const int isL = (fd.info >> 3) & 1;
             T* To = sTr + (j * 2) * 5 * FS;
             const T* Tn = To + 5 * FS;
             T UL[5], UR[5], Fo[5];
@@ -627,14 +679,15 @@ __global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant
                 UL[v] = isL ? uo : un;
                 UR[v] = isL ? un : uo;
             }
-            const T nd[4] = {T(rec.n[0]), T(rec.n[1]), T(rec.n[2]), T(rec.nmag)};
-            const double eref = kShift ? a.geo[rec.cls].eref : 0.0;
-            numerical_flux<T, kShift>(a.flux, a.gamma, UL, UR, nd, eref, Fo, status);
+            const T nd[4] = {T(fd.n[0]), T(fd.n[1]), T(fd.n[2]), T(fd.nmag)};
+            const double eref = kShift ? a.geo[fd.cls].eref : 0.0;
+            if (!kShift && a.flux == 0) dgp::flux_lax_friedrichs_sq(T(a.gamma), UL, UR, nd, nd[3], Fo);
+            else numerical_flux<T, kShift>(a.flux, a.gamma, UL, UR, nd, eref, Fo, status);
             const T w = Wt[c % M] * Wt[c / M];
 #pragma unroll
             for (int v = 0; v < 5; ++v) To[v * FS + c] = Fo[v] * w;
         }
-        __syncthreads();
+        cta_sync<NT>();
         for (int t = tid; t < FB * 5 * N; t += NT) {
             const int b0 = t % N, jv = t / N, v = jv % 5, j = jv / 5;
             if (f0 + j >= a.nface) continue;
@@ -656,15 +709,10 @@ __global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant
                 o[b1 * N] = s;
             }
         }
+        slot = next;
     }
     cp_async_wait_all();
     if (status) atomicOr(a.status, status);
-}
-
-template <int P, typename T, int FB>
-constexpr size_t face_lift_smem_bytes()
-{
-    return ((sizeof(T) * FB * 10 * Lay<P, 1, T>::FS + 15) / 16) * 16 + 2 * FB * sizeof(FaceRec) + 4 * FB * sizeof(int);
 }
 
 template <int P, int E, int NT, typename T, int MB>
@@ -676,22 +724,26 @@ cudaError_t launch_column(const StageArgs& a, int grid, cudaStream_t s)
 template <int P, typename T, int FB, int NT, int MB>
 cudaError_t launch_face_lift(const StageArgs& a, int grid, cudaStream_t s)
 {
-    face_lift_kernel<P, T, FB, NT, MB><<<grid, NT, face_lift_smem_bytes<P, T, FB>(), s>>>(a);
+    face_lift_kernel<P, T, FB, NT, MB><<<grid, NT, FaceLay<P, T, FB>::bytes, s>>>(a);
     return cudaGetLastError();
 }
 
 // E elements and NT threads per CTA, at least MB resident CTAs per SM asked of the
 // compiler; the default from min_per_sm elements per SM on (below, the stage
 // kernel's many threads per element finish sooner than one warp per element)
-template <int P, int E, int NT, typename T, int MB>
+// The face kernel's batch FB on FNT threads (FMB resident CTAs asked of the
+// compiler) is the measured best of batches of 2 .. 20 faces on 32 .. 256 threads:
+// small CTAs, whose barriers hold few warps, as long as one round of threads
+// covers most of the slices and points.
+template <int P, int E, int NT, typename T, int MB, int FB, int FNT, int FMB>
 StageVariant make_column_variant(int min_per_sm)
 {
     static_assert(ColLay<P, T>::bytes(E) <= 227 * 1024, "column kernel shared memory exceeds 227 KB");
-    constexpr int FB = face_batch<P, T>(), FNT = face_threads<P, T>(), FMB = 1;
+    static_assert(FaceLay<P, T, FB>::bytes <= 227 * 1024, "face kernel shared memory exceeds 227 KB");
     StageVariant v{E, NT, 1, sizeof(T) == 4 ? 1 : 0, kSB | kFX | kCF, ColLay<P, T>::bytes(E),
                    (const void*)column_kernel<P, E, NT, T, MB>, launch_column<P, E, NT, T, MB>, nullptr, 0, 0, nullptr, 0, min_per_sm};
     v.face_func = (const void*)face_lift_kernel<P, T, FB, FNT, FMB>;
-    v.face_smem = face_lift_smem_bytes<P, T, FB>();
+    v.face_smem = FaceLay<P, T, FB>::bytes;
     v.face_threads = FNT;
     v.face_launch = launch_face_lift<P, T, FB, FNT, FMB>;
     v.face_batch = FB;

@@ -157,6 +157,32 @@ DG_HD void flux_lax_friedrichs_fast(T gamma, const T* UL, const T* UR, const T* 
     for (int s = 0; s < 5; ++s) F[s] = n_mag * (T(0.5) * (FnL[s] + FnR[s]) - T(0.5) * a * (UR[s] - UL[s]));
 }
 
+// flux_lax_friedrichs_fast in three square roots instead of four: the larger
+// wave speed is picked by its square, (u + c)^2 = u^2 + c^2 + 2 sqrt(u^2 c^2),
+// and rooted once.  FP64 (a square root is 13 of an FP64 lane's multiply-adds).
+template <typename T>
+DG_HD void flux_lax_friedrichs_sq(T gamma, const T* UL, const T* UR, const T* n_hat, T n_mag, T* F)
+{
+    T Fn[2][5], a2[2];
+    for (int k = 0; k < 2; ++k) {
+        const T* U = k ? UR : UL;
+        const T r1 = T(1.) / U[0];
+        const T m2 = U[1] * U[1] + U[2] * U[2] + U[3] * U[3];
+        const T P = (gamma - T(1.0)) * (U[4] - T(0.5) * (m2 * r1));
+        const T mn = U[1] * n_hat[0] + U[2] * n_hat[1] + U[3] * n_hat[2];
+        const T vn = mn * r1;
+        Fn[k][0] = mn;
+        Fn[k][1] = U[1] * vn + P * n_hat[0];
+        Fn[k][2] = U[2] * vn + P * n_hat[1];
+        Fn[k][3] = U[3] * vn + P * n_hat[2];
+        Fn[k][4] = (U[4] + P) * vn;
+        const T u2 = m2 * r1 * r1, c2 = gamma * P * r1;
+        a2[k] = u2 + c2 + T(2.0) * sqrt(u2 * c2);
+    }
+    const T a = sqrt(a2[1] > a2[0] ? a2[1] : a2[0]);
+    for (int s = 0; s < 5; ++s) F[s] = n_mag * (T(0.5) * (Fn[0][s] + Fn[1][s]) - T(0.5) * a * (UR[s] - UL[s]));
+}
+
 // Lax-Friedrichs with the face's normal data precomputed (it is constant on a
 // face of an affine element): n_mag = |N| and n_hat = N / n_mag, evaluated
 // once on the host by the formulas of flux_lax_friedrichs.

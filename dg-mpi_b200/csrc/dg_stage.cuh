@@ -100,6 +100,23 @@ struct FaceRec {
 };
 static_assert(sizeof(FaceRec) == 48, "FaceRec is six 8-byte words");
 
+// One face of the face list for the column form's face kernel (64 bytes, built
+// on the device from the face records): the left element's normal data, each
+// side's boundary slice of the state -- entry (b0, b1) of the listed side (0) and
+// of the other one at base[side] + v (p+1)^3 + b0 s0 + b1 s1, the strides one
+// byte each: side 0's s0, s1, then side 1's --, the listed side's info word and
+// geometry class.
+struct FaceDesc {
+    double n[3];
+    double nmag;
+    long long base[2];
+    unsigned strides;
+    int info;
+    int cls;
+    int pad;
+};
+static_assert(sizeof(FaceDesc) == 64, "FaceDesc is four 16-byte words");
+
 enum StageMode : int {
     kModeResidual = 0,  // out = R(Us)
     kModeMassInv = 1,   // out = dt * M^-1 R(Us)
@@ -147,6 +164,7 @@ struct StageArgs {
     // face-kernel launch computes, and the fluxes [nface][5][(p+2)^2] (T
     // values, weights applied, unsigned)
     const int2* faces;
+    const FaceDesc* fdesc;  // [nface], the column form's face list
     int face_begin, nface;
     void* fflux;
     int fstride;            // elements per face in fflux: 5 (p+2)^2, or padded to a 16-byte multiple (TC)

@@ -12,7 +12,7 @@
 namespace dgk {
 
 static const StageVariant kVariants2[] = {
-    make_column_variant<2, 2, 32, double, 11>(6),
+    make_column_variant<2, 2, 32, double, 11, 6, 32, 1>(6),
     make_variant<2, 1, 32, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<2, 2, 64, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<2, 1, 32, 1, double, kUF | kSB | kFX>(),
@@ -22,7 +22,7 @@ static const StageVariant kVariants2[] = {
     make_variant<2, 2, 64, 1, double, kUF | kRS | kSB>(),
     make_variant<2, 1, 32, 1, double>(),
     make_variant<2, 2, 64, 1, double>(),
-    make_column_variant<2, 2, 32, float, 16>(16),
+    make_column_variant<2, 2, 32, float, 16, 8, 128, 1>(16),
     make_variant<2, 1, 32, 1, float, kUF | kSB | kFX | kMG>(),
     make_variant<2, 2, 64, 1, float, kUF | kSB | kFX | kMG>(),
     make_variant<2, 1, 32, 1, float, kUF | kSB | kFX>(),

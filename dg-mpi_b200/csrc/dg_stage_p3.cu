@@ -13,7 +13,7 @@
 namespace dgk {
 
 static const StageVariant kVariants3[] = {
-    make_column_variant<3, 1, 32, double, 12>(6),
+    make_column_variant<3, 1, 32, double, 12, 3, 32, 1>(6),
     make_variant<3, 1, 96, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<3, 1, 128, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<3, 1, 128, 1, double, kUF | kRS | kSB | kFX | kMG>(),
@@ -29,7 +29,7 @@ static const StageVariant kVariants3[] = {
     make_variant<3, 1, 64, 1, double, kUF | kSB | kK1>(),
     make_variant<3, 1, 32, 2, double, kSB>(),
     make_variant<3, 2, 64, 2, double>(),
-    make_column_variant<3, 1, 32, float, 16>(10),
+    make_column_variant<3, 1, 32, float, 16, 5, 64, 1>(10),
     make_variant<3, 1, 128, 1, float, kUF | kSB | kFX | kMG>(),
     make_variant<3, 1, 128, 1, float, kUF | kRS | kSB | kFX | kMG>(),
     make_variant<3, 1, 64, 1, float, kUF | kSB | kFX | kMG>(),

@@ -12,7 +12,7 @@
 namespace dgk {
 
 static const StageVariant kVariants4[] = {
-    make_column_variant<4, 1, 64, double, 5>(3),
+    make_column_variant<4, 1, 64, double, 5, 5, 64, 1>(3),
     make_variant<4, 1, 128, 1, double, kUF | kSB | kFX | kMG, 4>(),
     make_variant<4, 1, 96, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<4, 1, 128, 1, double, kUF | kSB | kFX, 4>(),
@@ -25,7 +25,7 @@ static const StageVariant kVariants4[] = {
     make_variant<4, 1, 128, 1, double, kUF | kRS | kSB | kK1>(),
     make_variant<4, 1, 96, 1, double, kUF | kRS | kSB | kK1>(),
     make_variant<4, 1, 64, 2, double>(),
-    make_column_variant<4, 1, 64, float, 8>(6),
+    make_column_variant<4, 1, 64, float, 8, 5, 64, 1>(6),
     make_variant<4, 1, 128, 1, float, kUF | kSB | kFX | kMG>(),
     make_variant<4, 1, 128, 1, float, kUF | kRS | kSB | kFX | kMG>(),
     make_variant<4, 1, 128, 1, float, kUF | kSB | kFX>(),

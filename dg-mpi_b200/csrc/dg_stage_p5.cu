@@ -12,7 +12,7 @@
 namespace dgk {
 
 static const StageVariant kVariants5[] = {
-    make_column_variant<5, 1, 64, double, 4>(3),
+    make_column_variant<5, 1, 64, double, 4, 5, 64, 1>(3),
     make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kFX | kMG, 2>(),
     make_variant<5, 1, 192, 1, double, kUF | kRS | kSB | kFX | kMG>(),
     make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kFX, 2>(),
@@ -21,7 +21,7 @@ static const StageVariant kVariants5[] = {
     make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kK1, 2>(),
     make_variant<5, 1, 128, 1, double, kUF | kRS | kSB | kK1>(),
     make_variant<5, 1, 128, 3, double>(),
-    make_column_variant<5, 1, 64, float, 6>(6),
+    make_column_variant<5, 1, 64, float, 6, 8, 128, 1>(6),
     make_variant<5, 1, 256, 1, float, kUF | kSB | kFX | kMG, 3>(),
     make_variant<5, 1, 256, 1, float, kUF | kRS | kSB | kFX | kMG, 3>(),
     make_variant<5, 1, 256, 1, float, kUF | kRS | kSB | kFX, 3>(),
