@@ -179,6 +179,7 @@ void stage_args(const dg_ctx* c, int mode, const double* Us, const double* U0, d
     a.gfsd = c->d_gfsd;
     a.faces = c->d_faces;
     a.fdesc = c->d_fdesc;
+    a.lrec = c->d_lrec;
     a.nface = c->nface;
     a.fflux = c->d_fflux;
     a.fstride = 5 * (c->p + 2) * (c->p + 2);
@@ -201,6 +202,10 @@ void stage_args(const dg_ctx* c, int mode, const double* Us, const double* U0, d
         if (mode == dgk::kModeResidual) {
             std::memcpy(a.tab.MB, a.tab.B, sizeof(a.tab.MB));
             std::memcpy(a.tab.MD, a.tab.D, sizeof(a.tab.MD));
+            for (int b = 0; b <= c->p; ++b) {
+                a.tab.ME[0][b] = b == 0 ? 1.0 : 0.0;
+                a.tab.ME[1][b] = b == c->p ? 1.0 : 0.0;
+            }
         }
     }
 }
@@ -318,6 +323,22 @@ __global__ void face_desc_kernel(const dgk::FaceRec* __restrict__ frec, const in
     d.cls = r.cls;
     d.pad = 0;
     out[i] = d;
+}
+
+// the element-to-face records (see dgk::StageArgs::lrec): a side whose node
+// permutation is the identity reads the lifts in the stored order too
+__global__ void lift_record_kernel(const dgk::FaceRec* __restrict__ frec, const uint8_t* __restrict__ cmapn, int nrec, int n,
+                                   int* __restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nrec) return;
+    const int pad = frec[i].pad, info = frec[i].info;
+    bool own = (pad >> 30) & 1;
+    if (!own) {
+        own = true;
+        for (int c = 0; c < n * n; ++c) own = own && cmapn[(info >> 4) * n * n + c] == c;
+    }
+    out[i] = (pad & 0x3fffffff) | (own ? 1 << 30 : 0) | (((info >> 3) & 1) ? (int)0x80000000u : 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -943,7 +964,7 @@ void release(dg_ctx* c)
     cudaFree(c->d_conn); cudaFree(c->d_frec); cudaFree(c->d_geo_class); cudaFree(c->d_geo); cudaFree(c->d_cmap);
     cudaFree(c->d_X0); cudaFree(c->d_partials); cudaFree(c->d_status);
     cudaFree(c->d_gjd); cudaFree(c->d_gnrm); cudaFree(c->d_gimm); cudaFree(c->d_gnodes); cudaFree(c->d_gfsd);
-    cudaFree(c->d_faces); cudaFree(c->d_fdesc); cudaFree(c->d_fflux); cudaFree(c->d_tcop);
+    cudaFree(c->d_faces); cudaFree(c->d_fflux); cudaFree(c->d_tcop);
     cudaFree(c->d_halo_send); cudaFree(c->d_halo_recv);
     for (cudaEvent_t e : c->chunk_ev) cudaEventDestroy(e);
     c->chunk_ev.clear();
@@ -1040,6 +1061,10 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
     for (size_t i = 0; i < c->tab.wq.size(); ++i) c->stage_tab.Wf[i] = static_cast<float>(c->tab.wq[i]);
     {   // the 1D inverse mass folded into the contraction tables: MB[q][b] = sum_k B[q][k] Minv[b][k]
         const int n = c->p + 1;
+        for (int b = 0; b < n; ++b) {
+            c->stage_tab.ME[0][b] = c->tab.Minv[b * n];
+            c->stage_tab.ME[1][b] = c->tab.Minv[b * n + n - 1];
+        }
         for (int q = 0; q < c->p + 2; ++q)
             for (int b = 0; b < n; ++b) {
                 long double sb = 0.0L, sd = 0.0L;
@@ -1253,17 +1278,19 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
         for (int v = 0; v < nv; ++v) has_fx = has_fx || (vs[v].flags & dgk::kFX);
         const size_t nflux = static_cast<size_t>(c->nface) * 5 * (c->p + 2) * (c->p + 2);
         if (has_fx && c->nface > 0) {
+            const size_t flux_bytes = (nflux * sizeof(double) + 255) / 256 * 256;
+            const size_t desc_bytes = faces.size() * sizeof(dgk::FaceDesc), lrec_bytes = static_cast<size_t>(c->ne) * 6 * sizeof(int);
             if (cudaMalloc((void**)&c->d_faces, faces.size() * sizeof(int2)) != cudaSuccess ||
-                cudaMalloc((void**)&c->d_fdesc, faces.size() * sizeof(dgk::FaceDesc)) != cudaSuccess ||
-                cudaMalloc((void**)&c->d_fflux, nflux * sizeof(double)) != cudaSuccess ||
+                cudaMalloc((void**)&c->d_fflux, flux_bytes + desc_bytes + lrec_bytes) != cudaSuccess ||
                 cudaMemcpy(c->d_faces, faces.data(), faces.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess) {
                 cudaGetLastError();
                 cudaFree(c->d_faces);
-                cudaFree(c->d_fdesc);
                 cudaFree(c->d_fflux);
                 c->d_faces = nullptr;
-                c->d_fdesc = nullptr;
                 c->d_fflux = nullptr;
+            } else {
+                c->d_fdesc = reinterpret_cast<dgk::FaceDesc*>(reinterpret_cast<char*>(c->d_fflux) + flux_bytes);
+                c->d_lrec = reinterpret_cast<int*>(c->d_fdesc + faces.size());
             }
         }
         // the tensor-core variants' operator table (FP32 residual on affine meshes)
@@ -1312,6 +1339,7 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
     }
     if (c->d_fdesc) {
         face_desc_kernel<<<(c->nface + 255) / 256, 256, 0, c->stream>>>(c->d_frec, c->d_faces, c->nface, c->p + 1, c->d_fdesc);
+        lift_record_kernel<<<(c->ne * 6 + 255) / 256, 256, 0, c->stream>>>(c->d_frec, c->d_cmapn, c->ne * 6, c->p + 1, c->d_lrec);
         if (cudaGetLastError() != cudaSuccess) {
             c->err = "face descriptor kernel failed";
             return bail(DG_ERR_CUDA);

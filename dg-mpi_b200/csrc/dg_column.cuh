@@ -30,12 +30,17 @@
 // memory between up to nine block barriers per element, and waits on them
 // (40^3, p = 3, FP64: 5140 warp instructions and 1640 shared wavefronts per
 // element, FP64 pipe 40 %, `barrier` the first stall).  Here a warp owns its
-// elements (no block barriers up to p = 3), 2610 instructions per element, the
-// column phase keeping 27 of the point array's 45 words in registers.  RK stage
-// (both kernels), stage kernel -> column form, GDOF/s: FP64 11.7 -> 20.5 (72^3,
-// p = 1), 24.5 -> 31.5 (60^3, p = 2), 31.9 -> 38.5 (48^3, p = 3), 30.2 -> 37.3
-// (40^3, p = 4), 31.9 -> 37.7 (32^3, p = 5); mixed 19.4 -> 26.3, 33.0 -> 37.7,
-// 39.7 -> 42.2, 44.0 -> 45.9, 41.8 -> 43.7.
+// elements (no block barriers up to p = 3), about 2500 instructions per element,
+// the column phase keeping 27 of the point array's 45 words in registers.  The
+// next batch's rows and face records wait in registers during the contractions
+// (reading them at the batch's top left long_scoreboard the first stall: 48^3,
+// p = 3, RK stage 0.821 -> 0.722 ms FP64, 0.769 -> 0.695 ms mixed); 12 warps per
+// SM at 168 registers beat 8 at 255 (0.777 ms) there, at p = 4 and 5 the other
+// way round (40^3, p = 4: 0.970 against 1.037 ms).  RK stage (both kernels), stage kernel
+// -> column form, GDOF/s: FP64 11.7 -> 24.4 (72^3, p = 1), 24.5 -> 39.7 (60^3,
+// p = 2), 31.9 -> 49.0 (48^3, p = 3), 30.2 -> 41.3 (40^3, p = 4), 31.9 -> 42.6
+// (32^3, p = 5); mixed 19.4 -> 29.8, 33.0 -> 44.2, 39.7 -> 50.9, 44.0 -> 49.8,
+// 41.8 -> 49.9.
 #pragma once
 #include "dg_stage.cuh"
 
@@ -121,6 +126,18 @@ __device__ __forceinline__ void prefetch_l2(const double* p, int n)
     if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(g & ~15ull), "r"(bytes) : "memory");
 }
 
+// x, in a way the compiler does not see through: index arithmetic on it is redone
+// in every iteration of the batch loop instead of being kept in registers across
+// the column phase, which needs them
+// (FP64 from p = 4 on, where it is short of registers: p = 4, eight warps, 88 B of
+// spills without it)
+template <bool ON>
+__device__ __forceinline__ int opaque(int x)
+{
+    if constexpr (ON) asm volatile("" : "+r"(x));
+    return x;
+}
+
 // contraction tables: with the inverse mass folded in (FP64), or the plain ones
 template <typename T> struct ColTab;
 template <> struct ColTab<double> {
@@ -168,60 +185,87 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
     const T* __restrict__ Ct = ColTab<T>::B(a.tab);
     const T* __restrict__ Dt = ColTab<T>::D(a.tab);
     const double* __restrict__ Mi = a.tab.Minv;
-    const int tid = threadIdx.x;
+    const int tid0 = threadIdx.x;
     const T gamma = T(a.gamma);
     const int mode = a.mode;
     const bool need_u0 = mode >= kModeRK1, need_acc = mode == kModeRK2 || mode == kModeRK3 || mode == kModeRK4;
     unsigned status = 0;
-    // spread of a face's lift along its normal: the end columns of the 1D inverse
-    // mass, or of the identity for the residual output
-    if (tid < 2 * N) {
-        const int b = tid % N, end = tid < N ? 0 : N - 1;
-        sM[tid] = mode == kModeResidual ? (b == end ? 1.0 : 0.0) : Mi[b * N + end];
-    }
+    if (tid0 < 2 * N) sM[tid0] = a.tab.ME[tid0 / N][tid0 % N];
 
+    // the next batch's coefficient rows and face records, fetched while this batch contracts
+    constexpr int R = (ROWS + NT - 1) / NT, LT = E * 6 * N2, RL = (LT + NT - 1) / NT;
+    double un[R][N];
+    int cl[R], fl[RL];
+    auto fetch = [&](int e0) {
+        const int tid = opaque<F64 && P >= 4>(tid0);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = tid + r * NT;
+            if (i < ROWS) {
+                const int e = i / (5 * N2), row = i - e * (5 * N2), ge = min(e0 + e, a.ne - 1);
+                load_row<N>(a.Us + ((size_t)ge * 5 * N2 + row) * N, un[r]);
+                if constexpr (kShift) cl[r] = a.geo_class[ge];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < RL; ++r) {
+            const int i = tid + r * NT;
+            if (i < LT) {
+                const int f = (i / N2) % 6, e = i / (6 * N2);
+                fl[r] = a.lrec[(size_t)min(e0 + e, a.ne - 1) * 6 + f];
+            }
+        }
+    };
     const int stride = gridDim.x * E;
-    for (int e0 = a.e_begin + blockIdx.x * E; e0 < a.ne; e0 += stride) {
-        // the next batch's rows and RK operands on their way into L2
-        if (tid < 3 && e0 + stride < a.ne && (tid == 0 || (tid == 1 ? need_u0 && a.U0 != a.Us : need_acc)))
-            prefetch_l2((tid == 0 ? a.Us : tid == 1 ? a.U0 : a.acc) + (size_t)(e0 + stride) * 5 * NB,
-                        min(E, a.ne - e0 - stride) * 5 * NB);
+    int e0 = a.e_begin + blockIdx.x * E;
+    if (e0 < a.ne) fetch(e0);
+    for (; e0 < a.ne; e0 += stride) {
+        // this batch's RK operands (read by the last pass) and the next batch's rows on
+        // their way into L2
+        if (tid0 < 3 && (tid0 == 0 ? e0 + stride < a.ne : tid0 == 1 ? need_u0 && a.U0 != a.Us : need_acc)) {
+            const int ep = tid0 == 0 ? e0 + stride : e0;
+            prefetch_l2((tid0 == 0 ? a.Us : tid0 == 1 ? a.U0 : a.acc) + (size_t)ep * 5 * NB, min(E, a.ne - ep) * 5 * NB);
+        }
         // ---- this batch's face lifts stream in (used by the last pass) ----
         {
             const T* gL = reinterpret_cast<const T*>(a.fflux);
-#pragma unroll 1
-            for (int i = tid; i < E * 6 * N2; i += NT) {
-                const int c = i % N2, f = (i / N2) % 6, e = i / (6 * N2);
-                // the second half of the face record: neighbour, info, class, listed face
-                const int4 fr = *(reinterpret_cast<const int4*>(a.frec + (size_t)min(e0 + e, a.ne - 1) * 6 + f) + 2);
-                const int pc = ((fr.w >> 30) & 1) ? c : a.cmapn[(fr.y >> 4) * N2 + c];
-                const T* src = gL + (size_t)(fr.w & 0x3fffffff) * a.fstride + pc;
-                T* dst = sL + e * L::LF + f * 5 * N2 + c;
+            const int tid = opaque<F64 && P >= 4>(tid0);
 #pragma unroll
-                for (int v = 0; v < 5; ++v) cp_async_t(dst + v * N2, src + v * N2);
-                if (c == 0) sSgn[e * 6 + f] = ((fr.y >> 3) & 1) ? T(-1) : T(1);
-                if (c == 0 && f == 0) sCls[e] = fr.z;
+            for (int r = 0; r < RL; ++r) {
+                const int i = tid + r * NT;
+                if (i < LT) {
+                    const int c = i % N2, f = (i / N2) % 6, e = i / (6 * N2);
+                    const int ge = min(e0 + e, a.ne - 1);
+                    const int pc = ((fl[r] >> 30) & 1) ? c : a.cmapn[(a.frec[(size_t)ge * 6 + f].info >> 4) * N2 + c];
+                    const T* src = gL + (size_t)(fl[r] & 0x3fffffff) * a.fstride + pc;
+                    T* dst = sL + e * L::LF + f * 5 * N2 + c;
+#pragma unroll
+                    for (int v = 0; v < 5; ++v) cp_async_t(dst + v * N2, src + v * N2);
+                    if (c == 0) sSgn[e * 6 + f] = fl[r] < 0 ? T(-1) : T(1);
+                }
             }
+            for (int e = tid; e < E; e += NT) sCls[e] = a.geo_class[min(e0 + e, a.ne - 1)];
             cp_async_commit();
         }
         // ---- x interpolation ----
-#pragma unroll 1
-        for (int i = tid; i < ROWS; i += NT) {
-            const int e = i / (5 * N2), row = i - e * (5 * N2), v = row / N2, byz = row - v * N2;
-            const int ge = min(e0 + e, a.ne - 1);
-            double ur[N];
-            load_row<N>(a.Us + ((size_t)ge * 5 * N2 + row) * N, ur);
-            const double sh = kShift && v == 4 ? a.geo[a.geo_class[ge]].eref : 0.0;
-            T u[N];
+        const int tid = opaque<F64 && P >= 4>(tid0);
 #pragma unroll
-            for (int b = 0; b < N; ++b) u[b] = kShift ? T(ur[b] - sh) : T(ur[b]);
-            T* o = sW + e * W + 5 * AS + v * X1S + byz * M;
+        for (int r = 0; r < R; ++r) {
+            const int i = tid + r * NT;
+            if (i < ROWS) {
+                const int e = i / (5 * N2), row = i - e * (5 * N2), v = row / N2, byz = row - v * N2;
+                const double sh = kShift && v == 4 ? a.geo[cl[r]].eref : 0.0;
+                T u[N];
 #pragma unroll
-            for (int q = 0; q < M; ++q) {
-                T s = T(0);
+                for (int b = 0; b < N; ++b) u[b] = kShift ? T(un[r][b] - sh) : T(un[r][b]);
+                T* o = sW + e * W + 5 * AS + v * X1S + byz * M;
 #pragma unroll
-                for (int b = 0; b < N; ++b) s += sym<M * N>(Bt, q * N + b) * u[b];
-                o[q] = s;
+                for (int q = 0; q < M; ++q) {
+                    T s = T(0);
+#pragma unroll
+                    for (int b = 0; b < N; ++b) s += sym<M * N>(Bt, q * N + b) * u[b];
+                    o[q] = s;
+                }
             }
         }
         cta_sync<NT>();
@@ -355,6 +399,7 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
             }
         }
         cta_sync<NT>();
+        fetch(e0 + stride);  // past the end: the last element again (a condition would keep the old rows alive)
         // ---- y contraction: By^T A0 over row 3v, Dy^T A1 + By^T A2 over row 3v+1 ----
 #pragma unroll 1
         for (int i = tid; i < E * 5 * N * M; i += NT) {
@@ -418,8 +463,8 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
 #pragma unroll
                 for (int b = 0; b < N; ++b) {
                     double s = x[b];
-                    s += sM[b] * l4;
-                    s += sM[N + b] * l2;
+                    s += a.tab.ME[0][b] * l4;
+                    s += a.tab.ME[1][b] * l2;
                     s += c1 * L1[b];
                     s += c3 * L3[b];
                     s += c0 * L0[b];

@@ -59,6 +59,9 @@ struct StageTables {
     // 1D mass matrix (or B and D themselves for the residual output)
     double MB[kTabB];
     double MD[kTabB];
+    // first and last column of the inverse 1D mass matrix (of the identity for
+    // the residual output): the spread of a face's lift along its normal
+    double ME[2][kMaxP + 1];
 };
 
 template <typename T> struct TabSel;
@@ -165,6 +168,7 @@ struct StageArgs {
     // values, weights applied, unsigned)
     const int2* faces;
     const FaceDesc* fdesc;  // [nface], the column form's face list
+    const int* lrec;        // [ne][6] face | 1 << 30 where its lift is read in its own node order | 1 << 31 on the left side
     int face_begin, nface;
     void* fflux;
     int fstride;            // elements per face in fflux: 5 (p+2)^2, or padded to a 16-byte multiple (TC)

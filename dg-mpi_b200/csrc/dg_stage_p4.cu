@@ -12,7 +12,7 @@
 namespace dgk {
 
 static const StageVariant kVariants4[] = {
-    make_column_variant<4, 1, 64, double, 5, 5, 64, 1>(3),
+    make_column_variant<4, 1, 64, double, 4, 5, 64, 1>(3),
     make_variant<4, 1, 128, 1, double, kUF | kSB | kFX | kMG, 4>(),
     make_variant<4, 1, 96, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<4, 1, 128, 1, double, kUF | kSB | kFX, 4>(),
