@@ -37,10 +37,12 @@
 // p = 3, RK stage 0.821 -> 0.722 ms FP64, 0.769 -> 0.695 ms mixed); 12 warps per
 // SM at 168 registers beat 8 at 255 (0.777 ms) there, at p = 4 and 5 the other
 // way round (40^3, p = 4: 0.970 against 1.037 ms).  RK stage (both kernels), stage kernel
-// -> column form, GDOF/s: FP64 11.7 -> 24.4 (72^3, p = 1), 24.5 -> 39.7 (60^3,
-// p = 2), 31.9 -> 49.0 (48^3, p = 3), 30.2 -> 41.3 (40^3, p = 4), 31.9 -> 42.6
-// (32^3, p = 5); mixed 19.4 -> 29.8, 33.0 -> 44.2, 39.7 -> 50.9, 44.0 -> 49.8,
-// 41.8 -> 49.9.
+// -> column form, GDOF/s: FP64 11.7 -> 24.4 (72^3, p = 1), 24.5 -> 39.0 (60^3,
+// p = 2), 31.9 -> 49.4 (48^3, p = 3), 30.2 -> 41.0 (40^3, p = 4), 31.9 -> 42.6
+// (32^3, p = 5); mixed 19.4 -> 29.6, 33.0 -> 44.6, 39.7 -> 55.2, 44.0 -> 52.3,
+// 41.8 -> 53.4.  The FP32 form is bound by instruction issue (3000 per element at
+// p = 3, 64 % of the issue slots): its lift sums take one y and one z face per row
+// and its residual block has constant strides (48^3, p = 3: 0.695 -> 0.641 ms).
 #pragma once
 #include "dg_stage.cuh"
 
@@ -69,7 +71,10 @@ struct ColLay {
     static constexpr int oyc = W8 ? (P == 3 || P == 4 ? 11 : 21) : (P == 1 ? 21 : P == 2 ? 15 : P == 4 ? 11 : 19);
     static_assert(PS >= NF && AS >= (N - 1) * PS + NF && 10 * AS >= 5 * X1S, "point-array rows overlap");
     static constexpr int W = 15 * AS;                     // point array, T
-    static constexpr int VS = odd(NB);                    // FP32 path: residual block stride, FP64
+    // FP32 path: the FP64 residual block, entry (bx, by, bz) at bz SZ + by SY + bx:
+    // x, y and z pencils of a variable fall on distinct bank pairs but for a few
+    // (N = 4: SY = 5, SZ = 20) and their words are constant offsets apart
+    static constexpr int SY = N % 2 ? N : N + 1, SZ = N * SY, VS = N * SZ;
     static constexpr int RES = W8 ? 0 : 5 * VS;           // FP64 residual of the FP32 path
     static constexpr int LF = 30 * N2;                    // the six faces' lifts, T
     static constexpr size_t f64_words(int E) { return static_cast<size_t>(E) * RES + 2 * N; }
@@ -169,7 +174,7 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
 {
     using L = ColLay<P, T>;
     constexpr int N = L::N, M = L::M, NB = L::NB, NF = L::NF, N2 = L::N2;
-    constexpr int PS = L::PS, AS = L::AS, X1S = L::X1S, W = L::W, VS = L::VS;
+    constexpr int PS = L::PS, AS = L::AS, X1S = L::X1S, W = L::W, VS = L::VS, SY = L::SY, SZ = L::SZ;
     constexpr bool F64 = sizeof(T) == 8;
     constexpr bool kShift = !F64;
     constexpr int ROWS = E * 5 * N2;                   // coefficient rows along x of a batch
@@ -189,6 +194,11 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
     const T gamma = T(a.gamma);
     const int mode = a.mode;
     const bool need_u0 = mode >= kModeRK1, need_acc = mode == kModeRK2 || mode == kModeRK3 || mode == kModeRK4;
+    // the update: out = U0 + cu (acc + k in the last stage, else k), acc' = acc + ca k,
+    // with U0 and acc zero where the mode does not read them
+    const bool put_acc = mode == kModeRK1 || mode == kModeRK2 || mode == kModeRK3, sum_acc = mode == kModeRK4;
+    const double cu = mode == kModeRK1 || mode == kModeRK2 ? 0.5 : (sum_acc ? 1.0 / 6.0 : 1.0);
+    const double ca = mode == kModeRK1 ? 1.0 : 2.0;
     unsigned status = 0;
     if (tid0 < 2 * N) sM[tid0] = a.tab.ME[tid0 / N][tid0 % N];
 
@@ -312,6 +322,7 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
             const T hr = kShift ? T(a.gamma * geo->eref) : T(0);
             const T pref = kShift ? T((a.gamma - 1.0) * geo->eref) : T(0);
             T vel[3][M], p[M];
+            bool sound = true;
 #pragma unroll
             for (int q = 0; q < M; ++q) {
                 // P = (gamma-1) (rE - |m|^2 / (2 rho)), as dgp::interior_flux_r1
@@ -319,10 +330,16 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                 p[q] = (gamma - T(1.0)) * (S[4][q] - T(0.5) * ((S[1][q] * S[1][q] + S[2][q] * S[2][q] + S[3][q] * S[3][q]) * r1));
 #pragma unroll
                 for (int d = 0; d < 3; ++d) vel[d][q] = S[1 + d][q] * r1;
-                if (!(S[0][q] > T(0))) status |= kStatusRho;
-                if (!(p[q] + pref > T(0))) status |= kStatusPressure;
-                if (S[0][q] != S[0][q] || p[q] != p[q]) status |= kStatusNaN;
+                sound = sound && S[0][q] > T(0) && p[q] + pref > T(0);  // a NaN is not
                 S[4][q] = kShift ? S[4][q] + p[q] + hr : S[4][q] + p[q];
+            }
+            if (!sound) {
+#pragma unroll
+                for (int q = 0; q < M; ++q) {
+                    if (!(S[0][q] > T(0))) status |= kStatusRho;
+                    if (!(p[q] + pref > T(0))) status |= kStatusPressure;
+                    if (S[0][q] != S[0][q] || p[q] != p[q]) status |= kStatusNaN;
+                }
             }
             T JD[9];
 #pragma unroll
@@ -433,7 +450,7 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
             const int e = i / (5 * N2), row = i - e * (5 * N2), v = row / N2, byz = row - v * N2;
             const int by = byz % N, bz = byz / N;
             const size_t g = ((size_t)min(e0 + e, a.ne - 1) * 5 * N2 + row) * N;
-            double u0[N], ac[N];
+            double u0[N] = {}, ac[N] = {};
             if constexpr (F64) {
                 if (need_u0) load_row<N>(a.U0 + g, u0);
                 if (need_acc) load_row<N>(a.acc + g, ac);
@@ -472,46 +489,32 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                     k[b] = scale * s;
                 }
                 if (e0 + e >= a.ne) continue;
-                double o[N], ao[N];
-                switch (mode) {
-                    case kModeRK1:
+                if (put_acc) {
+                    double ao[N];
 #pragma unroll
-                        for (int b = 0; b < N; ++b) { ao[b] = k[b]; o[b] = 0.5 * k[b] + u0[b]; }
-                        break;
-                    case kModeRK2:
-#pragma unroll
-                        for (int b = 0; b < N; ++b) { ao[b] = ac[b] + 2.0 * k[b]; o[b] = 0.5 * k[b] + u0[b]; }
-                        break;
-                    case kModeRK3:
-#pragma unroll
-                        for (int b = 0; b < N; ++b) { ao[b] = ac[b] + 2.0 * k[b]; o[b] = 1.0 * k[b] + u0[b]; }
-                        break;
-                    case kModeRK4:
-#pragma unroll
-                        for (int b = 0; b < N; ++b) o[b] = u0[b] + (1.0 / 6.0) * (ac[b] + k[b]);
-                        break;
-                    case kModeFE:
-#pragma unroll
-                        for (int b = 0; b < N; ++b) o[b] = u0[b] + 1.0 * k[b];
-                        break;
-                    default:  // residual, mass-inverse residual
-#pragma unroll
-                        for (int b = 0; b < N; ++b) o[b] = k[b];
-                        break;
+                    for (int b = 0; b < N; ++b) ao[b] = ac[b] + ca * k[b];
+                    store_row<N>(a.acc + g, ao);
                 }
-                if (mode == kModeRK1 || mode == kModeRK2 || mode == kModeRK3) store_row<N>(a.acc + g, ao);
+                double o[N];
+#pragma unroll
+                for (int b = 0; b < N; ++b) o[b] = u0[b] + cu * (sum_acc ? ac[b] + k[b] : k[b]);
                 store_row<N>(a.out + g, o);
             } else {
+                // the node's faces summed in face order (0, 1, 2, 3, 4, 5); a row meets at
+                // most one y face (1 or 3) and one z face (0 or 5), its ends faces 4 and 2
+                const bool y0 = by == 0, y1 = by == N - 1, z0 = bz == 0, z1 = bz == N - 1;
+                const T* Ly = Lv + (y1 ? 3 : 1) * 5 * N2 + bz * N;
+                const T* Lz = Lv + (z1 ? 5 : 0) * 5 * N2 + by * N;
+                const T sy = y0 || y1 ? sg[y1 ? 3 : 1] : T(0), sz = z0 || z1 ? sg[z1 ? 5 : 0] : T(0);
+                const double l4 = double(sg[4] * Lv[4 * 5 * N2 + byz]), l2 = double(sg[2] * Lv[2 * 5 * N2 + byz]);
                 double t[N];
 #pragma unroll
                 for (int b = 0; b < N; ++b) {
-                    double s = 0.0;  // the node's faces, in face order
-                    if (bz == 0) s += double(sg[0] * Lv[by * N + b]);
-                    if (by == 0) s += double(sg[1] * Lv[1 * 5 * N2 + bz * N + b]);
-                    if (b == N - 1) s += double(sg[2] * Lv[2 * 5 * N2 + byz]);
-                    if (by == N - 1) s += double(sg[3] * Lv[3 * 5 * N2 + bz * N + b]);
-                    if (b == 0) s += double(sg[4] * Lv[4 * 5 * N2 + byz]);
-                    if (bz == N - 1) s += double(sg[5] * Lv[5 * 5 * N2 + by * N + b]);
+                    const double ly = sy == T(0) ? 0.0 : double(sy * Ly[b]), lz = sz == T(0) ? 0.0 : double(sz * Lz[b]);
+                    double s;
+                    if (b == 0) s = ((z0 ? lz : 0.0) + ly + l4) + (z0 ? 0.0 : lz);
+                    else if (b == N - 1) s = ((z0 ? lz : 0.0) + (y0 ? ly : 0.0) + l2) + (y0 ? 0.0 : ly) + (z0 ? 0.0 : lz);
+                    else s = lz + ly;
                     t[b] = double(x[b]) + s;
                 }
                 if (mode == kModeResidual) {
@@ -524,7 +527,7 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                     double s = 0.0;
 #pragma unroll
                     for (int k = 0; k < N; ++k) s += Mi[j * N + k] * t[k];
-                    res[Lay<P, 1>::cw(j, by, bz)] = s;
+                    res[bz * SZ + by * SY + j] = s;
                 }
             }
         }
@@ -535,18 +538,17 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
 #pragma unroll 1
                 for (int i = tid; i < ROWS; i += NT) {
                     const int e = i / (5 * N2);
-                    int v, bx, bz;
-                    task3<TaskOrd<P, 4>::minvy, 5, N, N>(i - e * (5 * N2), v, bx, bz);
+                    const int r = i - e * (5 * N2), v = r / N2, bx = r % N, bz = (r / N) % N;
                     double* res = sRes + e * L::RES + v * VS;
                     double t[N];
 #pragma unroll
-                    for (int k = 0; k < N; ++k) t[k] = res[Lay<P, 1>::cw(bx, k, bz)];
+                    for (int k = 0; k < N; ++k) t[k] = res[bz * SZ + k * SY + bx];
 #pragma unroll
                     for (int j = 0; j < N; ++j) {
                         double s = 0.0;
 #pragma unroll
                         for (int k = 0; k < N; ++k) s += Mi[j * N + k] * t[k];
-                        res[Lay<P, 1>::cw(bx, j, bz)] = s;
+                        res[bz * SZ + j * SY + bx] = s;
                     }
                 }
                 cta_sync<NT>();
@@ -555,7 +557,7 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                     const int e = i / (5 * N2), row = i - e * (5 * N2), v = row / N2, bxy = row - v * N2;
                     if (e0 + e >= a.ne) continue;
                     const size_t g0 = ((size_t)(e0 + e) * 5 + v) * NB + bxy;
-                    double u0[N], ac[N];
+                    double u0[N] = {}, ac[N] = {};
 #pragma unroll
                     for (int k = 0; k < N; ++k) {
                         if (need_u0) u0[k] = a.U0[g0 + k * N2];
@@ -567,7 +569,7 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                     const double* res = sRes + e * L::RES + v * VS;
                     double t[N];
 #pragma unroll
-                    for (int k = 0; k < N; ++k) t[k] = res[Lay<P, 1>::cw(bx, by, k)];
+                    for (int k = 0; k < N; ++k) t[k] = res[k * SZ + by * SY + bx];
 #pragma unroll
                     for (int j = 0; j < N; ++j) {
                         double s = 0.0;
@@ -575,14 +577,8 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                         for (int k = 0; k < N; ++k) s += Mi[j * N + k] * t[k];
                         const double kk = scale * s;
                         const size_t g = g0 + (size_t)j * N2;
-                        switch (mode) {
-                            case kModeMassInv: a.out[g] = kk; break;
-                            case kModeRK1: a.acc[g] = kk; a.out[g] = 0.5 * kk + u0[j]; break;
-                            case kModeRK2: a.acc[g] = ac[j] + 2.0 * kk; a.out[g] = 0.5 * kk + u0[j]; break;
-                            case kModeRK3: a.acc[g] = ac[j] + 2.0 * kk; a.out[g] = 1.0 * kk + u0[j]; break;
-                            case kModeRK4: a.out[g] = u0[j] + (1.0 / 6.0) * (ac[j] + kk); break;
-                            default: a.out[g] = u0[j] + 1.0 * kk; break;
-                        }
+                        if (put_acc) a.acc[g] = ac[j] + ca * kk;
+                        a.out[g] = u0[j] + cu * (sum_acc ? ac[j] + kk : kk);
                     }
                 }
             }
