@@ -17,6 +17,7 @@
 #include "../host/partition.h"
 #include "dg_ctx.cuh"
 #include "dg_column.cuh"
+#include "dg_small.cuh"
 #include "dg_tc.cuh"
 
 using dgk::GeoDev;
@@ -112,13 +113,20 @@ int load_constant_tables(dg_ctx* c)
 // ---------------------------------------------------------------------------
 // stage launches
 
+// whether every element of the mesh can have its own thread group in the
+// small-mesh kernel (unpartitioned meshes)
+bool small_mesh(const dg_ctx* c, const dgk::StageVariant& sv)
+{
+    return c->ne_alloc == c->ne && c->d_fdesc && c->ne <= 1LL * sv.small_elems * c->sms;
+}
+
 bool variant_matches(const dg_ctx* c, int v)
 {
     const dgk::StageVariant* vs = nullptr;
     const int nv = dgk::stage_variants(c->p, &vs);
     return v >= 0 && v < nv && (vs[v].fp32 != 0) == (c->precision == DG_PREC_MIXED_FP32) &&
            ((vs[v].flags & dgk::kGE) != 0) == c->pm.general && (!(vs[v].flags & dgk::kFX) || c->d_fflux) &&
-           (!(vs[v].flags & dgk::kTC) || c->d_tcop);
+           (!(vs[v].flags & dgk::kTC) || c->d_tcop) && (!(vs[v].flags & dgk::kSM) || small_mesh(c, vs[v]));
 }
 
 // Sets the variant's shared-memory attribute and its persistent grid size
@@ -154,6 +162,16 @@ int prepare_variant(dg_ctx* c, int v)
         if (face_per_sm < 1) return fail(c, DG_ERR_UNSUPPORTED, "face kernel does not fit on an SM");
         const int fb = sv.face_batch;
         c->variant_face_grid[v] = std::max(1, std::min((c->nface + fb - 1) / fb, dev_sms * face_per_sm));
+    }
+    if (sv.flags & dgk::kSM) {
+        int small_per_sm = 0;
+        DG_CUDA(c, cudaFuncSetAttribute(sv.small_func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sv.small_smem));
+        DG_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&small_per_sm, sv.small_func, sv.small_threads, sv.small_smem));
+        if (small_per_sm < 1) return fail(c, DG_ERR_UNSUPPORTED, "small-mesh kernel does not fit on an SM");
+        // enough blocks for one column group per block and one face per face warp
+        const int groups = (c->ne + sv.small_group_elems - 1) / sv.small_group_elems;
+        const int face_blocks = (c->nface + sv.small_face_warps - 1) / sv.small_face_warps;
+        c->variant_small_grid[v] = std::min(dev_sms, std::max(groups, face_blocks));
     }
     c->variant_grid[v] = std::max(1, std::min(batches, dev_sms * per_sm));
     return DG_OK;
@@ -832,15 +850,56 @@ __global__ void __launch_bounds__(256) ke_finalize_noalloc(const double* __restr
     if (threadIdx.x == 0) out[0] = red[0][0] / red[1][0];
 }
 
-int check_status(dg_ctx* c)
+// Pinned words for the contexts' status reads (a pageable target costs the copy a
+// second wait: 4^3, one step a call, 5 us of 45): one page for the process, a word
+// to a context from its first read until it is destroyed; contexts beyond the page
+// read into pageable memory
+constexpr int kStatusSlots = 1024;
+std::mutex g_slot_mutex;
+unsigned* g_slots = nullptr;
+std::vector<int> g_free_slots;
+bool g_slots_tried = false;
+
+unsigned* take_status_slot()
 {
-    unsigned st = 0;
-    DG_CUDA(c, cudaMemcpyAsync(&st, c->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+    std::lock_guard<std::mutex> lk(g_slot_mutex);
+    if (!g_slots_tried) {
+        g_slots_tried = true;
+        if (cudaHostAlloc((void**)&g_slots, kStatusSlots * sizeof(unsigned), cudaHostAllocPortable) == cudaSuccess) {
+            for (int i = 0; i < kStatusSlots; ++i) g_free_slots.push_back(i);
+        } else {
+            cudaGetLastError();
+            g_slots = nullptr;
+        }
+    }
+    if (g_free_slots.empty()) return nullptr;
+    const int i = g_free_slots.back();
+    g_free_slots.pop_back();
+    return g_slots + i;
+}
+
+void give_status_slot(unsigned* p)
+{
+    if (!p) return;
+    std::lock_guard<std::mutex> lk(g_slot_mutex);
+    g_free_slots.push_back(static_cast<int>(p - g_slots));
+}
+
+int check_status(dg_ctx* c, bool handed)
+{
+    unsigned word = 0;
+    if (!c->h_status) c->h_status = take_status_slot();
+    unsigned* to = c->h_status ? c->h_status : &word;
+    if (!handed) DG_CUDA(c, cudaMemcpyAsync(to, c->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     DG_CUDA(c, cudaStreamSynchronize(c->stream));
+    const unsigned st = *to;
     if (st) {
         c->status_accum |= st;
-        DG_CUDA(c, cudaMemsetAsync(c->d_status, 0, sizeof(unsigned), c->stream));
+        // (after a timeout the small-mesh kernel's counters start again)
+        const bool timeout = st & dgk::kStatusTimeout;
+        DG_CUDA(c, cudaMemsetAsync(c->d_status, 0, (timeout ? kStatusWords : 1) * sizeof(unsigned), c->stream));
         DG_CUDA(c, cudaStreamSynchronize(c->stream));
+        if (timeout) c->sync_base = c->done_base = 0;
         char buf[160];
         if (st & dgk::kStatusTimeout) {
             snprintf(buf, sizeof(buf), "a bounded device wait gave up (status 0x%x)", st);
@@ -970,6 +1029,7 @@ void release(dg_ctx* c)
     c->chunk_ev.clear();
     if (c->stream2) cudaStreamDestroy(c->stream2);
     if (c->stream) cudaStreamDestroy(c->stream);
+    give_status_slot(c->h_status);
 }
 
 }  // namespace dgi
@@ -1167,6 +1227,7 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
     const size_t ncls = c->pm.classes.size();
     int dev_sms = 0;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device);
+    c->sms = dev_sms;
     c->red_grid = std::max(1, std::min(c->ne, 8 * dev_sms));
     struct Alloc { void** p; size_t bytes; } allocs[] = {
         {(void**)&c->d_U0, nstate * sizeof(double)},
@@ -1180,18 +1241,18 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
         {(void**)&c->d_geo, ncls * (sizeof(GeoDev) + 9 * sizeof(double))},
         {(void**)&c->d_cmap, std::max<size_t>(1, c->pm.cmap.size() + c->pm.cmapn.size())},
         {(void**)&c->d_X0, static_cast<size_t>(c->ne_alloc) * 3 * sizeof(double)},
-        {(void**)&c->d_halo_send, std::max<size_t>(1, c->nslices) * sizeof(int2)},
-        {(void**)&c->d_halo_recv, std::max<size_t>(1, c->nslices) * sizeof(int2)},
+        {(void**)&c->d_halo_send, static_cast<size_t>(c->nslices) * sizeof(int2)},
+        {(void**)&c->d_halo_recv, static_cast<size_t>(c->nslices) * sizeof(int2)},
         {(void**)&c->d_partials, static_cast<size_t>(c->red_grid) * 5 * sizeof(double)},
-        {(void**)&c->d_status, sizeof(unsigned)},
-        {(void**)&c->d_gjd, std::max<size_t>(1, c->pm.gjd.size()) * sizeof(double)},
-        {(void**)&c->d_gnrm, std::max<size_t>(1, gnrm.size()) * sizeof(double)},
-        {(void**)&c->d_gimm, std::max<size_t>(1, gimm.size()) * sizeof(double)},
-        {(void**)&c->d_gnodes, std::max<size_t>(1, c->pm.gnodes.size()) * sizeof(double)},
-        {(void**)&c->d_gfsd, (c->pm.general && c->precision == DG_PREC_MIXED_FP32 ? nstate : 1) * sizeof(double)},
+        {(void**)&c->d_status, kStatusWords * sizeof(unsigned)},
+        {(void**)&c->d_gjd, c->pm.gjd.size() * sizeof(double)},
+        {(void**)&c->d_gnrm, gnrm.size() * sizeof(double)},
+        {(void**)&c->d_gimm, gimm.size() * sizeof(double)},
+        {(void**)&c->d_gnodes, c->pm.gnodes.size() * sizeof(double)},
+        {(void**)&c->d_gfsd, (c->pm.general && c->precision == DG_PREC_MIXED_FP32 ? nstate : 0) * sizeof(double)},
     };
     for (auto& al : allocs) {
-        if (cudaMalloc(al.p, al.bytes) != cudaSuccess) {
+        if (al.bytes && cudaMalloc(al.p, al.bytes) != cudaSuccess) {
             cudaGetLastError();
             c->err = "device allocation of " + std::to_string(al.bytes) + " bytes failed";
             return bail(DG_ERR_NOMEM);
@@ -1313,7 +1374,7 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
                 break;
             }
     }
-    std::vector<int2> hs(std::max(1, c->nslices)), hr(std::max(1, c->nslices));
+    std::vector<int2> hs(c->nslices), hr(c->nslices);
     for (int i = 0; i < c->nslices; ++i) {
         hs[i] = make_int2(plan.send_elem[i], plan.send_face[i]);
         hr[i] = make_int2(plan.recv_elem[i], plan.recv_face[i]);
@@ -1321,8 +1382,9 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
     bool ok = cudaMemcpy(c->d_conn, conn.data(), conn.size() * sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(c->d_frec, frec.data(), frec.size() * sizeof(dgk::FaceRec), cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(c->d_geo_class, c->pm.geo_class.data(), c->ne_alloc * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
-              cudaMemcpy(c->d_halo_send, hs.data(), hs.size() * sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess &&
-              cudaMemcpy(c->d_halo_recv, hr.data(), hr.size() * sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess &&
+              (c->nslices == 0 ||
+               (cudaMemcpy(c->d_halo_send, hs.data(), hs.size() * sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess &&
+                cudaMemcpy(c->d_halo_recv, hr.data(), hr.size() * sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess)) &&
               cudaMemcpy(c->d_X0, c->pm.X0.data(), c->pm.X0.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&
               (cmaps.empty() || cudaMemcpy(c->d_cmap, cmaps.data(), cmaps.size(), cudaMemcpyHostToDevice) == cudaSuccess) &&
               (!c->pm.general ||
@@ -1330,7 +1392,7 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
                 cudaMemcpy(c->d_gnrm, gnrm.data(), gnrm.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&
                 cudaMemcpy(c->d_gimm, gimm.data(), gimm.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&
                 cudaMemcpy(c->d_gnodes, c->pm.gnodes.data(), c->pm.gnodes.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess)) &&
-              cudaMemset(c->d_status, 0, sizeof(unsigned)) == cudaSuccess &&
+              cudaMemset(c->d_status, 0, kStatusWords * sizeof(unsigned)) == cudaSuccess &&
               cudaMemset(c->d_U0, 0, nstate * sizeof(double)) == cudaSuccess &&
               cudaMemset(c->d_acc, 0, nstate * sizeof(double)) == cudaSuccess;
     if (!ok) {
@@ -1626,6 +1688,43 @@ int launch_stage_chunked(dg_ctx* c, int stage, int mode, const double* Us, const
     return DG_OK;
 }
 
+// RK4 steps in the small-mesh kernel, at most kSmallSteps to a launch (queued
+// on the context's stream)
+constexpr int kSmallSteps = 256;
+
+int launch_small_steps(dg_ctx* c, double dt, int nsteps)
+{
+    int rc = prepare_variant(c, c->variant);
+    if (rc) return rc;
+    const dgk::StageVariant* vs = nullptr;
+    dgk::stage_variants(c->p, &vs);
+    const dgk::StageVariant& sv = vs[c->variant];
+    const int grid = c->variant_small_grid[c->variant], warps = grid * sv.small_face_warps;
+    dgk::SmallArgs s;
+    stage_args(c, dgk::kModeRK1, c->d_U0, c->d_U0, nullptr, dt, 0, c->ne, s.a);
+    s.Ua = c->d_Ua;
+    s.Ub = c->d_Ub;
+    s.fpt = std::min(sv.small_face_batch, (c->nface + warps - 1) / warps);
+    s.sync = c->d_status + kSyncWord;
+    for (int done = 0; done < nsteps; done += s.nsteps) {
+        s.nsteps = std::min(kSmallSteps, nsteps - done);
+        s.base = c->sync_base;
+        s.done_base = c->done_base;
+        s.host_status = done + s.nsteps == nsteps ? c->h_status : nullptr;
+        DG_CUDA(c, sv.small_launch(s, grid, c->stream));
+        c->sync_base += 4u * grid * s.nsteps;
+        c->done_base += grid;
+    }
+    return DG_OK;
+}
+
+bool runs_small(const dg_ctx* c)
+{
+    const dgk::StageVariant* vs = nullptr;
+    dgk::stage_variants(c->p, &vs);
+    return (vs[c->variant].flags & dgk::kSM) && c->chunks == 1;
+}
+
 int prepare_rk4_graph(dg_ctx* c, double dt)
 {
     if (c->graph_exec && c->graph_dt == dt) return DG_OK;
@@ -1663,19 +1762,23 @@ int dg_rk4_steps_timed(dg_ctx* c, double dt, int nsteps, double* device_ms)
     dgi::NvtxRange nvtx_("dg_rk4_steps_timed");
     if (!c || nsteps < 0 || !device_ms || !std::isfinite(dt)) return fail(c, DG_ERR_ARG, "dg_rk4_steps_timed: bad argument");
     DG_CUDA(c, cudaSetDevice(c->device));
-    int rc = prepare_rk4_graph(c, dt);
+    const bool small = runs_small(c);
+    int rc = small ? prepare_variant(c, c->variant) : prepare_rk4_graph(c, dt);
     if (rc) return rc;
     cudaEvent_t ev[2];
     DG_CUDA(c, cudaEventCreate(&ev[0]));
     if (cudaEventCreate(&ev[1]) != cudaSuccess) { cudaEventDestroy(ev[0]); return fail(c, DG_ERR_CUDA, "cudaEventCreate"); }
     cudaError_t ce = cudaEventRecord(ev[0], c->stream);
-    for (int s = 0; s < nsteps && ce == cudaSuccess; ++s) ce = cudaGraphLaunch(c->graph_exec, c->stream);
+    if (small && ce == cudaSuccess) rc = launch_small_steps(c, dt, nsteps);
+    else
+        for (int s = 0; s < nsteps && ce == cudaSuccess; ++s) ce = cudaGraphLaunch(c->graph_exec, c->stream);
     if (ce == cudaSuccess) ce = cudaEventRecord(ev[1], c->stream);
     if (ce == cudaSuccess) ce = cudaEventSynchronize(ev[1]);
     float ms = 0.0f;
     if (ce == cudaSuccess) ce = cudaEventElapsedTime(&ms, ev[0], ev[1]);
     cudaEventDestroy(ev[0]);
     cudaEventDestroy(ev[1]);
+    if (rc) return rc;
     if (ce != cudaSuccess) return fail(c, DG_ERR_CUDA, std::string("timed RK4: ") + cudaGetErrorString(ce));
     *device_ms = ms;
     return check_status(c);
@@ -1713,7 +1816,7 @@ int dg_set_stage_variant(dg_ctx* c, int v)
     if (!c) return DG_ERR_ARG;
     if (v < 0 || v >= dg_num_stage_variants(c->p)) return fail(c, DG_ERR_ARG, "stage variant index out of range");
     if (!variant_matches(c, v))
-        return fail(c, DG_ERR_ARG, "stage variant has the other residual precision or geometry kind");
+        return fail(c, DG_ERR_ARG, "stage variant has the other residual precision or geometry kind, or is for smaller meshes");
     if (v != c->variant) {
         c->variant = v;
         if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
@@ -1787,6 +1890,13 @@ int dg_tune_stage(dg_ctx* c, int reps, int* best, double* ms_per_variant)
     cudaEventDestroy(ev[1]);
     c->variant = keep;
     if (rc) return rc;
+    // the small-mesh forms run other variants' stage launches here; where one
+    // matches, its steps are the fastest (every element has its own threads)
+    const dgk::StageVariant* vs = nullptr;
+    dgk::stage_variants(c->p, &vs);
+    if (c->chunks == 1)
+        for (int v = nv - 1; v >= 0; --v)
+            if ((vs[v].flags & dgk::kSM) && variant_matches(c, v)) winner = v;
     rc = dg_set_stage_variant(c, winner);
     if (rc) return rc;
     if (best) *best = winner;
@@ -1799,11 +1909,15 @@ int dg_rk4_steps(dg_ctx* c, double dt, int nsteps)
     if (!c || nsteps < 0 || !std::isfinite(dt)) return fail(c, DG_ERR_ARG, "dg_rk4_steps: bad argument");
     if (nsteps == 0) return DG_OK;
     DG_CUDA(c, cudaSetDevice(c->device));
+    if (runs_small(c)) {
+        if (!c->h_status) c->h_status = take_status_slot();
+        const int rc = launch_small_steps(c, dt, nsteps);
+        return rc ? rc : check_status(c, c->h_status != nullptr);
+    }
     int rc = prepare_rk4_graph(c, dt);
     if (rc) return rc;
     for (int s = 0; s < nsteps; ++s) DG_CUDA(c, cudaGraphLaunch(c->graph_exec, c->stream));
-    DG_CUDA(c, cudaStreamSynchronize(c->stream));
-    return check_status(c);
+    return check_status(c);  // waits for the stream
 }
 
 int dg_fe_steps(dg_ctx* c, double dt, int nsteps)

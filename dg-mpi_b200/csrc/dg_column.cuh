@@ -50,6 +50,8 @@ namespace dgk {
 
 // launch option: the column form (needs the face kernel's fluxes lifted)
 constexpr int kCF = 8192;
+// launch option: RK4 steps of small meshes in one launch (dg_small.cuh)
+constexpr int kSM = 16384;
 
 // Shared-memory layout of a batch element.  The point array has 15 rows (v, d)
 // of [bz][qy][qx] with plane stride PS and row stride AS; the x-interpolated
@@ -169,51 +171,87 @@ __device__ __forceinline__ float add_two(float c, float d, float x, float b, flo
     return __fadd_rn(c, __fmaf_rn(d, x, __fmul_rn(b, y)));
 }
 
-template <int P, int E, int NT, typename T, int MB>
-__global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ StageArgs a)
-{
+// what a launch of one stage reads and writes (the arguments are passed to every
+// function rather than kept by reference: loads of them stay parameter loads)
+struct StageIO {
+    static __device__ __forceinline__ const double* Us(const StageArgs& a) { return a.Us; }
+    static __device__ __forceinline__ const double* U0(const StageArgs& a) { return a.U0; }
+    static __device__ __forceinline__ double* acc(const StageArgs& a) { return a.acc; }
+    static __device__ __forceinline__ double* out(const StageArgs& a) { return a.out; }
+    static __device__ __forceinline__ int mode(const StageArgs& a) { return a.mode; }
+    static __device__ __forceinline__ double dt(const StageArgs& a) { return a.dt; }
+};
+template <int NT>
+struct CtaSync {
+    __device__ __forceinline__ void operator()() const { cta_sync<NT>(); }
+};
+
+// One batch of E elements on NT threads that synchronise through Sync (a whole
+// CTA, or the threads of one group of a larger one): thread tid0 of NT, the
+// group's shared memory, the stage's buffers through IO.
+template <int P, int E, int NT, typename T, typename IO, typename Sync>
+struct Column {
     using L = ColLay<P, T>;
-    constexpr int N = L::N, M = L::M, NB = L::NB, NF = L::NF, N2 = L::N2;
-    constexpr int PS = L::PS, AS = L::AS, X1S = L::X1S, W = L::W, VS = L::VS, SY = L::SY, SZ = L::SZ;
-    constexpr bool F64 = sizeof(T) == 8;
-    constexpr bool kShift = !F64;
-    constexpr int ROWS = E * 5 * N2;                   // coefficient rows along x of a batch
-    extern __shared__ double csm[];
-    double* sRes = csm;                                // [E][5][VS] (FP32 path)
-    double* sM = sRes + E * L::RES;                    // [2][N] end columns of the 1D inverse mass
-    T* sW = reinterpret_cast<T*>(sM + 2 * N);          // [E][W]
-    T* sL = sW + E * W;                                // [E][6][5][N2] lifts in this element's node order
-    T* sSgn = sL + E * L::LF;                          // [E][6] -1 on the left side, +1 on the right
-    int* sCls = reinterpret_cast<int*>(sSgn + E * 6);  // [E]
-    const T* __restrict__ Bt = TabSel<T>::B(a.tab);
-    const T* __restrict__ Wt = TabSel<T>::W(a.tab);
-    const T* __restrict__ Ct = ColTab<T>::B(a.tab);
-    const T* __restrict__ Dt = ColTab<T>::D(a.tab);
-    const double* __restrict__ Mi = a.tab.Minv;
-    const int tid0 = threadIdx.x;
-    const T gamma = T(a.gamma);
-    const int mode = a.mode;
-    const bool need_u0 = mode >= kModeRK1, need_acc = mode == kModeRK2 || mode == kModeRK3 || mode == kModeRK4;
+    static constexpr int N = L::N, M = L::M, NB = L::NB, NF = L::NF, N2 = L::N2;
+    static constexpr int PS = L::PS, AS = L::AS, X1S = L::X1S, W = L::W, VS = L::VS, SY = L::SY, SZ = L::SZ;
+    static constexpr bool F64 = sizeof(T) == 8, kShift = !F64;
+    static constexpr int ROWS = E * 5 * N2;            // coefficient rows along x of a batch
+    static constexpr int LT = E * 6 * N2;              // its face nodes
+    static constexpr int R = (ROWS + NT - 1) / NT, RL = (LT + NT - 1) / NT;
+    IO io;
+    Sync sync;
+    const int tid0;
+    double* sRes;                                      // [E][5][VS] (FP32 path)
+    double* sM;                                        // [2][N] end columns of the 1D inverse mass
+    T* sW;                                             // [E][W]
+    T* sL;                                             // [E][6][5][N2] lifts in this element's node order
+    T* sSgn;                                           // [E][6] -1 on the left side, +1 on the right
+    int* sCls;                                         // [E]
     // the update: out = U0 + cu (acc + k in the last stage, else k), acc' = acc + ca k,
     // with U0 and acc zero where the mode does not read them
-    const bool put_acc = mode == kModeRK1 || mode == kModeRK2 || mode == kModeRK3, sum_acc = mode == kModeRK4;
-    const double cu = mode == kModeRK1 || mode == kModeRK2 ? 0.5 : (sum_acc ? 1.0 / 6.0 : 1.0);
-    const double ca = mode == kModeRK1 ? 1.0 : 2.0;
+    bool need_u0, need_acc, put_acc, sum_acc;
+    double cu, ca;
     unsigned status = 0;
-    if (tid0 < 2 * N) sM[tid0] = a.tab.ME[tid0 / N][tid0 % N];
-
-    // the next batch's coefficient rows and face records, fetched while this batch contracts
-    constexpr int R = (ROWS + NT - 1) / NT, LT = E * 6 * N2, RL = (LT + NT - 1) / NT;
+    // a batch's coefficient rows and face records
     double un[R][N];
-    int cl[R], fl[RL];
-    auto fetch = [&](int e0) {
+    int cl[R], fl[RL], cls;
+
+    __device__ __forceinline__ Column(const StageArgs& a, IO io_, Sync sync_, int tid, double* smem)
+        : io(io_), sync(sync_), tid0(tid)
+    {
+        sRes = smem;
+        sM = sRes + E * L::RES;
+        sW = reinterpret_cast<T*>(sM + 2 * N);
+        sL = sW + E * W;
+        sSgn = sL + E * L::LF;
+        sCls = reinterpret_cast<int*>(sSgn + E * 6);
+        if (tid0 < 2 * N) sM[tid0] = a.tab.ME[tid0 / N][tid0 % N];
+        set_mode(a);
+    }
+
+    // after a change of the stage
+    __device__ __forceinline__ void set_mode(const StageArgs& a)
+    {
+        const int mode = io.mode(a);
+        need_u0 = mode >= kModeRK1;
+        need_acc = mode == kModeRK2 || mode == kModeRK3 || mode == kModeRK4;
+        put_acc = mode == kModeRK1 || mode == kModeRK2 || mode == kModeRK3;
+        sum_acc = mode == kModeRK4;
+        cu = mode == kModeRK1 || mode == kModeRK2 ? 0.5 : (sum_acc ? 1.0 / 6.0 : 1.0);
+        ca = mode == kModeRK1 ? 1.0 : 2.0;
+    }
+
+    // rows and face records of the batch at e0 into registers (elements past the end repeat the last one)
+    __device__ __forceinline__ void fetch(const StageArgs& a, int e0)
+    {
+        cls = a.geo_class[min(e0 + min(tid0, E - 1), a.ne - 1)];
         const int tid = opaque<F64 && P >= 4>(tid0);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int i = tid + r * NT;
             if (i < ROWS) {
                 const int e = i / (5 * N2), row = i - e * (5 * N2), ge = min(e0 + e, a.ne - 1);
-                load_row<N>(a.Us + ((size_t)ge * 5 * N2 + row) * N, un[r]);
+                load_row<N>(io.Us(a) + ((size_t)ge * 5 * N2 + row) * N, un[r]);
                 if constexpr (kShift) cl[r] = a.geo_class[ge];
             }
         }
@@ -225,19 +263,17 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                 fl[r] = a.lrec[(size_t)min(e0 + e, a.ne - 1) * 6 + f];
             }
         }
-    };
-    const int stride = gridDim.x * E;
-    int e0 = a.e_begin + blockIdx.x * E;
-    if (e0 < a.ne) fetch(e0);
-    for (; e0 < a.ne; e0 += stride) {
-        // this batch's RK operands (read by the last pass) and the next batch's rows on
-        // their way into L2
-        if (tid0 < 3 && (tid0 == 0 ? e0 + stride < a.ne : tid0 == 1 ? need_u0 && a.U0 != a.Us : need_acc)) {
-            const int ep = tid0 == 0 ? e0 + stride : e0;
-            prefetch_l2((tid0 == 0 ? a.Us : tid0 == 1 ? a.U0 : a.acc) + (size_t)ep * 5 * NB, min(E, a.ne - ep) * 5 * NB);
-        }
-        // ---- this batch's face lifts stream in (used by the last pass) ----
-        {
+    }
+
+    // the fetched batch's geometry classes
+    __device__ __forceinline__ void classes()
+    {
+        if (tid0 < E) sCls[tid0] = cls;
+    }
+
+    // the batch's face lifts on their way into shared memory
+    __device__ __forceinline__ void lifts(const StageArgs& a, int e0)
+    {
             const T* gL = reinterpret_cast<const T*>(a.fflux);
             const int tid = opaque<F64 && P >= 4>(tid0);
 #pragma unroll
@@ -254,10 +290,20 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                     if (c == 0) sSgn[e * 6 + f] = fl[r] < 0 ? T(-1) : T(1);
                 }
             }
-            for (int e = tid; e < E; e += NT) sCls[e] = a.geo_class[min(e0 + e, a.ne - 1)];
+            classes();
             cp_async_commit();
-        }
-        // ---- x interpolation ----
+    }
+
+    // x interpolation of the fetched rows
+    __device__ __forceinline__ void interp_x(const StageArgs& a)
+    {
+        const T* __restrict__ Bt = TabSel<T>::B(a.tab);
+        const T* __restrict__ Wt = TabSel<T>::W(a.tab);
+        const T* __restrict__ Ct = ColTab<T>::B(a.tab);
+        const T* __restrict__ Dt = ColTab<T>::D(a.tab);
+        const double* __restrict__ Mi = a.tab.Minv;
+        const T gamma = T(a.gamma);
+        (void)Bt, (void)Wt, (void)Ct, (void)Dt, (void)Mi, (void)gamma;
         const int tid = opaque<F64 && P >= 4>(tid0);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -278,7 +324,20 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                 }
             }
         }
-        cta_sync<NT>();
+    }
+
+    // y interpolation, then per quadrature column the z interpolation, flux and z contraction
+    __device__ __forceinline__ void columns(const StageArgs& a)
+    {
+        const T* __restrict__ Bt = TabSel<T>::B(a.tab);
+        const T* __restrict__ Wt = TabSel<T>::W(a.tab);
+        const T* __restrict__ Ct = ColTab<T>::B(a.tab);
+        const T* __restrict__ Dt = ColTab<T>::D(a.tab);
+        const double* __restrict__ Mi = a.tab.Minv;
+        const T gamma = T(a.gamma);
+        (void)Bt, (void)Wt, (void)Ct, (void)Dt, (void)Mi, (void)gamma;
+        const int tid = opaque<F64 && P >= 5>(tid0);
+        sync();
         // ---- y interpolation ----
 #pragma unroll 1
         for (int i = tid; i < E * 5 * N * M; i += NT) {
@@ -298,7 +357,7 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                 o[q * M] = s;
             }
         }
-        cta_sync<NT>();
+        sync();
         // ---- columns: z interpolation, flux, z contraction in registers ----
 #pragma unroll 1
         for (int i = tid; i < E * NF; i += NT) {
@@ -415,8 +474,19 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                     });
             }
         }
-        cta_sync<NT>();
-        fetch(e0 + stride);  // past the end: the last element again (a condition would keep the old rows alive)
+        sync();
+    }
+
+    __device__ __forceinline__ void contract_y(const StageArgs& a)
+    {
+        const T* __restrict__ Bt = TabSel<T>::B(a.tab);
+        const T* __restrict__ Wt = TabSel<T>::W(a.tab);
+        const T* __restrict__ Ct = ColTab<T>::B(a.tab);
+        const T* __restrict__ Dt = ColTab<T>::D(a.tab);
+        const double* __restrict__ Mi = a.tab.Minv;
+        const T gamma = T(a.gamma);
+        (void)Bt, (void)Wt, (void)Ct, (void)Dt, (void)Mi, (void)gamma;
+        const int tid = opaque<F64 && P >= 4>(tid0);
         // ---- y contraction: By^T A0 over row 3v, Dy^T A1 + By^T A2 over row 3v+1 ----
 #pragma unroll 1
         for (int i = tid; i < E * 5 * N * M; i += NT) {
@@ -442,8 +512,19 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                 A0[AS + b * M] = c12[b];
             }
         }
-        cp_async_wait_group<0>();  // the lifts have landed
-        cta_sync<NT>();
+    }
+
+    // x contraction, face lifts, inverse mass (FP32 path) and stage update
+    __device__ __forceinline__ void finish(const StageArgs& a, int e0)
+    {
+        const T* __restrict__ Bt = TabSel<T>::B(a.tab);
+        const T* __restrict__ Wt = TabSel<T>::W(a.tab);
+        const T* __restrict__ Ct = ColTab<T>::B(a.tab);
+        const T* __restrict__ Dt = ColTab<T>::D(a.tab);
+        const double* __restrict__ Mi = a.tab.Minv;
+        const T gamma = T(a.gamma);
+        (void)Bt, (void)Wt, (void)Ct, (void)Dt, (void)Mi, (void)gamma;
+        const int tid = opaque<F64 && P >= 4>(tid0);
         // ---- x contraction, face lifts; FP64: the stage update ----
 #pragma unroll 1
         for (int i = tid; i < ROWS; i += NT) {
@@ -452,8 +533,8 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
             const size_t g = ((size_t)min(e0 + e, a.ne - 1) * 5 * N2 + row) * N;
             double u0[N] = {}, ac[N] = {};
             if constexpr (F64) {
-                if (need_u0) load_row<N>(a.U0 + g, u0);
-                if (need_acc) load_row<N>(a.acc + g, ac);
+                if (need_u0) load_row<N>(io.U0(a) + g, u0);
+                if (need_acc) load_row<N>(io.acc(a) + g, ac);
             }
             const T* C0 = sW + e * W + (3 * v) * AS + bz * PS + by * M;
             T x[N];
@@ -475,7 +556,7 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                 const double* L3 = Lv + 3 * 5 * N2 + bz * N;
                 const double* L0 = Lv + by * N;
                 const double* L5 = Lv + 5 * 5 * N2 + by * N;
-                const double scale = mode == kModeResidual ? 1.0 : a.dt * a.geo[sCls[e]].dtf * a.geo[sCls[e]].inv_djac;
+                const double scale = io.mode(a) == kModeResidual ? 1.0 : io.dt(a) * a.geo[sCls[e]].dtf * a.geo[sCls[e]].inv_djac;
                 double k[N];
 #pragma unroll
                 for (int b = 0; b < N; ++b) {
@@ -493,12 +574,12 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                     double ao[N];
 #pragma unroll
                     for (int b = 0; b < N; ++b) ao[b] = ac[b] + ca * k[b];
-                    store_row<N>(a.acc + g, ao);
+                    store_row<N>(io.acc(a) + g, ao);
                 }
                 double o[N];
 #pragma unroll
                 for (int b = 0; b < N; ++b) o[b] = u0[b] + cu * (sum_acc ? ac[b] + k[b] : k[b]);
-                store_row<N>(a.out + g, o);
+                store_row<N>(io.out(a) + g, o);
             } else {
                 // the node's faces summed in face order (0, 1, 2, 3, 4, 5); a row meets at
                 // most one y face (1 or 3) and one z face (0 or 5), its ends faces 4 and 2
@@ -517,8 +598,8 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                     else s = lz + ly;
                     t[b] = double(x[b]) + s;
                 }
-                if (mode == kModeResidual) {
-                    if (e0 + e < a.ne) store_row<N>(a.out + ((size_t)(e0 + e) * 5 * N2 + row) * N, t);
+                if (io.mode(a) == kModeResidual) {
+                    if (e0 + e < a.ne) store_row<N>(io.out(a) + ((size_t)(e0 + e) * 5 * N2 + row) * N, t);
                     continue;
                 }
                 double* res = sRes + e * L::RES + v * VS;
@@ -532,9 +613,9 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
             }
         }
         if constexpr (!F64) {
-            if (mode != kModeResidual) {
+            if (io.mode(a) != kModeResidual) {
                 // ---- FP64 inverse mass along y, then z fused with the update ----
-                cta_sync<NT>();
+                sync();
 #pragma unroll 1
                 for (int i = tid; i < ROWS; i += NT) {
                     const int e = i / (5 * N2);
@@ -551,7 +632,7 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                         res[bz * SZ + j * SY + bx] = s;
                     }
                 }
-                cta_sync<NT>();
+                sync();
 #pragma unroll 1
                 for (int i = tid; i < ROWS; i += NT) {
                     const int e = i / (5 * N2), row = i - e * (5 * N2), v = row / N2, bxy = row - v * N2;
@@ -560,12 +641,12 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                     double u0[N] = {}, ac[N] = {};
 #pragma unroll
                     for (int k = 0; k < N; ++k) {
-                        if (need_u0) u0[k] = a.U0[g0 + k * N2];
-                        if (need_acc) ac[k] = a.acc[g0 + k * N2];
+                        if (need_u0) u0[k] = io.U0(a)[g0 + k * N2];
+                        if (need_acc) ac[k] = io.acc(a)[g0 + k * N2];
                     }
                     const int bx = bxy % N, by = bxy / N;
                     const GeoDev& gg = a.geo[sCls[e]];
-                    const double scale = a.dt * gg.dtf * gg.inv_djac;
+                    const double scale = io.dt(a) * gg.dtf * gg.inv_djac;
                     const double* res = sRes + e * L::RES + v * VS;
                     double t[N];
 #pragma unroll
@@ -577,15 +658,45 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
                         for (int k = 0; k < N; ++k) s += Mi[j * N + k] * t[k];
                         const double kk = scale * s;
                         const size_t g = g0 + (size_t)j * N2;
-                        if (put_acc) a.acc[g] = ac[j] + ca * kk;
-                        a.out[g] = u0[j] + cu * (sum_acc ? ac[j] + kk : kk);
+                        if (put_acc) io.acc(a)[g] = ac[j] + ca * kk;
+                        io.out(a)[g] = u0[j] + cu * (sum_acc ? ac[j] + kk : kk);
                     }
                 }
             }
         }
+    }
+};
+
+template <int P, int E, int NT, typename T, int MB>
+__global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ StageArgs a)
+{
+    extern __shared__ double csm[];
+    constexpr int NB = ColLay<P, T>::NB;
+    Column<P, E, NT, T, StageIO, CtaSync<NT>> c(a, StageIO(), CtaSync<NT>(), threadIdx.x, csm);
+    const int tid = threadIdx.x;
+    const int stride = gridDim.x * E;
+    int e0 = a.e_begin + blockIdx.x * E;
+    if (e0 < a.ne) c.fetch(a, e0);
+    for (; e0 < a.ne; e0 += stride) {
+        // this batch's RK operands (read by the last pass) and the next batch's rows on
+        // their way into L2
+        if (tid < 3 && (tid == 0 ? e0 + stride < a.ne : tid == 1 ? c.need_u0 && a.U0 != a.Us : c.need_acc)) {
+            const int ep = tid == 0 ? e0 + stride : e0;
+            prefetch_l2((tid == 0 ? a.Us : tid == 1 ? a.U0 : a.acc) + (size_t)ep * 5 * NB, min(E, a.ne - ep) * 5 * NB);
+        }
+        c.lifts(a, e0);
+        c.interp_x(a);
+        c.columns(a);
+        // the next batch's rows and records, in flight during the contractions (past
+        // the end the last element's: a condition would keep the old rows alive)
+        c.fetch(a, e0 + stride);
+        c.contract_y(a);
+        cp_async_wait_all();  // the lifts have landed
+        cta_sync<NT>();
+        c.finish(a, e0);
         cta_sync<NT>();  // the point array and the lifts are the next batch's
     }
-    if (status) atomicOr(a.status, status);
+    if (c.status) atomicOr(a.status, c.status);
 }
 
 // ---------------------------------------------------------------------------
@@ -620,39 +731,22 @@ struct FaceLay {
     static constexpr size_t bytes = tr_bytes + sl_bytes + 3 * FB * sizeof(FaceDesc);
 };
 
-template <int P, typename T, int FB, int NT, int MB>
-__global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant__ StageArgs a)
-{
+// the phases of a batch of nf <= FB faces on NT threads; a synchronisation of the
+// threads belongs between any two of them
+template <int P, typename T, int FB, int NT>
+struct FacePhases {
     using L = FaceLay<P, T, FB>;
-    constexpr int N = L::N, M = L::M, NB = N * N * N, NF = L::NF, N2 = L::N2, FS = L::FS, NS = L::NS;
-    constexpr bool kShift = sizeof(T) == 4;
-    extern __shared__ __align__(16) unsigned char fraw[];
-    T* sTr = reinterpret_cast<T*>(fraw);                              // [FB][2][5][FS]
-    double* sSl = reinterpret_cast<double*>(fraw + L::tr_bytes);      // [FB][2][5][NS]
-    FaceDesc* sDesc = reinterpret_cast<FaceDesc*>(fraw + L::tr_bytes + L::sl_bytes);  // [3][FB]
-    const T* __restrict__ Bt = TabSel<T>::B(a.tab);
-    const T* __restrict__ Wt = TabSel<T>::W(a.tab);
-    const T* __restrict__ Ct = ColTab<T>::B(a.tab);
-    T* out = reinterpret_cast<T*>(a.fflux);
-    const int tid = threadIdx.x;
-    unsigned status = 0;
-    const int fstep = gridDim.x * FB;
-    // the descriptors of batch f (the last face repeated past the end)
-    auto fetch = [&](int f, int slot) {
-        if (f < a.nface)
-            for (int i = tid; i < FB * 4; i += NT) {
-                const int j = i / 4, w = i % 4;
-                cp_async16(reinterpret_cast<char*>(sDesc + slot * FB + j) + 16 * w,
-                           reinterpret_cast<const char*>(a.fdesc + min(f + j, a.nface - 1)) + 16 * w);
-            }
-    };
-    // the slices of batch f, whose descriptors have landed in slot
-    auto gather = [&](int f, int slot) {
-        if (!L::COOP || f >= a.nface) return;
+    static constexpr int N = L::N, M = L::M, NB = N * N * N, NF = L::NF, N2 = L::N2, FS = L::FS, NS = L::NS;
+    static constexpr bool kShift = sizeof(T) == 4;
+
+    // the faces' slices (cp.async)
+    static __device__ __forceinline__ void gather(const double* Us, const FaceDesc* sD, int nf, double* sSl, int tid)
+    {
         for (int sj = tid / 32; sj < 2 * FB; sj += NT / 32) {
-            const FaceDesc& fd = sDesc[slot * FB + sj / 2];
+            if (sj >= 2 * nf) break;
+            const FaceDesc& fd = sD[sj / 2];
             const int st = fd.strides >> (16 * (sj % 2)), s0 = st & 255, s1 = (st >> 8) & 255;
-            const double* src = a.Us + fd.base[sj % 2];
+            const double* src = Us + fd.base[sj % 2];
             double* dst = sSl + sj * 5 * NS;
 #pragma unroll
             for (int r = 0; r < (5 * N2 + 31) / 32; ++r) {
@@ -660,33 +754,22 @@ __global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant
                 if (i < 5 * N2) cp_async8(dst + v * NS + c, src + v * NB + (c % N) * s0 + (c / N) * s1);
             }
         }
-    };
-    int f0 = a.face_begin + blockIdx.x * FB;
-    if (f0 < a.nface) {
-        fetch(f0, 0);
-        fetch(f0 + fstep, 1);
-        cp_async_commit();
-        cp_async_wait_all();
-        cta_sync<NT>();
-        gather(f0, 0);
-        cp_async_commit();
     }
-    int slot = 0;
-    for (; f0 < a.nface; f0 += fstep) {
-        const FaceDesc* sD = sDesc + slot * FB;
-        const int next = slot == 2 ? 0 : slot + 1, after = next == 2 ? 0 : next + 1;
-        cp_async_wait_all();  // this batch's slices, the next one's descriptors
-        cta_sync<NT>();
-        fetch(f0 + 2 * fstep, after);
-        // traces, both sides in the listed side's energy frame
+
+    // both sides' traces, in the listed side's energy frame
+    static __device__ __forceinline__ void traces(const StageArgs& a, const double* Us, const FaceDesc* sD, int nf,
+                                                  const double* sSl, T* sTr, int tid)
+    {
+        const T* __restrict__ Bt = TabSel<T>::B(a.tab);
         for (int t = tid; t < FB * 10; t += NT) {
+            if (t >= nf * 10) break;
             const FaceDesc& fd = sD[t / 10];
             const double sh = kShift && t % 5 == 4 ? a.geo[fd.cls].eref : 0.0;
             const double* s = sSl + t * NS;
             int s0 = 1, s1 = N;
             if constexpr (!L::COOP) {
                 const int side = (t / 5) % 2, st = fd.strides >> (16 * side);
-                s = a.Us + fd.base[side] + (t % 5) * NB;
+                s = Us + fd.base[side] + (t % 5) * NB;
                 s0 = st & 255;
                 s1 = (st >> 8) & 255;
             }
@@ -702,12 +785,15 @@ __global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant
                 for (int b0 = 0; b0 < N; ++b0) sl[b1][b0] = kShift ? T(x[b1][b0] - sh) : T(x[b1][b0]);
             interp2d<N, M, T>(Bt, sl, sTr + t * FS);
         }
-        cta_sync<NT>();
-        gather(f0 + fstep, next);
-        cp_async_commit();
+    }
+
+    // the flux at the listed side's face points, over that side's trace
+    static __device__ __forceinline__ void flux(const StageArgs& a, const FaceDesc* sD, int nf, T* sTr, unsigned& status, int tid)
+    {
+        const T* __restrict__ Wt = TabSel<T>::W(a.tab);
         for (int i = tid; i < FB * NF; i += NT) {
             const int c = i % NF, j = i / NF;
-            if (f0 + j >= a.nface) continue;
+            if (j >= nf) continue;
             const FaceDesc& fd = sD[j];
             const int cn = a.cmap[(fd.info >> 4) * NF + c];
             const int isL = (fd.info >> 3) & 1;
@@ -728,10 +814,16 @@ __global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant
 #pragma unroll
             for (int v = 0; v < 5; ++v) To[v * FS + c] = Fo[v] * w;
         }
-        cta_sync<NT>();
+    }
+
+    // the lifts of faces f0 .. f0 + nf - 1
+    static __device__ __forceinline__ void lift(const StageArgs& a, int f0, int nf, const T* sTr, int tid)
+    {
+        const T* __restrict__ Ct = ColTab<T>::B(a.tab);
+        T* out = reinterpret_cast<T*>(a.fflux);
         for (int t = tid; t < FB * 5 * N; t += NT) {
             const int b0 = t % N, jv = t / N, v = jv % 5, j = jv / 5;
-            if (f0 + j >= a.nface) continue;
+            if (j >= nf) continue;
             const T* F = sTr + (j * 2) * 5 * FS + v * FS;
             T r[M];
 #pragma unroll
@@ -750,6 +842,58 @@ __global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant
                 o[b1 * N] = s;
             }
         }
+    }
+};
+
+template <int P, typename T, int FB, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant__ StageArgs a)
+{
+    using L = FaceLay<P, T, FB>;
+    using F = FacePhases<P, T, FB, NT>;
+    extern __shared__ __align__(16) unsigned char fraw[];
+    T* sTr = reinterpret_cast<T*>(fraw);                              // [FB][2][5][FS]
+    double* sSl = reinterpret_cast<double*>(fraw + L::tr_bytes);      // [FB][2][5][NS]
+    FaceDesc* sDesc = reinterpret_cast<FaceDesc*>(fraw + L::tr_bytes + L::sl_bytes);  // [3][FB]
+    const int tid = threadIdx.x;
+    unsigned status = 0;
+    const int fstep = gridDim.x * FB;
+    // the descriptors of batch f (the last face repeated past the end)
+    auto fetch = [&](int f, int slot) {
+        if (f < a.nface)
+            for (int i = tid; i < FB * 4; i += NT) {
+                const int j = i / 4, w = i % 4;
+                cp_async16(reinterpret_cast<char*>(sDesc + slot * FB + j) + 16 * w,
+                           reinterpret_cast<const char*>(a.fdesc + min(f + j, a.nface - 1)) + 16 * w);
+            }
+    };
+    auto gather = [&](int f, int slot) {
+        if (L::COOP && f < a.nface) F::gather(a.Us, sDesc + slot * FB, FB, sSl, tid);
+    };
+    int f0 = a.face_begin + blockIdx.x * FB;
+    if (f0 < a.nface) {
+        fetch(f0, 0);
+        fetch(f0 + fstep, 1);
+        cp_async_commit();
+        cp_async_wait_all();
+        cta_sync<NT>();
+        gather(f0, 0);
+        cp_async_commit();
+    }
+    int slot = 0;
+    for (; f0 < a.nface; f0 += fstep) {
+        const FaceDesc* sD = sDesc + slot * FB;
+        const int next = slot == 2 ? 0 : slot + 1, after = next == 2 ? 0 : next + 1;
+        const int nf = min(FB, a.nface - f0);
+        cp_async_wait_all();  // this batch's slices, the next one's descriptors
+        cta_sync<NT>();
+        fetch(f0 + 2 * fstep, after);
+        F::traces(a, a.Us, sD, FB, sSl, sTr, tid);
+        cta_sync<NT>();
+        gather(f0 + fstep, next);
+        cp_async_commit();
+        F::flux(a, sD, nf, sTr, status, tid);
+        cta_sync<NT>();
+        F::lift(a, f0, nf, sTr, tid);
         slot = next;
     }
     cp_async_wait_all();
@@ -782,7 +926,8 @@ StageVariant make_column_variant(int min_per_sm)
     static_assert(ColLay<P, T>::bytes(E) <= 227 * 1024, "column kernel shared memory exceeds 227 KB");
     static_assert(FaceLay<P, T, FB>::bytes <= 227 * 1024, "face kernel shared memory exceeds 227 KB");
     StageVariant v{E, NT, 1, sizeof(T) == 4 ? 1 : 0, kSB | kFX | kCF, ColLay<P, T>::bytes(E),
-                   (const void*)column_kernel<P, E, NT, T, MB>, launch_column<P, E, NT, T, MB>, nullptr, 0, 0, nullptr, 0, min_per_sm};
+                   (const void*)column_kernel<P, E, NT, T, MB>, launch_column<P, E, NT, T, MB>};
+    v.min_per_sm = min_per_sm;
     v.face_func = (const void*)face_lift_kernel<P, T, FB, FNT, FMB>;
     v.face_smem = FaceLay<P, T, FB>::bytes;
     v.face_threads = FNT;

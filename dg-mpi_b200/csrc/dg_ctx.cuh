@@ -15,6 +15,7 @@
 
 namespace dgi {
 constexpr int kMaxVariants = 48;  // launch variants per order (checked in prepare_variant)
+constexpr int kSyncWord = 32, kStatusWords = 128;
 
 // NVTX range named after a C-ABI call, for timelines of Nsight tools (a no-op
 // when no tool is attached)
@@ -74,8 +75,12 @@ struct dg_ctx {
     uint16_t* d_tcop = nullptr;
     int variant_face_grid[dgi::kMaxVariants] = {};  // face kernel grid per FX variant
     double* d_partials = nullptr;
-    unsigned* d_status = nullptr;
+    unsigned* d_status = nullptr;      // the status word, then (kSyncWord) the small-mesh kernel's counters
+    unsigned* h_status = nullptr;      // its pinned copy on the host (see check_status)
+    unsigned sync_base = 0, done_base = 0;  // the counters' values
+    int variant_small_grid[dgi::kMaxVariants] = {};  // blocks of the small-mesh kernel, 0: not that form
     int red_grid = 0;
+    int sms = 0;  // multiprocessors of the device
     int variant = 0;                                // index into dgk::stage_variants(p)
     int variant_grid[dgi::kMaxVariants] = {};       // persistent grid per variant, 0 = not prepared
     dgk::StageTables stage_tab{};
@@ -119,7 +124,9 @@ void stage_args(const dg_ctx* c, int mode, const double* Us, const double* U0, d
 // stage launch over the owned elements [e_begin, e_end) (e_end < 0: all)
 int launch_stage(dg_ctx* c, int mode, const double* Us, const double* U0, double* out, double dt, int e_begin = 0,
                  int e_end = -1);
-int check_status(dg_ctx* c);
+// waits for the stream and turns the status word into a return code; handed: the
+// queued work copies the word to c->h_status itself
+int check_status(dg_ctx* c, bool handed = false);
 
 // state of elements [e0, e0 + ne) between the host layout [ne][nb][5] and the
 // device layout [ne][5][nb] (staged through d_out / d_Ub); synchronous

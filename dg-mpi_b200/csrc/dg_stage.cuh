@@ -1530,6 +1530,8 @@ constexpr size_t stage_smem_bytes()
 
 // ---- compiled launch variants (one translation unit per order) ----
 
+struct SmallArgs;
+
 struct StageVariant {
     int E, NT, G;        // elements per CTA, threads per CTA, variable groups
     int fp32;            // 1: residual arithmetic in FP32 (mixed precision), 0: FP64
@@ -1548,6 +1550,12 @@ struct StageVariant {
     cudaError_t (*face_launch)(const StageArgs&, int grid, cudaStream_t);
     int face_batch;      // faces per CTA batch of the face kernel
     int min_per_sm;      // elements per SM from which the variant may be the untuned default
+    // small-mesh variants (kSM, dg_small.cuh): RK4 steps in one cooperative launch
+    // of up to one block per SM while the mesh has at most small_elems elements per SM
+    const void* small_func;
+    cudaError_t (*small_launch)(SmallArgs&, int grid, cudaStream_t);
+    size_t small_smem;
+    int small_threads, small_elems, small_group_elems, small_face_warps, small_face_batch;
 };
 
 template <int P, typename T, bool GEO>
@@ -1587,7 +1595,7 @@ StageVariant make_variant()
     if constexpr (MB > 0) func = (const void*)stage_kernel_mb<P, E, NT, G, T, FL, MB>;
     else func = (const void*)stage_kernel<P, E, NT, G, T, FL>;
     StageVariant v{E, NT, G, sizeof(T) == 4 ? 1 : 0, FL | (MB << 8), stage_smem_bytes<P, E, G, T, FL>(),
-                   func, launch_stage_variant<P, E, NT, G, T, FL, MB>, nullptr, 0, 0, nullptr, 0, 0};
+                   func, launch_stage_variant<P, E, NT, G, T, FL, MB>};
     if constexpr ((FL & 64) != 0) {
         static_assert(face_smem_bytes<P, T>() <= 227 * 1024, "face kernel shared memory exceeds 227 KB");
         constexpr bool geo = (FL & 32) != 0;

@@ -7,16 +7,18 @@
 // general-geometry (kGE) entries only, the others never do.  The
 // first variant of each precision is the default (the measured best); dg_tune_stage may pick another.
 #include "dg_stage.cuh"
-#include "dg_column.cuh"
+#include "dg_small.cuh"
 
 namespace dgk {
 
 static const StageVariant kVariants1[] = {
+    make_small_variant<1, 1, 32, 8, 4, 3, double>(make_column_variant<1, 3, 32, double, 16, 3, 32, 20>(0)),
     make_column_variant<1, 3, 32, double, 16, 3, 32, 20>(0),
     make_variant<1, 8, 128, 1, double>(),
     make_variant<1, 4, 64, 1, double>(),
     make_variant<1, 2, 64, 1, double>(),
     make_variant<1, 1, 32, 1, double>(),
+    make_small_variant<1, 1, 32, 8, 4, 3, float>(make_column_variant<1, 3, 32, float, 20, 12, 128, 1>(0)),
     make_column_variant<1, 3, 32, float, 20, 12, 128, 1>(0),
     make_variant<1, 8, 128, 1, float, kUF | kSB | kFX>(),
     make_variant<1, 4, 64, 1, float, kUF | kSB | kFX>(),

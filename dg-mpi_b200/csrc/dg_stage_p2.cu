@@ -7,12 +7,14 @@
 // general-geometry (kGE) entries only, the others never do.  The
 // first variant of each precision is the default (the measured best); dg_tune_stage may pick another.
 #include "dg_stage.cuh"
-#include "dg_column.cuh"
+#include "dg_small.cuh"
 
 namespace dgk {
 
 static const StageVariant kVariants2[] = {
-    make_column_variant<2, 2, 32, double, 11, 6, 32, 1>(6),
+    make_small_variant<2, 1, 64, 3, 6, 2, double>(make_column_variant<2, 2, 32, double, 11, 6, 32, 1>(0)),
+    make_small_variant<2, 1, 32, 6, 6, 2, double>(make_column_variant<2, 2, 32, double, 11, 6, 32, 1>(0)),
+    make_column_variant<2, 2, 32, double, 11, 6, 32, 1>(0),
     make_variant<2, 1, 32, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<2, 2, 64, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<2, 1, 32, 1, double, kUF | kSB | kFX>(),
@@ -22,7 +24,9 @@ static const StageVariant kVariants2[] = {
     make_variant<2, 2, 64, 1, double, kUF | kRS | kSB>(),
     make_variant<2, 1, 32, 1, double>(),
     make_variant<2, 2, 64, 1, double>(),
-    make_column_variant<2, 2, 32, float, 16, 8, 128, 1>(16),
+    make_small_variant<2, 1, 64, 3, 6, 2, float>(make_column_variant<2, 2, 32, float, 16, 8, 128, 1>(0)),
+    make_small_variant<2, 1, 32, 6, 6, 2, float>(make_column_variant<2, 2, 32, float, 16, 8, 128, 1>(0)),
+    make_column_variant<2, 2, 32, float, 16, 8, 128, 1>(0),
     make_variant<2, 1, 32, 1, float, kUF | kSB | kFX | kMG>(),
     make_variant<2, 2, 64, 1, float, kUF | kSB | kFX | kMG>(),
     make_variant<2, 1, 32, 1, float, kUF | kSB | kFX>(),

@@ -7,13 +7,14 @@
 // general-geometry (kGE) entries only, the others never do.  The
 // first variant of each precision is the default (the measured best); dg_tune_stage may pick another.
 #include "dg_stage.cuh"
-#include "dg_column.cuh"
+#include "dg_small.cuh"
 #include "dg_tc.cuh"
 
 namespace dgk {
 
 static const StageVariant kVariants3[] = {
-    make_column_variant<3, 1, 32, double, 12, 3, 32, 1>(6),
+    make_small_variant<3, 1, 64, 4, 4, 3, double>(make_column_variant<3, 1, 32, double, 12, 3, 32, 1>(0)),
+    make_column_variant<3, 1, 32, double, 12, 3, 32, 1>(0),
     make_variant<3, 1, 96, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<3, 1, 128, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<3, 1, 128, 1, double, kUF | kRS | kSB | kFX | kMG>(),
@@ -29,7 +30,8 @@ static const StageVariant kVariants3[] = {
     make_variant<3, 1, 64, 1, double, kUF | kSB | kK1>(),
     make_variant<3, 1, 32, 2, double, kSB>(),
     make_variant<3, 2, 64, 2, double>(),
-    make_column_variant<3, 1, 32, float, 16, 5, 64, 1>(10),
+    make_small_variant<3, 1, 64, 4, 8, 1, float>(make_column_variant<3, 1, 32, float, 16, 5, 64, 1>(0)),
+    make_column_variant<3, 1, 32, float, 16, 5, 64, 1>(0),
     make_variant<3, 1, 128, 1, float, kUF | kSB | kFX | kMG>(),
     make_variant<3, 1, 128, 1, float, kUF | kRS | kSB | kFX | kMG>(),
     make_variant<3, 1, 64, 1, float, kUF | kSB | kFX | kMG>(),

@@ -7,12 +7,13 @@
 // general-geometry (kGE) entries only, the others never do.  The
 // first variant of each precision is the default (the measured best); dg_tune_stage may pick another.
 #include "dg_stage.cuh"
-#include "dg_column.cuh"
+#include "dg_small.cuh"
 
 namespace dgk {
 
 static const StageVariant kVariants4[] = {
-    make_column_variant<4, 1, 64, double, 4, 5, 64, 1>(3),
+    make_small_variant<4, 1, 64, 2, 4, 1, double>(make_column_variant<4, 1, 64, double, 4, 5, 64, 1>(0)),
+    make_column_variant<4, 1, 64, double, 4, 5, 64, 1>(0),
     make_variant<4, 1, 128, 1, double, kUF | kSB | kFX | kMG, 4>(),
     make_variant<4, 1, 96, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<4, 1, 128, 1, double, kUF | kSB | kFX, 4>(),
@@ -25,7 +26,8 @@ static const StageVariant kVariants4[] = {
     make_variant<4, 1, 128, 1, double, kUF | kRS | kSB | kK1>(),
     make_variant<4, 1, 96, 1, double, kUF | kRS | kSB | kK1>(),
     make_variant<4, 1, 64, 2, double>(),
-    make_column_variant<4, 1, 64, float, 8, 5, 64, 1>(6),
+    make_small_variant<4, 1, 64, 3, 6, 1, float>(make_column_variant<4, 1, 64, float, 8, 5, 64, 1>(0)),
+    make_column_variant<4, 1, 64, float, 8, 5, 64, 1>(0),
     make_variant<4, 1, 128, 1, float, kUF | kSB | kFX | kMG>(),
     make_variant<4, 1, 128, 1, float, kUF | kRS | kSB | kFX | kMG>(),
     make_variant<4, 1, 128, 1, float, kUF | kSB | kFX>(),

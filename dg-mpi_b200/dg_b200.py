@@ -544,7 +544,7 @@ class Case:
                                             ctypes.byref(pr))
             self._lib.dg_stage_variant_flags(self.order, v, ctypes.byref(fl))
             opts = "+".join(n for b, n in ((1, "pz"), (2, "sb"), (4, "uf"), (8, "rs"), (16, "k1"), (32, "ge"), (64, "fx"),
-                                           (128, "tc"), (4096, "mg"), (8192, "cf")) if fl.value & b)
+                                           (128, "tc"), (4096, "mg"), (8192, "cf"), (16384, "sm")) if fl.value & b)
             if (fl.value >> 8) & 15:
                 opts += ("+" if opts else "") + "mb%d" % ((fl.value >> 8) & 15)
             out.append((E.value, NT.value, G.value, "mixed_fp32" if pr.value == 1 else "fp64", opts))
