@@ -12,24 +12,28 @@
 // mult_inv_mass_matrix (tools.cpp:124-139) and the RK4 / FE stage updates
 // (stepper.cpp:23-142).
 //
-// Per element (one warp; shared memory per warp, no block barriers):
-//   load U [4][nb];  x and y interpolation to the (p+2)^2 Gauss points
-//   (sum-factorised: B is the 1D basis at the volume points); the Euler flux
-//   at each point (dgp::interior_flux on the state with a zero third
-//   momentum: the reference's 2D flux, functions.cpp:43-61, is the 3D one
-//   without the third components), times (ijac djac)(x) w_q; the x and y
-//   contractions with the 1D derivative and basis into the residual; for each
-//   of the 4 edges and each of its p+1 Gauss points the element's trace and
-//   the neighbour's (only the edge's p+1 nodes carry the trace of an
-//   equidistant Lagrange basis, the others vanish there exactly, so the sums
-//   equal the reference's dense B_f U term by term), the numerical flux in the
-//   reference's L/R roles with the left element's normal (dgp::flux_*, the
-//   2D Lax-Friedrichs / HLLC of functions.cpp:196-297 being the 3D ones on
-//   (nx, ny, 0)), times the edge weight, -F on the left and +F on the right;
-//   the lift of the four edges into the residual; the Kronecker inverse mass
-//   over det J and the fused RK / FE update.  Each edge flux is evaluated by
-//   both of its elements in the same argument order, so both see the same
-//   value.
+// Two launches per stage.
+//   edge2d_kernel   every interior edge's numerical flux once: one thread per
+//       (edge, Gauss point), the p + 1 threads of an edge in one warp.  Each holds
+//       one edge node of both sides (the other basis functions vanish on the edge
+//       exactly, so the traces equal the reference's dense B_f U term by term);
+//       traces, and the lift onto either side's nodes (-F on the left, +F on the
+//       right, times the edge weights), are sums over the warp's shuffles.
+//   stage2d_kernel  a warp per E = 32 / (p+2) elements, no block barriers: the x
+//       interpolation from the rows of a state to shared memory; one lane per
+//       quadrature column: the y interpolation to its p+2 points, the Euler flux,
+//       the contravariant transform and the y contraction in registers; the x
+//       contraction of a row, its edges' lifts, and the fused RK / FE update
+//       straight to global memory.  The 1D inverse mass is folded into the
+//       contraction tables and the lifts (the residual output takes the plain ones).
+// An edge that is no interior edge keeps a zero lift: it adds nothing, as in the
+// reference, whose residual loops over the interior faces.
+//
+// Why: the kernel this replaces ran one task per value through shared memory, two
+// loads to a multiply-add, and each edge's flux twice (512^2, p = 3: load/store and
+// issue bound at 31 % of the FP64 pipe).  RK stage, HLLC, 256^2: p = 1 108 -> 23, p = 2
+// 141 -> 42, p = 3 179 -> 60, p = 4 319 -> 103, p = 5 463 -> 135 us; 64^2, p = 3 16.5 ->
+// 9.8 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,7 +44,7 @@
 
 #include "../../include/dg_b200.h"
 #include "../host/numerics.h"
-#include "dg_physics.cuh"
+#include "dg_small.cuh"
 
 namespace dgi {
 int fail(dg_ctx* c, int code, const std::string& msg);
@@ -50,19 +54,19 @@ namespace d2 {
 
 constexpr int kNS = 4;
 constexpr int kMaxN = 6, kMaxM = 7;
-constexpr int kWarps = 4;  // elements in flight per CTA
+
+constexpr int kSyncWord = 32, kStatusWords = 96;  // the status word, and two counters kSyncWord words on
 
 enum Mode : int { kResidual = 0, kRK1 = 2, kRK2 = 3, kRK3 = 4, kRK4 = 5, kFE = 6 };
 enum Status : unsigned { kRho = 1u, kPressure = 2u, kNaN = 4u, kHLLC = 8u };
 
-// the order's tables (copied to shared memory by every CTA)
+// the order's tables of the edges (copied to shared memory by every CTA): trace
+// of edge node m at edge point j of face f, its product with the 1D inverse mass
+// (the lift of the update), and the weights
 struct Tab {
-    double B[kMaxM * kMaxN], D[kMaxM * kMaxN], wv[kMaxM];  // volume: [q][i]
-    double FB[4 * kMaxN * kMaxN];                          // [f][j][m]: edge node m at edge point j
-    double fw[kMaxN];                                      // edge weights
-    double Minv[kMaxN * kMaxN];                            // 1D inverse mass
-    int fnode[4 * kMaxN];                                  // [f][m]: basis index of edge node m (ascending)
-    int lift[4 * kMaxN * kMaxN];                           // [f][b]: m with fnode[f][m] == b, else -1
+    double FB[4 * kMaxN * kMaxN];  // [f][j][m]
+    double MF[4 * kMaxN * kMaxN];
+    double fw[kMaxN];
 };
 
 struct Geo {
@@ -71,10 +75,15 @@ struct Geo {
     double pad[3];
 };
 
-struct Face {
-    int nbr;
-    int code;  // neighbour face | role << 2 (0 left, 1 right) | flip << 3 | my orientation << 4
-    double N[2];
+// one interior edge, by its left element: unit normal as the numerical flux wants
+// it and |N|, both elements, and left face | right face << 2 | flip << 4 |
+// (left orientation) << 5
+struct Edge {
+    double n[2];
+    double nmag;
+    int eL, eR;
+    int code;
+    int pad;
 };
 
 struct Args {
@@ -83,231 +92,405 @@ struct Args {
     const double* U0;
     double* acc;
     const Geo* geo;
-    const Face* faces;
+    const Edge* edges;
+    double* elift;  // [ne][4 faces][4][n], zero for edges that are no interior ones
     const Tab* tab;
     unsigned* status;
-    int ne, mode, flux;
+    int ne, nedge, mode, flux;
     double dt, gamma;
+    // 1D tables: basis and weights at the volume points; contraction tables and end
+    // columns of the inverse mass (plain ones and the identity's for the residual)
+    double B[kMaxM * kMaxN], MB[kMaxM * kMaxN], MD[kMaxM * kMaxN], W[kMaxM];
+    double ME[2][kMaxN];
 };
+
+constexpr int kEdgeThreads = 128;
+
+__device__ __forceinline__ void load_tab(const Args& a, Tab& T)
+{
+    const double* src = reinterpret_cast<const double*>(a.tab);
+    double* dst = reinterpret_cast<double*>(&T);
+    for (int i = threadIdx.x; i < static_cast<int>(sizeof(Tab) / 8); i += blockDim.x) dst[i] = src[i];
+    __syncthreads();
+}
+
+// the edge of this lane in the batch of edges at i0
+template <int P>
+__device__ __forceinline__ Edge edge_of(const Args& a, int i0)
+{
+    const int k = (threadIdx.x & 31) / (P + 1);
+    return a.edges[k < 32 / (P + 1) && i0 + k < a.nedge ? i0 + k : a.nedge - 1];
+}
+
+// the edges of warp `warp` of nwarp, at the state Us; `held`: the warp's only batch
+// of edges, read before
+template <int P>
+__device__ __forceinline__ void edge_phase(const Args& a, const double* Us, int mode, const Tab& T, int warp, int nwarp,
+                                           unsigned& status, const Edge* held = nullptr)
+{
+    constexpr int N = P + 1, NB = N * N, EPW = 32 / N;  // edges per warp
+    const double* C = mode == kResidual ? T.FB : T.MF;
+    const int lane = threadIdx.x & 31, k = lane / N, j = lane - k * N;
+    for (int i0 = warp * EPW; i0 < a.nedge; i0 += nwarp * EPW) {
+        const bool on = k < EPW && i0 + k < a.nedge;
+        const Edge ed = held ? *held : edge_of<P>(a, i0);
+        const int fL = ed.code & 3, fR = (ed.code >> 2) & 3, flip = (ed.code >> 4) & 1, mine = (ed.code >> 5) & 1;
+        // edge node m of face f: basis index o + m s
+        auto node = [](int f, int m) { return (f == 1 ? N - 1 : f == 2 ? (N - 1) * N : 0) + m * (f == 1 || f == 3 ? N : 1); };
+        const int jr = flip ? N - 1 - j : j;           // the right side's point
+        const int q = mine ? N - 1 - j : j;            // the face's quadrature point
+        const double* pL = Us + static_cast<size_t>(ed.eL) * kNS * NB + node(fL, j);
+        const double* pR = Us + static_cast<size_t>(ed.eR) * kNS * NB + node(fR, j);
+        double uL[kNS], uR[kNS], tL[N], tR[N];
+#pragma unroll
+        for (int v = 0; v < kNS; ++v) {
+            uL[v] = pL[v * NB];
+            uR[v] = pR[v * NB];
+        }
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            tL[m] = T.FB[(fL * N + j) * N + m];
+            tR[m] = T.FB[(fR * N + jr) * N + m];
+        }
+        constexpr int s3[4] = {0, 1, 2, 4};
+        double UL[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, UR[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int v = 0; v < kNS; ++v) {
+            double sl = 0.0, sr = 0.0;
+#pragma unroll
+            for (int m = 0; m < N; ++m) {
+                sl += tL[m] * __shfl_sync(0xffffffffu, uL[v], k * N + m);
+                sr += tR[m] * __shfl_sync(0xffffffffu, uR[v], k * N + m);
+            }
+            UL[s3[v]] = sl;
+            UR[s3[v]] = sr;
+        }
+        const double n3[3] = {ed.n[0], ed.n[1], 0.0};
+        double F5[5];
+        unsigned bad = 0;
+        if (a.flux == DG_FLUX_HLLC) {
+            if (!dgp::flux_hllc_n(a.gamma, UL, UR, n3, ed.nmag, F5)) bad = kHLLC;
+        } else {
+            dgp::flux_lax_friedrichs_sq(a.gamma, UL, UR, n3, ed.nmag, F5);
+        }
+        if (on) status |= bad;
+        const double w = T.fw[q];
+        double* oL = a.elift + (static_cast<size_t>(ed.eL) * 4 + fL) * kNS * N + j;
+        double* oR = a.elift + (static_cast<size_t>(ed.eR) * 4 + fR) * kNS * N + j;
+#pragma unroll
+        for (int v = 0; v < kNS; ++v) {
+            const double F = F5[s3[v]] * w;
+            double sl = 0.0, sr = 0.0;
+#pragma unroll
+            for (int m = 0; m < N; ++m) {  // point m; node j of either side
+                const double Fm = __shfl_sync(0xffffffffu, F, k * N + m);
+                sl += C[(fL * N + m) * N + j] * Fm;
+                sr += C[(fR * N + (flip ? N - 1 - m : m)) * N + j] * Fm;
+            }
+            if (on) {
+                oL[v * N] = -sl;
+                oR[v * N] = sr;
+            }
+        }
+    }
+}
+
+template <int P>
+__global__ void __launch_bounds__(kEdgeThreads) edge2d_kernel(const __grid_constant__ Args a)
+{
+    __shared__ Tab T;
+    load_tab(a, T);
+    unsigned status = 0;
+    edge_phase<P>(a, a.Us, a.mode, T, (blockIdx.x * kEdgeThreads + threadIdx.x) >> 5, gridDim.x * kEdgeThreads / 32, status);
+    if (status) atomicOr(a.status, status);
+}
 
 template <int P>
 struct Cfg {
-    static constexpr int N = P + 1, M = P + 2, NB = N * N, NQ = M * M, NF = P + 1;
-    // per-warp shared memory (doubles): U, R, the interpolation / contraction
-    // area (T1 + Uq, later H), the point fluxes G, the edge fluxes Fe
-    static constexpr int kU = 0, kR = kU + kNS * NB, kA = kR + kNS * NB;
-    static constexpr int kAsz = kNS * N * M + kNS * M * M;  // >= 2 kNS M N (M > N)
-    static constexpr int kG = kA + kAsz, kFe = kG + 2 * kNS * NQ, kEnd = kFe + 4 * NF * kNS;
+    static constexpr int N = P + 1, M = P + 2, NB = N * N;
+    static constexpr int E = 32 / M;                    // elements per warp, one lane per column
+    static constexpr int MS = M | 1;                    // odd row stride
+    static constexpr int kA = 2 * kNS * N * MS;         // [d][v][j][qx]
+    static constexpr int ES = kA + ((M - kA) % 16 + 16) % 16;  // = M modulo 16: the elements' columns follow one another over the banks
+    static constexpr int kRows = E * kNS * N, R = (kRows + 31) / 32;
+    static constexpr int kL = 4 * kNS * N;              // an element's lifts
+    static constexpr size_t smem = sizeof(double) * ((static_cast<size_t>(E) * (ES + kL) + 2 * N + 1) / 2 * 2);
 };
 
-constexpr size_t kTabDoubles = (sizeof(Tab) + 7) / 8;
-
-template <int P>
-__global__ void __launch_bounds__(32 * kWarps) stage2d_kernel(const Args a)
+// the batches of warp `warp` of nwarp; sm: the warp's shared memory. With LATE the
+// batch's lifts are there only once lifts_ready() has returned true (false: give up).
+template <int P, bool LATE, typename Ready>
+__device__ __forceinline__ void stage_phase(const Args& a, const double* Us, const double* U0, double* out, int mode, double* sm,
+                                            int warp, int nwarp, unsigned& status, Ready&& lifts_ready)
 {
     using C = Cfg<P>;
-    constexpr int N = C::N, M = C::M, NB = C::NB, NQ = C::NQ, NF = C::NF;
-    extern __shared__ double sm[];
-    Tab& T = *reinterpret_cast<Tab*>(sm);
-    {
-        const double* src = reinterpret_cast<const double*>(a.tab);
-        for (int i = threadIdx.x; i < static_cast<int>(kTabDoubles); i += blockDim.x) sm[i] = src[i];
-    }
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* W = sm + kTabDoubles + static_cast<size_t>(warp) * C::kEnd;
-    double* U = W + C::kU;
-    double* R = W + C::kR;
-    double* T1 = W + C::kA;               // [v][j][qx]
-    double* Uq = T1 + kNS * N * M;        // [v][qy][qx]
-    double* H = W + C::kA;                // [d][v][qy][i], after Uq is dead
-    double* G = W + C::kG;                // [d][v][qy][qx]
-    double* Fe = W + C::kFe;              // [f][j][v]
-    unsigned status = 0;
-    const double gam = a.gamma;
-    for (int e = blockIdx.x * kWarps + warp; e < a.ne; e += gridDim.x * kWarps) {
-        const double* Ue = a.Us + static_cast<size_t>(e) * kNS * NB;
-        for (int i = lane; i < kNS * NB; i += 32) U[i] = Ue[i];
-        const Geo g = a.geo[e];
-        __syncwarp();
-        // x interpolation: T1[v][j][qx] = sum_i B[qx][i] U[v][j][i]
-        for (int t = lane; t < kNS * N * M; t += 32) {
-            const int qx = t % M, j = (t / M) % N, v = t / (M * N);
-            double s = 0.0;
+    constexpr int N = C::N, M = C::M, NB = C::NB, E = C::E, MS = C::MS, ES = C::ES, R = C::R, kRows = C::kRows, MN = M * N;
+    double* sL = sm;                      // [E][4][4][N]
+    double* sA = sL + E * C::kL;          // [E][ES]: x-interpolated rows, then the y-contracted columns
+    double* sM = sA + E * ES;             // [2][N]
+    const int lane = threadIdx.x & 31;
+    if (lane < 2 * N) sM[lane] = a.ME[lane / N][lane % N];
+    const bool need_u0 = mode >= kRK1, need_acc = mode == kRK2 || mode == kRK3 || mode == kRK4;
+    const bool put_acc = mode == kRK1 || mode == kRK2 || mode == kRK3, sum_acc = mode == kRK4;
+    const double cu = mode == kRK1 || mode == kRK2 ? 0.5 : (sum_acc ? 1.0 / 6.0 : 1.0), ca = mode == kRK1 ? 1.0 : 2.0;
+    double un[R][N];  // rows (e, v, j), fetched a batch ahead
+    auto fetch = [&](int e0) {
 #pragma unroll
-            for (int i = 0; i < N; ++i) s += T.B[qx * N + i] * U[v * NB + j * N + i];
-            T1[t] = s;
+        for (int r = 0; r < R; ++r) {
+            const int i = lane + 32 * r, e = i / (kNS * N), row = i - e * (kNS * N);
+            if (i < kRows) dgk::load_row<N>(Us + (static_cast<size_t>(min(e0 + e, a.ne - 1)) * kNS * N + row) * N, un[r]);
+        }
+    };
+    const int stride = nwarp * E;
+    int e0 = warp * E;
+    if (e0 < a.ne) fetch(e0);
+    for (; e0 < a.ne; e0 += stride) {
+        // the batch's lifts, for the last pass
+        auto get_lifts = [&]() {
+            const int nl = min(E, a.ne - e0) * C::kL;
+            for (int i = 2 * lane; i < nl; i += 64) dgk::cp_async16(sL + i, a.elift + static_cast<size_t>(e0) * C::kL + i);
+            dgk::cp_async_commit();
+        };
+        if constexpr (!LATE) get_lifts();
+        // x interpolation
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = lane + 32 * r, e = i / (kNS * N), row = i - e * (kNS * N);
+            if (i < kRows) {
+                double* o = sA + e * ES + row * MS;
+#pragma unroll
+                for (int q = 0; q < M; ++q) {
+                    double s = 0.0;
+#pragma unroll
+                    for (int b = 0; b < N; ++b) s += dgk::sym<MN>(a.B, q * N + b) * un[r][b];
+                    o[q] = s;
+                }
+            }
         }
         __syncwarp();
-        // y interpolation: Uq[v][qy][qx] = sum_j B[qy][j] T1[v][j][qx]
-        for (int t = lane; t < kNS * NQ; t += 32) {
-            const int qx = t % M, qy = (t / M) % M, v = t / NQ;
-            double s = 0.0;
-#pragma unroll
-            for (int j = 0; j < N; ++j) s += T.B[qy * N + j] * T1[(v * N + j) * M + qx];
-            Uq[t] = s;
-        }
-        __syncwarp();
-        // pointwise flux times (ijac djac)(x) w
-        for (int q = lane; q < NQ; q += 32) {
-            const double u5[5] = {Uq[q], Uq[NQ + q], Uq[2 * NQ + q], 0.0, Uq[3 * NQ + q]};
-            double F[15];
-            dgp::interior_flux(gam, u5, F);
-            const double p = dgp::pressure(gam, u5);
-            if (!(u5[0] > 0.0)) status |= kRho;
-            if (!(p > 0.0)) status |= kPressure;
-            if (u5[0] != u5[0] || p != p) status |= kNaN;
-            const double w = T.wv[q % M] * T.wv[q / M];
-            constexpr int s3[4] = {0, 1, 2, 4};
+        // columns: y interpolation, flux, contravariant transform, y contraction
+        if (lane < E * M) {
+            const int e = lane / M, qx = lane - e * M;
+            double* col = sA + e * ES + qx;
+            const Geo* g = a.geo + min(e0 + e, a.ne - 1);
+            double S[kNS][M];
 #pragma unroll
             for (int v = 0; v < kNS; ++v) {
-                const double fx = F[s3[v]], fy = F[5 + s3[v]];
+                double x[N];
 #pragma unroll
-                for (int d = 0; d < 2; ++d) G[(d * kNS + v) * NQ + q] = (fx * g.jd[d * 2 + 0] + fy * g.jd[d * 2 + 1]) * w;
+                for (int b = 0; b < N; ++b) x[b] = col[(v * N + b) * MS];
+#pragma unroll
+                for (int q = 0; q < M; ++q) {
+                    double s = 0.0;
+#pragma unroll
+                    for (int b = 0; b < N; ++b) s += dgk::sym<MN>(a.B, q * N + b) * x[b];
+                    S[v][q] = s;
+                }
             }
-        }
-        __syncwarp();
-        // x contraction: H0 = D^T along x of G0, H1 = B^T along x of G1
-        for (int t = lane; t < 2 * kNS * M * N; t += 32) {
-            const int i = t % N, qy = (t / N) % M, dv = t / (N * M);
-            const double* Op = dv < kNS ? T.D : T.B;
-            const double* g0 = G + dv * NQ + qy * M;
-            double s = 0.0;
+            const double jd[4] = {g->jd[0], g->jd[1], g->jd[2], g->jd[3]};
+            double V[2][M], p[M];
+            bool sound = true;
 #pragma unroll
-            for (int qx = 0; qx < M; ++qx) s += Op[qx * N + i] * g0[qx];
-            H[t] = s;
-        }
-        __syncwarp();
-        // y contraction into the residual
-        for (int t = lane; t < kNS * NB; t += 32) {
-            const int i = t % N, j = (t / N) % N, v = t / NB;
-            const double* h0 = H + (v * M) * N + i;
-            const double* h1 = H + ((kNS + v) * M) * N + i;
-            double s = 0.0;
+            for (int q = 0; q < M; ++q) {
+                const double r1 = 1. / S[0][q];
+                const double u = S[1][q] * r1, v = S[2][q] * r1;
+                p[q] = (a.gamma - 1.0) * (S[3][q] - 0.5 * (S[1][q] * u + S[2][q] * v));
+                sound = sound && S[0][q] > 0.0 && p[q] > 0.0;  // a NaN is not
+                if (!sound) {
+                    if (!(S[0][q] > 0.0)) status |= kRho;
+                    if (!(p[q] > 0.0)) status |= kPressure;
+                    if (S[0][q] != S[0][q] || p[q] != p[q]) status |= kNaN;
+                }
+                const double w = a.W[qx] * a.W[q];
+                S[3][q] += p[q];
 #pragma unroll
-            for (int qy = 0; qy < M; ++qy) s += T.B[qy * N + j] * h0[qy * N] + T.D[qy * N + j] * h1[qy * N];
-            R[t] = s;
-        }
-        // edges: one lane per (face, point)
-        if (lane < 4 * NF) {
-            const int f = lane / NF, j = lane % NF;
-            const Face fr = a.faces[static_cast<size_t>(e) * 4 + f];
-            if (fr.nbr < 0) {
+                for (int d = 0; d < 2; ++d) V[d][q] = (u * jd[d * 2] + v * jd[d * 2 + 1]) * w;
+                p[q] *= w;
+            }
 #pragma unroll
-                for (int v = 0; v < kNS; ++v) Fe[(f * NF + j) * kNS + v] = 0.0;
-            } else {
-                const int nf = fr.code & 3, role = (fr.code >> 2) & 1, flip = (fr.code >> 3) & 1, mine = (fr.code >> 4) & 1;
-                const int jn = flip ? NF - 1 - j : j;
-                const int q = mine ? NF - 1 - j : j;  // the face's quadrature point
-                const double* Un = a.Us + static_cast<size_t>(fr.nbr) * kNS * NB;
-                double uo[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, un[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-                constexpr int s3[4] = {0, 1, 2, 4};
-    #pragma unroll
-                for (int v = 0; v < kNS; ++v) {
-                    double so = 0.0, sn = 0.0;
-    #pragma unroll
-                    for (int m = 0; m < N; ++m) {
-                        so += T.FB[(f * N + j) * N + m] * U[v * NB + T.fnode[f * N + m]];
-                        sn += T.FB[(nf * N + jn) * N + m] * __ldg(Un + v * NB + T.fnode[nf * N + m]);
+            for (int v = 0; v < kNS; ++v) {
+                double a0[N], a1[N];
+#pragma unroll
+                for (int b = 0; b < N; ++b) { a0[b] = 0.0; a1[b] = 0.0; }
+#pragma unroll
+                for (int q = 0; q < M; ++q) {
+                    double g0 = S[v][q] * V[0][q], g1 = S[v][q] * V[1][q];
+                    if (v == 1 || v == 2) {
+                        g0 += p[q] * jd[v - 1];
+                        g1 += p[q] * jd[2 + v - 1];
                     }
-                    uo[s3[v]] = so;
-                    un[s3[v]] = sn;
+#pragma unroll
+                    for (int b = 0; b < N; ++b) {
+                        a0[b] += dgk::sym<MN>(a.MB, q * N + b) * g0;
+                        a1[b] += dgk::asym<MN>(a.MD, q * N + b) * g1;
+                    }
                 }
-                const double* UL = role == 0 ? uo : un;
-                const double* UR = role == 0 ? un : uo;
-                const double N3[3] = {fr.N[0], fr.N[1], 0.0};
-                double F5[5];
-                if (a.flux == DG_FLUX_HLLC) {
-                    if (!dgp::flux_hllc(gam, UL, UR, N3, F5)) status |= kHLLC;
-                } else {
-                    dgp::flux_lax_friedrichs(gam, UL, UR, N3, F5);
+#pragma unroll
+                for (int b = 0; b < N; ++b) {
+                    col[(v * N + b) * MS] = a0[b];
+                    col[(kNS * N + v * N + b) * MS] = a1[b];
                 }
-                const double sgn = role == 0 ? -1.0 : 1.0;
-    #pragma unroll
-                for (int v = 0; v < kNS; ++v) Fe[(f * NF + j) * kNS + v] = sgn * (F5[s3[v]] * T.fw[q]);
             }
         }
         __syncwarp();
-        // lift of the four edges: the edge nodes of b, face by face
-        for (int t = lane; t < kNS * NB; t += 32) {
-            const int b = t % NB, v = t / NB;
-            double s = 0.0;
+        if constexpr (LATE) {
+            if (!lifts_ready()) return;
+            get_lifts();
+        } else {
+            fetch(e0 + stride);  // past the end: the last element again
+        }
+        dgk::cp_async_wait_all();
+        __syncwarp();
+        // x contraction, the row's edges (bottom 0, right 1, top 2, left 3) and the update
+#pragma unroll 1
+        for (int i = lane; i < kRows; i += 32) {
+            const int e = i / (kNS * N), row = i - e * (kNS * N), v = row / N, jy = row - v * N;
+            const int ge = min(e0 + e, a.ne - 1);
+            const size_t gi = (static_cast<size_t>(ge) * kNS * N + row) * N;
+            double u0[N] = {}, ac[N] = {};
+            if (need_u0) dgk::load_row<N>(U0 + gi, u0);
+            if (need_acc) dgk::load_row<N>(a.acc + gi, ac);
+            const double* A0 = sA + e * ES + row * MS;
+            double x[N];
 #pragma unroll
-            for (int f = 0; f < 4; ++f) {
-                const int m = T.lift[f * kMaxN * kMaxN + b];
-                if (m >= 0)
+            for (int b = 0; b < N; ++b) x[b] = 0.0;
 #pragma unroll
-                    for (int j = 0; j < NF; ++j) s += T.FB[(f * N + j) * N + m] * Fe[(f * NF + j) * kNS + v];
+            for (int q = 0; q < M; ++q) {
+                const double c0 = A0[q], c1 = A0[kNS * N * MS + q];
+#pragma unroll
+                for (int b = 0; b < N; ++b)
+                    x[b] = dgk::add_two(x[b], dgk::asym<MN>(a.MD, q * N + b), c0, dgk::sym<MN>(a.MB, q * N + b), c1);
             }
-            R[t] += s;
-        }
-        __syncwarp();
-        double* Oe = a.out + static_cast<size_t>(e) * kNS * NB;
-        if (a.mode == kResidual) {
-            for (int i = lane; i < kNS * NB; i += 32) Oe[i] = R[i];
-            __syncwarp();
-            continue;
-        }
-        // inverse mass: (Minv x Minv) R / det J, x then y; then the stage update
-        for (int t = lane; t < kNS * NB; t += 32) {
-            const int i = t % N, jv = t / N;
-            double s = 0.0;
+            const double* Lv = sL + e * C::kL + v * N;
+            const double m0 = sM[jy], m1 = sM[N + jy], l3 = Lv[3 * kNS * N + jy], l1 = Lv[kNS * N + jy];
+            const double scale = mode == kResidual ? 1.0 : a.dt * a.geo[ge].idj;
+            if (e0 + e >= a.ne) continue;
+            double k[N], o[N];
 #pragma unroll
-            for (int k = 0; k < N; ++k) s += T.Minv[i * N + k] * R[jv * N + k];
-            T1[t] = s;
-        }
-        __syncwarp();
-        const double* U0e = a.U0 + static_cast<size_t>(e) * kNS * NB;
-        double* Ae = a.acc + static_cast<size_t>(e) * kNS * NB;
-        for (int t = lane; t < kNS * NB; t += 32) {
-            const int i = t % N, j = (t / N) % N, v = t / NB;
-            double s = 0.0;
-#pragma unroll
-            for (int k = 0; k < N; ++k) s += T.Minv[j * N + k] * T1[(v * N + k) * N + i];
-            const double kk = a.dt * (s * g.idj);
-            const double u0 = U0e[t];
-            switch (a.mode) {
-                case kRK1: Ae[t] = kk; Oe[t] = 0.5 * kk + u0; break;
-                case kRK2: Ae[t] = Ae[t] + 2.0 * kk; Oe[t] = 0.5 * kk + u0; break;
-                case kRK3: Ae[t] = Ae[t] + 2.0 * kk; Oe[t] = 1.0 * kk + u0; break;
-                case kRK4: Oe[t] = u0 + (1.0 / 6.0) * (Ae[t] + kk); break;
-                default: Oe[t] = u0 + kk; break;
+            for (int b = 0; b < N; ++b) {
+                double s = x[b];
+                s += m0 * Lv[b];
+                s += m1 * Lv[2 * kNS * N + b];
+                s += a.ME[0][b] * l3;
+                s += a.ME[1][b] * l1;
+                k[b] = scale * s;
             }
+            if (put_acc) {
+                double ao[N];
+#pragma unroll
+                for (int b = 0; b < N; ++b) ao[b] = ac[b] + ca * k[b];
+                dgk::store_row<N>(a.acc + gi, ao);
+            }
+#pragma unroll
+            for (int b = 0; b < N; ++b) o[b] = u0[b] + cu * (sum_acc ? ac[b] + k[b] : k[b]);
+            dgk::store_row<N>(out + gi, o);
         }
-        __syncwarp();
+        __syncwarp();  // the columns and the lifts are the next batch's
     }
-    // one atomic per warp
-    for (int off = 16; off > 0; off >>= 1) status |= __shfl_xor_sync(0xffffffffu, status, off);
-    if (lane == 0 && status) atomicOr(a.status, status);
 }
 
-template <int P>
-size_t smem_bytes()
+// one warp per CTA; registers for MB resident warps per SM
+template <int P, int MB>
+__global__ void __launch_bounds__(32, MB) stage2d_kernel(const __grid_constant__ Args a)
 {
-    return (kTabDoubles + static_cast<size_t>(kWarps) * Cfg<P>::kEnd) * sizeof(double);
+    extern __shared__ __align__(16) double sm[];
+    unsigned status = 0;
+    stage_phase<P, false>(a, a.Us, a.U0, a.out, a.mode, sm, blockIdx.x, gridDim.x, status, []() { return true; });
+    if (status) atomicOr(a.status, status);
+}
+
+// RK4 steps of a small mesh in one cooperative launch, as small_steps_kernel
+// (dg_small.cuh) runs them in 3D: every stage warp keeps one batch of elements and
+// goes up to the y contraction while the edge warps compute the stage's lifts; two
+// counters order them, each wait bounded. Taken while every stage warp has at most
+// one batch, where it beats the two launches by their latency (stage, HLLC: 32^2,
+// p = 1 7.3 -> 6.4, p = 3 8.3 -> 6.7, p = 5 11.4 -> 7.6 us).
+struct StepArgs {
+    Args a;
+    double *U0, *Ua, *Ub;
+    int nsteps;
+    unsigned* sync;  // [0] arrivals of the stage warps, [32] of the edge warps, one per block and stage
+    unsigned base;   // both values before the launch
+};
+constexpr int kStageWarps = 4, kEdgeWarps = 4, kStepThreads = 32 * (kStageWarps + kEdgeWarps);
+
+template <int P>
+__global__ void __launch_bounds__(kStepThreads, 1) steps2d_kernel(const __grid_constant__ StepArgs s)
+{
+    extern __shared__ __align__(16) double sm[];
+    __shared__ Tab T;
+    __shared__ int dead[2];
+    if (threadIdx.x < 2) dead[threadIdx.x] = 0;
+    load_tab(s.a, T);
+    const int w = threadIdx.x / 32, nb = gridDim.x;
+    unsigned status = 0, target = s.base;
+    const int ew = (w - kStageWarps) * nb + blockIdx.x, epw = 32 / (P + 1);  // edge warps: index, edges to a batch
+    const bool once = w >= kStageWarps && (ew + nb * kEdgeWarps) * epw >= s.a.nedge && s.a.nedge > 0;
+    const Edge held = once ? edge_of<P>(s.a, ew * epw) : Edge{};
+    bool ok = true;
+    for (int step = 0; step < s.nsteps && ok; ++step)
+#pragma unroll 1
+        for (int stage = 1; stage <= 4 && ok; ++stage) {
+            const double* Us = stage == 1 ? s.U0 : stage == 3 ? s.Ub : s.Ua;
+            double* out = stage == 4 ? s.U0 : stage == 2 ? s.Ub : s.Ua;
+            if (w < kStageWarps) {
+                target += nb;
+                auto ready = [&]() {
+                    return ok = dgk::role_wait<32 * kStageWarps>(s.sync + 32, target, s.a.status, dead, 1, threadIdx.x);
+                };
+                const int warp = w * nb + blockIdx.x;
+                if (warp * Cfg<P>::E < s.a.ne)
+                    stage_phase<P, true>(s.a, Us, s.U0, out, kRK1 + stage - 1, sm + w * (Cfg<P>::smem / sizeof(double)), warp,
+                                         nb * kStageWarps, status, ready);
+                else
+                    ready();
+                if (ok) dgk::role_arrive<32 * kStageWarps>(s.sync, 1, threadIdx.x);
+            } else {
+                const int t = threadIdx.x - 32 * kStageWarps;
+                if (step > 0 || stage > 1) {
+                    target += nb;
+                    ok = dgk::role_wait<32 * kEdgeWarps>(s.sync, target, s.a.status, dead + 1, 2, t);
+                    if (!ok) break;
+                }
+                edge_phase<P>(s.a, Us, kRK1 + stage - 1, T, ew, nb * kEdgeWarps, status, once ? &held : nullptr);
+                dgk::role_arrive<32 * kEdgeWarps>(s.sync + 32, 2, t);
+            }
+        }
+    if (status) atomicOr(s.a.status, status);
 }
 
 using KernelFn = void (*)(const Args);
-KernelFn kernel_of(int p)
+struct Kernels {
+    KernelFn edge, stage;
+    void (*steps)(const StepArgs);
+    size_t smem;
+    int elems, edges_per_warp;
+};
+template <int P, int MB>
+constexpr Kernels kernels()
+{
+    return Kernels{edge2d_kernel<P>, stage2d_kernel<P, MB>, steps2d_kernel<P>, Cfg<P>::smem, Cfg<P>::E, 32 / (P + 1)};
+}
+Kernels kernels_of(int p)
 {
     switch (p) {
-        case 0: return stage2d_kernel<0>;
-        case 1: return stage2d_kernel<1>;
-        case 2: return stage2d_kernel<2>;
-        case 3: return stage2d_kernel<3>;
-        case 4: return stage2d_kernel<4>;
-        default: return stage2d_kernel<5>;
+        case 0: return kernels<0, 16>();
+        case 1: return kernels<1, 16>();
+        case 2: return kernels<2, 16>();
+        case 3: return kernels<3, 16>();
+        case 4: return kernels<4, 12>();
+        default: return kernels<5, 12>();
     }
 }
-size_t smem_of(int p)
+
+// [ne][4][nb] <-> [ne][nb][4]
+__global__ void transpose2d_kernel(const double* __restrict__ src, double* __restrict__ dst, long long n, int nb, int to_host)
 {
-    switch (p) {
-        case 0: return smem_bytes<0>();
-        case 1: return smem_bytes<1>();
-        case 2: return smem_bytes<2>();
-        case 3: return smem_bytes<3>();
-        case 4: return smem_bytes<4>();
-        default: return smem_bytes<5>();
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const long long e = i / (kNS * nb);
+        const int r = static_cast<int>(i - e * kNS * nb);
+        if (to_host) dst[i] = src[(e * kNS + r % kNS) * nb + r / kNS];
+        else dst[i] = src[(e * nb + r % nb) * kNS + r / nb];
     }
 }
 
@@ -318,26 +501,17 @@ size_t smem_of(int p)
 constexpr int kFaceNodes[4][2] = {{0, 1}, {1, 3}, {3, 2}, {2, 0}};
 constexpr double kRefX[4] = {-1., 1., -1., 1.}, kRefY[4] = {-1., -1., 1., 1.};
 
-// the order's tables: volume rule of (p+2) points per direction, edge rule of
-// p+1 points, edge traces from the 2D basis at the edge points computed as
+// the order's edge tables: rule of p+1 points, edge traces from the 2D basis at
+// the edge points computed as
 // get_points_on_face_quadrilateral and get_lagrange_basis_val_2D do
 bool make_tab(int p, const dgh::Tables1D& t1, Tab& T)
 {
     std::memset(&T, 0, sizeof(T));
-    const int n = p + 1, m = p + 2, nf = p + 1;
-    for (int q = 0; q < m; ++q) {
-        T.wv[q] = t1.wq[q];
-        for (int i = 0; i < n; ++i) {
-            T.B[q * n + i] = t1.B[q * n + i];
-            T.D[q * n + i] = t1.D[q * n + i];
-        }
-    }
-    for (int i = 0; i < n * n; ++i) T.Minv[i] = t1.Minv[i];
+    const int n = p + 1, nf = p + 1;
     std::vector<double> s, w;
     dgh::gauss_legendre(nf, s, w);
     for (int q = 0; q < nf; ++q) T.fw[q] = w[q];
     const std::vector<double> xn = dgh::equidistant_nodes(n);
-    for (int i = 0; i < 4 * kMaxN * kMaxN; ++i) T.lift[i] = -1;
     for (int f = 0; f < 4; ++f) {
         const int a = kFaceNodes[f][0], b = kFaceNodes[f][1];
         std::vector<double> val(static_cast<size_t>(nf) * n * n);
@@ -363,12 +537,17 @@ bool make_tab(int p, const dgh::Tables1D& t1, Tab& T)
                     if (std::fabs(val[static_cast<size_t>(q) * n * n + k]) > 1e-14) return false;
                 continue;
             }
-            T.fnode[f * n + cnt] = k;
-            T.lift[f * kMaxN * kMaxN + k] = cnt;
             for (int q = 0; q < nf; ++q) T.FB[(f * n + q) * n + cnt] = val[static_cast<size_t>(q) * n * n + k];
             ++cnt;
         }
         if (cnt != n) return false;
+        // the lift of the update: the edge's nodes through the 1D inverse mass
+        for (int q = 0; q < nf; ++q)
+            for (int mm = 0; mm < n; ++mm) {
+                double v = 0.0;
+                for (int k = 0; k < n; ++k) v += t1.Minv[mm * n + k] * T.FB[(f * n + q) * n + k];
+                T.MF[(f * n + q) * n + mm] = v;
+            }
     }
     return true;
 }
@@ -381,15 +560,18 @@ struct dg_ctx2d {
     cudaStream_t stream = nullptr;
     double *d_U0 = nullptr, *d_Ua = nullptr, *d_Ub = nullptr, *d_acc = nullptr, *d_res = nullptr;
     d2::Geo* d_geo = nullptr;
-    d2::Face* d_faces = nullptr;
+    d2::Edge* d_edges = nullptr;
+    double* d_elift = nullptr;
     d2::Tab* d_tab = nullptr;
     unsigned* d_status = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     double graph_dt = 0.0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    int grid = 1;
-    size_t smem = 0;
+    int nedge = 0, grid = 1, edge_grid = 1;
+    int step_grid = 0;       // blocks of the small-mesh steps, 0: the mesh is too large for them
+    unsigned sync_base = 0;  // their counters' value
+    d2::Args args{};  // tables and geometry of every launch
     dgh::Tables1D t1;
     std::vector<double> coords;  // [nnode][2]
     std::vector<unsigned> e2n;   // [ne][4]
@@ -422,7 +604,8 @@ void release(dg_ctx2d* c)
     cudaFree(c->d_acc);
     cudaFree(c->d_res);
     cudaFree(c->d_geo);
-    cudaFree(c->d_faces);
+    cudaFree(c->d_edges);
+    cudaFree(c->d_elift);
     cudaFree(c->d_tab);
     cudaFree(c->d_status);
     if (c->ev0) cudaEventDestroy(c->ev0);
@@ -432,21 +615,26 @@ void release(dg_ctx2d* c)
 
 int launch(dg_ctx2d* c, const double* Us, double* out, int mode, double dt)
 {
-    d2::Args a{};
+    d2::Args a = c->args;
     a.Us = Us;
     a.out = out;
     a.U0 = c->d_U0;
-    a.acc = c->d_acc;
-    a.geo = c->d_geo;
-    a.faces = c->d_faces;
-    a.tab = c->d_tab;
-    a.status = c->d_status;
-    a.ne = c->ne;
     a.mode = mode;
-    a.flux = c->flux;
     a.dt = dt;
-    a.gamma = c->gamma;
-    d2::kernel_of(c->p)<<<c->grid, 32 * d2::kWarps, c->smem, c->stream>>>(a);
+    if (mode == d2::kResidual) {  // no inverse mass
+        const int n = c->p + 1;
+        for (int i = 0; i < n * (n + 1); ++i) {
+            a.MB[i] = c->t1.B[i];
+            a.MD[i] = c->t1.D[i];
+        }
+        for (int b = 0; b < n; ++b) {
+            a.ME[0][b] = b == 0 ? 1.0 : 0.0;
+            a.ME[1][b] = b == n - 1 ? 1.0 : 0.0;
+        }
+    }
+    const d2::Kernels k = d2::kernels_of(c->p);
+    if (c->nedge > 0) k.edge<<<c->edge_grid, d2::kEdgeThreads, 0, c->stream>>>(a);
+    k.stage<<<c->grid, 32, k.smem, c->stream>>>(a);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? DG_OK : fail2(c, DG_ERR_CUDA, std::string("stage2d launch: ") + cudaGetErrorString(e));
 }
@@ -456,24 +644,35 @@ int check_status(dg_ctx2d* c)
     unsigned s = 0;
     DG2_CUDA(c, cudaMemcpyAsync(&s, c->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     DG2_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (s & dgk::kStatusTimeout) {
+        DG2_CUDA(c, cudaMemsetAsync(c->d_status, 0, d2::kStatusWords * sizeof(unsigned), c->stream));
+        DG2_CUDA(c, cudaStreamSynchronize(c->stream));
+        c->sync_base = 0;
+        return fail2(c, DG_ERR_TIMEOUT, "a bounded device wait gave up (status " + std::to_string(s) + ")");
+    }
     if (s) return fail2(c, DG_ERR_NONPHYSICAL, "non-physical state (status " + std::to_string(s) + ")");
     return DG_OK;
 }
 
-// host layout [ne][nb][4] <-> device layout [ne][4][nb]
-void to_device_layout(const double* h, double* d, int ne, int nb)
+// a state between its host layout [ne][nb][4] and device layout [ne][4][nb],
+// through the device scratch buffer `scratch`
+int to_device(dg_ctx2d* c, const double* h, double* d, double* scratch)
 {
-    for (int e = 0; e < ne; ++e)
-        for (int b = 0; b < nb; ++b)
-            for (int v = 0; v < d2::kNS; ++v)
-                d[(static_cast<size_t>(e) * d2::kNS + v) * nb + b] = h[(static_cast<size_t>(e) * nb + b) * d2::kNS + v];
+    const long long n = 1LL * c->ne * d2::kNS * c->nb;
+    DG2_CUDA(c, cudaMemcpyAsync(scratch, h, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    d2::transpose2d_kernel<<<1024, 256, 0, c->stream>>>(scratch, d, n, c->nb, 0);
+    DG2_CUDA(c, cudaGetLastError());
+    DG2_CUDA(c, cudaStreamSynchronize(c->stream));
+    return DG_OK;
 }
-void to_host_layout(const double* d, double* h, int ne, int nb)
+int to_host(dg_ctx2d* c, const double* d, double* h, double* scratch)
 {
-    for (int e = 0; e < ne; ++e)
-        for (int b = 0; b < nb; ++b)
-            for (int v = 0; v < d2::kNS; ++v)
-                h[(static_cast<size_t>(e) * nb + b) * d2::kNS + v] = d[(static_cast<size_t>(e) * d2::kNS + v) * nb + b];
+    const long long n = 1LL * c->ne * d2::kNS * c->nb;
+    d2::transpose2d_kernel<<<1024, 256, 0, c->stream>>>(d, scratch, n, c->nb, 1);
+    DG2_CUDA(c, cudaGetLastError());
+    DG2_CUDA(c, cudaMemcpyAsync(h, scratch, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    DG2_CUDA(c, cudaStreamSynchronize(c->stream));
+    return DG_OK;
 }
 
 // the IC families of the 2D path at (x, y): the 3D families at (x, y, 0)
@@ -519,6 +718,28 @@ void ref_to_phys(const dg_ctx2d* c, int e, double xi, double eta, double& x, dou
         x += gv[n] * c->coords[2 * c->e2n[4 * e + n]];
         y += gv[n] * c->coords[2 * c->e2n[4 * e + n] + 1];
     }
+}
+
+// RK4 steps of a small mesh, at most 256 to a launch (queued on the stream)
+int launch_steps(dg_ctx2d* c, double dt, int nsteps)
+{
+    const d2::Kernels k = d2::kernels_of(c->p);
+    d2::StepArgs s{};
+    s.a = c->args;
+    s.a.dt = dt;
+    s.U0 = c->d_U0;
+    s.Ua = c->d_Ua;
+    s.Ub = c->d_Ub;
+    s.sync = c->d_status + d2::kSyncWord;
+    for (int done = 0; done < nsteps; done += s.nsteps) {
+        s.nsteps = std::min(256, nsteps - done);
+        s.base = c->sync_base;
+        void* args[] = {&s};
+        DG2_CUDA(c, cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k.steps), dim3(c->step_grid), dim3(d2::kStepThreads),
+                                                args, k.smem * d2::kStageWarps, c->stream));
+        c->sync_base += static_cast<unsigned>(c->step_grid) * 4u * s.nsteps;
+    }
+    return DG_OK;
 }
 
 int prepare_graph(dg_ctx2d* c, double dt)
@@ -605,12 +826,12 @@ int dg2d_create(const dg_case_desc* cd, const dg_mesh2d_desc* md, dg_ctx2d** out
             geo[e].idj = 1.0 / det;
             c->djac[e] = det;
         }
-        // faces: per element and local face, the neighbour, its face, the
-        // roles and orientations, and the left element's normal; an edge that
-        // is no interior face (a boundary edge of a non-periodic mesh) keeps
-        // nbr = -1 and adds nothing, as the reference's residual, which loops
-        // over the interior faces only (base.cpp:470-561)
-        std::vector<d2::Face> faces(4 * static_cast<size_t>(c->ne), d2::Face{-1, 0, {0.0, 0.0}});
+        // interior edges: both elements and faces, the orientations, and the
+        // left element's normal (boundary edges of a non-periodic mesh are not
+        // listed: the reference's residual loops over the interior faces only,
+        // base.cpp:470-561)
+        std::vector<d2::Edge> edges;
+        edges.reserve(md->nface);
         std::vector<char> seen(4 * static_cast<size_t>(c->ne), 0);
         for (int f = 0; f < md->nface; ++f) {
             const unsigned* r = md->interior_faces + 8 * static_cast<size_t>(f);
@@ -631,8 +852,17 @@ int dg2d_create(const dg_case_desc* cd, const dg_mesh2d_desc* md, dg_ctx2d** out
             const double dx = XA[0] * g0 + XB[0] * g1, dy = XA[1] * g0 + XB[1] * g1;
             const double N0 = 1.0 * dy, N1 = -1.0 * 1.0 * dx;
             const int flip = static_cast<int>(oL ^ oR);
-            faces[4 * eL + fL] = d2::Face{static_cast<int>(eR), static_cast<int>(fR) | (0 << 2) | (flip << 3) | (static_cast<int>(oL) << 4), {N0, N1}};
-            faces[4 * eR + fR] = d2::Face{static_cast<int>(eL), static_cast<int>(fL) | (1 << 2) | (flip << 3) | (static_cast<int>(oR) << 4), {N0, N1}};
+            // N / |N| (base/functions.cpp:40-49), or N (1/|N|) as HLLC takes it
+            // (euler/functions.cpp:309-311)
+            const double nm = std::sqrt(N0 * N0 + N1 * N1), inv = 1. / nm;
+            d2::Edge ed{};
+            ed.n[0] = c->flux == DG_FLUX_HLLC ? N0 * inv : N0 / nm;
+            ed.n[1] = c->flux == DG_FLUX_HLLC ? N1 * inv : N1 / nm;
+            ed.nmag = nm;
+            ed.eL = static_cast<int>(eL);
+            ed.eR = static_cast<int>(eR);
+            ed.code = static_cast<int>(fL | fR << 2) | flip << 4 | static_cast<int>(oL) << 5;
+            edges.push_back(ed);
         }
         c->t1 = dgh::make_tables(c->p);
         d2::Tab tab;
@@ -640,35 +870,79 @@ int dg2d_create(const dg_case_desc* cd, const dg_mesh2d_desc* md, dg_ctx2d** out
 
         if (cudaSetDevice(c->device) != cudaSuccess) return bail(DG_ERR_CUDA, "cudaSetDevice failed");
         const size_t nstate = static_cast<size_t>(c->ne) * d2::kNS * c->nb * sizeof(double);
+        const size_t lift_bytes = static_cast<size_t>(c->ne) * 4 * d2::kNS * (c->p + 1) * sizeof(double);
+        c->nedge = static_cast<int>(edges.size());
         bool ok = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess &&
                   cudaEventCreate(&c->ev0) == cudaSuccess && cudaEventCreate(&c->ev1) == cudaSuccess &&
                   cudaMalloc((void**)&c->d_U0, nstate) == cudaSuccess && cudaMalloc((void**)&c->d_Ua, nstate) == cudaSuccess &&
                   cudaMalloc((void**)&c->d_Ub, nstate) == cudaSuccess && cudaMalloc((void**)&c->d_acc, nstate) == cudaSuccess &&
                   cudaMalloc((void**)&c->d_res, nstate) == cudaSuccess &&
                   cudaMalloc((void**)&c->d_geo, geo.size() * sizeof(d2::Geo)) == cudaSuccess &&
-                  cudaMalloc((void**)&c->d_faces, faces.size() * sizeof(d2::Face)) == cudaSuccess &&
+                  cudaMalloc((void**)&c->d_edges, std::max<size_t>(1, edges.size()) * sizeof(d2::Edge)) == cudaSuccess &&
+                  cudaMalloc((void**)&c->d_elift, lift_bytes) == cudaSuccess &&
                   cudaMalloc((void**)&c->d_tab, sizeof(d2::Tab)) == cudaSuccess &&
-                  cudaMalloc((void**)&c->d_status, sizeof(unsigned)) == cudaSuccess;
+                  cudaMalloc((void**)&c->d_status, d2::kStatusWords * sizeof(unsigned)) == cudaSuccess;
         if (!ok) {
             cudaGetLastError();
             return bail(DG_ERR_NOMEM, "device allocation failed");
         }
         ok = cudaMemcpy(c->d_geo, geo.data(), geo.size() * sizeof(d2::Geo), cudaMemcpyHostToDevice) == cudaSuccess &&
-             cudaMemcpy(c->d_faces, faces.data(), faces.size() * sizeof(d2::Face), cudaMemcpyHostToDevice) == cudaSuccess &&
+             (edges.empty() || cudaMemcpy(c->d_edges, edges.data(), edges.size() * sizeof(d2::Edge), cudaMemcpyHostToDevice) == cudaSuccess) &&
+             cudaMemset(c->d_elift, 0, lift_bytes) == cudaSuccess &&
              cudaMemcpy(c->d_tab, &tab, sizeof(d2::Tab), cudaMemcpyHostToDevice) == cudaSuccess &&
-             cudaMemset(c->d_status, 0, sizeof(unsigned)) == cudaSuccess &&
+             cudaMemset(c->d_status, 0, d2::kStatusWords * sizeof(unsigned)) == cudaSuccess &&
              cudaMemset(c->d_U0, 0, nstate) == cudaSuccess && cudaMemset(c->d_acc, 0, nstate) == cudaSuccess;
         if (!ok) return bail(DG_ERR_CUDA, "device upload failed");
-        c->smem = d2::smem_of(c->p);
-        if (cudaFuncSetAttribute(reinterpret_cast<const void*>(d2::kernel_of(c->p)), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(c->smem)) != cudaSuccess)
-            return bail(DG_ERR_CUDA, "kernel attribute");
-        int per_sm = 0, sms = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(d2::kernel_of(c->p)),
-                                                      32 * d2::kWarps, c->smem);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-        const int need = (c->ne + d2::kWarps - 1) / d2::kWarps;
-        c->grid = std::max(1, std::min(need, std::max(1, per_sm) * std::max(1, sms)));
+        d2::Args& a = c->args;
+        a.acc = c->d_acc;
+        a.geo = c->d_geo;
+        a.edges = c->d_edges;
+        a.elift = c->d_elift;
+        a.tab = c->d_tab;
+        a.status = c->d_status;
+        a.ne = c->ne;
+        a.nedge = c->nedge;
+        a.flux = c->flux;
+        a.gamma = c->gamma;
+        const int n = c->p + 1, m = c->p + 2;
+        for (int q = 0; q < m; ++q) {
+            a.W[q] = c->t1.wq[q];
+            for (int b = 0; b < n; ++b) {
+                a.B[q * n + b] = c->t1.B[q * n + b];
+                long double sb = 0.0L, sd = 0.0L;
+                for (int k = 0; k < n; ++k) {
+                    sb += static_cast<long double>(c->t1.B[q * n + k]) * c->t1.Minv[b * n + k];
+                    sd += static_cast<long double>(c->t1.D[q * n + k]) * c->t1.Minv[b * n + k];
+                }
+                a.MB[q * n + b] = static_cast<double>(sb);
+                a.MD[q * n + b] = static_cast<double>(sd);
+            }
+        }
+        for (int b = 0; b < n; ++b) {
+            a.ME[0][b] = c->t1.Minv[b * n];
+            a.ME[1][b] = c->t1.Minv[b * n + n - 1];
+        }
+        const d2::Kernels k = d2::kernels_of(c->p);
+        int per_sm = 0, edge_per_sm = 0, sms = 0;
+        if (cudaFuncSetAttribute(reinterpret_cast<const void*>(k.stage), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(k.smem)) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(k.stage), 32, k.smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&edge_per_sm, reinterpret_cast<const void*>(k.edge), d2::kEdgeThreads, 0) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess)
+            return bail(DG_ERR_CUDA, "kernel attributes");
+        c->grid = std::max(1, std::min((c->ne + k.elems - 1) / k.elems, std::max(1, per_sm) * std::max(1, sms)));
+        // small meshes: one batch of elements per warp, at most one block per SM
+        const int warps = (c->ne + k.elems - 1) / k.elems;
+        if (warps <= sms * d2::kStageWarps) {
+            int steps_per_sm = 0;
+            const int smem = static_cast<int>(k.smem * d2::kStageWarps);
+            if (cudaFuncSetAttribute(reinterpret_cast<const void*>(k.steps), cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&steps_per_sm, reinterpret_cast<const void*>(k.steps), d2::kStepThreads, smem) != cudaSuccess)
+                return bail(DG_ERR_CUDA, "kernel attributes");
+            if (steps_per_sm > 0) c->step_grid = std::min(sms, warps);
+        }
+        const int per_cta = k.edges_per_warp * (d2::kEdgeThreads / 32);
+        c->edge_grid = std::max(1, std::min((c->nedge + per_cta - 1) / per_cta, std::max(1, edge_per_sm) * std::max(1, sms)));
     } catch (const std::bad_alloc&) {
         return bail(DG_ERR_NOMEM, "host allocation failed");
     }
@@ -692,23 +966,15 @@ int dg2d_num_basis(const dg_ctx2d* c) { return c ? c->nb : 0; }
 int dg2d_set_state(dg_ctx2d* c, const double* Uc)
 {
     if (!c || !Uc) return fail2(c, DG_ERR_ARG, "dg2d_set_state: null argument");
-    std::vector<double> d(static_cast<size_t>(c->ne) * d2::kNS * c->nb);
-    to_device_layout(Uc, d.data(), c->ne, c->nb);
     DG2_CUDA(c, cudaSetDevice(c->device));
-    DG2_CUDA(c, cudaMemcpyAsync(c->d_U0, d.data(), d.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    DG2_CUDA(c, cudaStreamSynchronize(c->stream));
-    return DG_OK;
+    return to_device(c, Uc, c->d_U0, c->d_res);
 }
 
 int dg2d_get_state(dg_ctx2d* c, double* Uc)
 {
     if (!c || !Uc) return fail2(c, DG_ERR_ARG, "dg2d_get_state: null argument");
-    std::vector<double> d(static_cast<size_t>(c->ne) * d2::kNS * c->nb);
     DG2_CUDA(c, cudaSetDevice(c->device));
-    DG2_CUDA(c, cudaMemcpyAsync(d.data(), c->d_U0, d.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    DG2_CUDA(c, cudaStreamSynchronize(c->stream));
-    to_host_layout(d.data(), Uc, c->ne, c->nb);
-    return DG_OK;
+    return to_host(c, c->d_U0, Uc, c->d_res);
 }
 
 int dg2d_residual(dg_ctx2d* c, double* res)
@@ -717,21 +983,22 @@ int dg2d_residual(dg_ctx2d* c, double* res)
     DG2_CUDA(c, cudaSetDevice(c->device));
     int rc = launch(c, c->d_U0, c->d_res, d2::kResidual, 0.0);
     if (rc) return rc;
-    std::vector<double> d(static_cast<size_t>(c->ne) * d2::kNS * c->nb);
-    DG2_CUDA(c, cudaMemcpyAsync(d.data(), c->d_res, d.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if ((rc = check_status(c))) return rc;
-    to_host_layout(d.data(), res, c->ne, c->nb);
-    return DG_OK;
+    return to_host(c, c->d_res, res, c->d_Ub);
 }
 
 int dg2d_rk4_steps_timed(dg_ctx2d* c, double dt, int nsteps, double* device_ms)
 {
     if (!c || nsteps < 0 || !(dt > 0.0)) return fail2(c, DG_ERR_ARG, "dg2d_rk4_steps: bad argument");
     DG2_CUDA(c, cudaSetDevice(c->device));
-    int rc = prepare_graph(c, dt);
+    int rc = c->step_grid ? DG_OK : prepare_graph(c, dt);
     if (rc) return rc;
     DG2_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-    for (int s = 0; s < nsteps; ++s) DG2_CUDA(c, cudaGraphLaunch(c->graph_exec, c->stream));
+    if (c->step_grid) {
+        if ((rc = launch_steps(c, dt, nsteps))) return rc;
+    } else {
+        for (int s = 0; s < nsteps; ++s) DG2_CUDA(c, cudaGraphLaunch(c->graph_exec, c->stream));
+    }
     DG2_CUDA(c, cudaEventRecord(c->ev1, c->stream));
     if ((rc = check_status(c))) return rc;
     if (device_ms) {
