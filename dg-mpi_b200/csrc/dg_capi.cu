@@ -1339,10 +1339,12 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
         for (int v = 0; v < nv; ++v) has_fx = has_fx || (vs[v].flags & dgk::kFX);
         const size_t nflux = static_cast<size_t>(c->nface) * 5 * (c->p + 2) * (c->p + 2);
         if (has_fx && c->nface > 0) {
-            const size_t flux_bytes = (nflux * sizeof(double) + 255) / 256 * 256;
-            const size_t desc_bytes = faces.size() * sizeof(dgk::FaceDesc), lrec_bytes = static_cast<size_t>(c->ne) * 6 * sizeof(int);
-            if (cudaMalloc((void**)&c->d_faces, faces.size() * sizeof(int2)) != cudaSuccess ||
-                cudaMalloc((void**)&c->d_fflux, flux_bytes + desc_bytes + lrec_bytes) != cudaSuccess ||
+            // the face list, the column form's descriptors and element-to-face records
+            // in one allocation, the fluxes in another
+            const size_t face_bytes = (faces.size() * sizeof(int2) + 255) / 256 * 256, desc_bytes = faces.size() * sizeof(dgk::FaceDesc);
+            const size_t lrec_bytes = static_cast<size_t>(c->ne) * 6 * sizeof(int);
+            if (cudaMalloc((void**)&c->d_faces, face_bytes + desc_bytes + lrec_bytes) != cudaSuccess ||
+                cudaMalloc((void**)&c->d_fflux, nflux * sizeof(double)) != cudaSuccess ||
                 cudaMemcpy(c->d_faces, faces.data(), faces.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess) {
                 cudaGetLastError();
                 cudaFree(c->d_faces);
@@ -1350,7 +1352,7 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
                 c->d_faces = nullptr;
                 c->d_fflux = nullptr;
             } else {
-                c->d_fdesc = reinterpret_cast<dgk::FaceDesc*>(reinterpret_cast<char*>(c->d_fflux) + flux_bytes);
+                c->d_fdesc = reinterpret_cast<dgk::FaceDesc*>(reinterpret_cast<char*>(c->d_faces) + face_bytes);
                 c->d_lrec = reinterpret_cast<int*>(c->d_fdesc + faces.size());
             }
         }

@@ -57,7 +57,7 @@ struct dg_ctx {
     // face kernel's fluxes [nface][5][(p+2)^2]
     int nface = 0, nface_inner = 0;
     int2* d_faces = nullptr;
-    // the column form's face descriptors and element-to-face records, in d_fflux's allocation
+    // the column form's face descriptors and element-to-face records, in d_faces' allocation
     dgk::FaceDesc* d_fdesc = nullptr;
     int* d_lrec = nullptr;
     double* d_fflux = nullptr;
