@@ -891,7 +891,9 @@ int dg2d_create(const dg_case_desc* cd, const dg_mesh2d_desc* md, dg_ctx2d** out
              cudaMemset(c->d_elift, 0, lift_bytes) == cudaSuccess &&
              cudaMemcpy(c->d_tab, &tab, sizeof(d2::Tab), cudaMemcpyHostToDevice) == cudaSuccess &&
              cudaMemset(c->d_status, 0, d2::kStatusWords * sizeof(unsigned)) == cudaSuccess &&
-             cudaMemset(c->d_U0, 0, nstate) == cudaSuccess && cudaMemset(c->d_acc, 0, nstate) == cudaSuccess;
+             cudaMemset(c->d_U0, 0, nstate) == cudaSuccess && cudaMemset(c->d_acc, 0, nstate) == cudaSuccess &&
+             // (the context's stream does not wait for the default stream)
+             cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess;
         if (!ok) return bail(DG_ERR_CUDA, "device upload failed");
         d2::Args& a = c->args;
         a.acc = c->d_acc;

@@ -1001,7 +1001,9 @@ int unit_pressure_residual(dg_ctx* c)
             U[(e * 5 + 0) * c->nb + b] = 1.0;
             U[(e * 5 + 4) * c->nb + b] = 1.0 / (c->gamma - 1.0);
         }
-    DG_CUDA(c, cudaMemcpy(c->d_U0, U.data(), nstate * sizeof(double), cudaMemcpyHostToDevice));
+    // (on the context's own stream: a copy from pageable memory on another one may
+    // still be under way when the call returns)
+    DG_CUDA(c, cudaMemcpyAsync(c->d_U0, U.data(), nstate * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     const int keep = c->variant;
     c->variant = v64;
     int rc = launch_stage(c, dgk::kModeResidual, c->d_U0, c->d_U0, c->d_gfsd, 0.0);
@@ -1396,7 +1398,10 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
                 cudaMemcpy(c->d_gnodes, c->pm.gnodes.data(), c->pm.gnodes.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess)) &&
               cudaMemset(c->d_status, 0, kStatusWords * sizeof(unsigned)) == cudaSuccess &&
               cudaMemset(c->d_U0, 0, nstate * sizeof(double)) == cudaSuccess &&
-              cudaMemset(c->d_acc, 0, nstate * sizeof(double)) == cudaSuccess;
+              cudaMemset(c->d_acc, 0, nstate * sizeof(double)) == cudaSuccess &&
+              // c->stream does not wait for the default stream, on which the last
+              // of these copies and memsets may still be running
+              cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess;
     if (!ok) {
         c->err = std::string("table upload failed: ") + cudaGetErrorString(cudaGetLastError());
         return bail(DG_ERR_CUDA);
@@ -2140,8 +2145,9 @@ int dg_status(dg_ctx* c, unsigned* flags)
     if (!c || !flags) return fail(c, DG_ERR_ARG, "dg_status: null argument");
     unsigned st = 0;
     DG_CUDA(c, cudaSetDevice(c->device));
-    DG_CUDA(c, cudaMemcpy(&st, c->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost));
-    DG_CUDA(c, cudaMemset(c->d_status, 0, sizeof(unsigned)));
+    DG_CUDA(c, cudaMemcpyAsync(&st, c->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+    DG_CUDA(c, cudaMemsetAsync(c->d_status, 0, sizeof(unsigned), c->stream));
+    DG_CUDA(c, cudaStreamSynchronize(c->stream));
     *flags = st | c->status_accum;
     c->status_accum = 0;
     return DG_OK;
