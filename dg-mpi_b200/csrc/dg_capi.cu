@@ -216,8 +216,9 @@ void stage_args(const dg_ctx* c, int mode, const double* Us, const double* U0, d
     if (vs[c->variant].flags & dgk::kTC) a.fstride = dgk::tc_face_stride(c->p);
     if (vs[c->variant].flags & dgk::kCF) {
         // the face kernel stores lifted fluxes; the residual output takes the plain tables
+        // (as the general geometry does, whose inverse mass is a pass of its own)
         a.fstride = 5 * (c->p + 1) * (c->p + 1);
-        if (mode == dgk::kModeResidual) {
+        if (mode == dgk::kModeResidual || c->pm.general) {
             std::memcpy(a.tab.MB, a.tab.B, sizeof(a.tab.MB));
             std::memcpy(a.tab.MD, a.tab.D, sizeof(a.tab.MD));
             for (int b = 0; b <= c->p; ++b) {
@@ -339,7 +340,7 @@ __global__ void face_desc_kernel(const dgk::FaceRec* __restrict__ frec, const in
     }
     d.info = r.info;
     d.cls = r.cls;
-    d.pad = 0;
+    d.side = ef.x * 6 + ef.y;
     out[i] = d;
 }
 

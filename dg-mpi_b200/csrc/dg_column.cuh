@@ -58,7 +58,7 @@ constexpr int kSM = 16384;
 // block [v][bz][by][qx] (stride X1S) sits in its rows 5.. .  Strides and task
 // orders (see TaskOrd for their coding) minimise the wavefronts of the passes'
 // addresses (FP64 served per half-warp on 16 bank pairs, FP32 per warp on 32).
-template <int P, typename T>
+template <int P, typename T, bool GE = false>
 struct ColLay {
     static constexpr bool W8 = sizeof(T) == 8;
     static constexpr int N = P + 1, M = P + 2, NB = N * N * N, NF = M * M, N2 = N * N;
@@ -73,11 +73,11 @@ struct ColLay {
     static constexpr int oyc = W8 ? (P == 3 || P == 4 ? 11 : 21) : (P == 1 ? 21 : P == 2 ? 15 : P == 4 ? 11 : 19);
     static_assert(PS >= NF && AS >= (N - 1) * PS + NF && 10 * AS >= 5 * X1S, "point-array rows overlap");
     static constexpr int W = 15 * AS;                     // point array, T
-    // FP32 path: the FP64 residual block, entry (bx, by, bz) at bz SZ + by SY + bx:
+    // FP32 path and general geometry: the FP64 residual block, entry (bx, by, bz) at bz SZ + by SY + bx:
     // x, y and z pencils of a variable fall on distinct bank pairs but for a few
     // (N = 4: SY = 5, SZ = 20) and their words are constant offsets apart
     static constexpr int SY = N % 2 ? N : N + 1, SZ = N * SY, VS = N * SZ;
-    static constexpr int RES = W8 ? 0 : 5 * VS;           // FP64 residual of the FP32 path
+    static constexpr int RES = W8 && !GE ? 0 : 5 * VS;
     static constexpr int LF = 30 * N2;                    // the six faces' lifts, T
     static constexpr size_t f64_words(int E) { return static_cast<size_t>(E) * RES + 2 * N; }
     static constexpr size_t t_words(int E) { return static_cast<size_t>(E) * (W + LF + 6); }
@@ -123,14 +123,6 @@ __device__ __forceinline__ void store_row(double* p, const double (&x)[N])
 #pragma unroll
         for (int k = 0; k < N; ++k) p[k] = x[k];
     }
-}
-
-// starts fetching n doubles at p into L2 (whole 16-byte pieces of them)
-__device__ __forceinline__ void prefetch_l2(const double* p, int n)
-{
-    const unsigned long long g = __cvta_generic_to_global(p);
-    const unsigned bytes = (static_cast<unsigned>(n) * 8u) & ~15u;
-    if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(g & ~15ull), "r"(bytes) : "memory");
 }
 
 // x, in a way the compiler does not see through: index arithmetic on it is redone
@@ -189,9 +181,12 @@ struct CtaSync {
 // One batch of E elements on NT threads that synchronise through Sync (a whole
 // CTA, or the threads of one group of a larger one): thread tid0 of NT, the
 // group's shared memory, the stage's buffers through IO.
-template <int P, int E, int NT, typename T, typename IO, typename Sync>
+// GE: general (trilinear) geometry in FP64 -- per-point metric terms, plain tables,
+// and the element's dense inverse mass matrix after the contraction.
+template <int P, int E, int NT, typename T, typename IO, typename Sync, bool GE = false>
 struct Column {
-    using L = ColLay<P, T>;
+    using L = ColLay<P, T, GE>;
+    static_assert(!GE || (sizeof(T) == 8 && E == 1), "general geometry: FP64, one element at a time");
     static constexpr int N = L::N, M = L::M, NB = L::NB, NF = L::NF, N2 = L::N2;
     static constexpr int PS = L::PS, AS = L::AS, X1S = L::X1S, W = L::W, VS = L::VS, SY = L::SY, SZ = L::SZ;
     static constexpr bool F64 = sizeof(T) == 8, kShift = !F64;
@@ -201,7 +196,7 @@ struct Column {
     IO io;
     Sync sync;
     const int tid0;
-    double* sRes;                                      // [E][5][VS] (FP32 path)
+    double* sRes;                                      // [E][5][VS] (FP32 path, GE)
     double* sM;                                        // [2][N] end columns of the 1D inverse mass
     T* sW;                                             // [E][W]
     T* sL;                                             // [E][6][5][N2] lifts in this element's node order
@@ -327,7 +322,7 @@ struct Column {
     }
 
     // y interpolation, then per quadrature column the z interpolation, flux and z contraction
-    __device__ __forceinline__ void columns(const StageArgs& a)
+    __device__ __forceinline__ void columns(const StageArgs& a, int e0)
     {
         const T* __restrict__ Bt = TabSel<T>::B(a.tab);
         const T* __restrict__ Wt = TabSel<T>::W(a.tab);
@@ -400,9 +395,13 @@ struct Column {
                     if (S[0][q] != S[0][q] || p[q] != p[q]) status |= kStatusNaN;
                 }
             }
+            // GE: entry k of the metric terms at point q of the column
+            auto metric = [&](int k, int q) { return a.gjd[((size_t)min(e0 + e, a.ne - 1) * 9 + k) * (M * NF) + q * NF + qxy]; };
             T JD[9];
+            if constexpr (!GE) {
 #pragma unroll
-            for (int k = 0; k < 9; ++k) JD[k] = T(geo->JD[k]);
+                for (int k = 0; k < 9; ++k) JD[k] = T(geo->JD[k]);
+            }
             const T wxy = Wt[qxy % M] * Wt[qxy / M];
             // contract the components g_d(v, q) of each variable along z
             auto contract = [&](auto&& component) {
@@ -437,15 +436,17 @@ struct Column {
                 for (int q = 0; q < M; ++q) {
                     const T wq = wxy * Wt[q], u = vel[0][q], v = vel[1][q], w = vel[2][q];
 #pragma unroll
-                    for (int d = 0; d < 3; ++d)
-                        vel[d][q] = (u * JD[d * 3 + 0] + v * JD[d * 3 + 1] + w * JD[d * 3 + 2]) * wq;
+                    for (int d = 0; d < 3; ++d) {
+                        if constexpr (GE) vel[d][q] = (u * metric(d * 3, q) + v * metric(d * 3 + 1, q) + w * metric(d * 3 + 2, q)) * wq;
+                        else vel[d][q] = (u * JD[d * 3 + 0] + v * JD[d * 3 + 1] + w * JD[d * 3 + 2]) * wq;
+                    }
                     p[q] *= wq;
                 }
                 contract([&](int v, int q, T (&g)[3]) {
 #pragma unroll
                     for (int d = 0; d < 3; ++d) {
                         g[d] = S[v][q] * vel[d][q];
-                        if (v >= 1 && v <= 3) g[d] += p[q] * JD[d * 3 + v - 1];
+                        if (v >= 1 && v <= 3) g[d] += p[q] * (GE ? metric(d * 3 + v - 1, q) : JD[d * 3 + v - 1]);
                     }
                 });
             } else {
@@ -514,6 +515,47 @@ struct Column {
         }
     }
 
+    // GE: the element's dense inverse mass matrix, streamed from global memory, and
+    // the stage update; a thread's rows (two with 16-byte loads where their number
+    // is even) of all five variables
+    __device__ __forceinline__ void dense_inverse_mass(const StageArgs& a, int e0)
+    {
+        constexpr int V2 = NB % 2 == 0 ? 2 : 1, RP = NB / V2;
+        const size_t ge = e0;
+        const double scale = io.dt(a) * a.geo[sCls[0]].dtf;
+#pragma unroll 1
+        for (int rp = tid0; rp < RP; rp += NT) {
+            const double* im = a.gimm + ge * NB * NB + V2 * rp;  // iMM[V2 rp + i][k] at im[k NB + i]
+            double s[V2][5] = {};
+            for (int kz = 0; kz < N; ++kz)
+#pragma unroll
+                for (int kyx = 0; kyx < N2; ++kyx) {
+                    double m[V2];
+                    load_row<V2>(im + (size_t)(kz * N2 + kyx) * NB, m);
+                    const double* r = sRes + kz * SZ + (kyx / N) * SY + kyx % N;
+#pragma unroll
+                    for (int v = 0; v < 5; ++v)
+#pragma unroll
+                        for (int i = 0; i < V2; ++i) s[i][v] += m[i] * r[v * VS];
+                }
+#pragma unroll
+            for (int v = 0; v < 5; ++v) {
+                const size_t g = (ge * 5 + v) * NB + V2 * rp;
+                double u0[V2] = {}, ac[V2] = {}, o[V2], ao[V2];
+                if (need_u0) load_row<V2>(io.U0(a) + g, u0);
+                if (need_acc) load_row<V2>(io.acc(a) + g, ac);
+#pragma unroll
+                for (int i = 0; i < V2; ++i) {
+                    const double k = scale * s[i][v];
+                    ao[i] = ac[i] + ca * k;
+                    o[i] = u0[i] + cu * (sum_acc ? ac[i] + k : k);
+                }
+                if (put_acc) store_row<V2>(io.acc(a) + g, ao);
+                store_row<V2>(io.out(a) + g, o);
+            }
+        }
+    }
+
     // x contraction, face lifts, inverse mass (FP32 path) and stage update
     __device__ __forceinline__ void finish(const StageArgs& a, int e0)
     {
@@ -532,7 +574,7 @@ struct Column {
             const int by = byz % N, bz = byz / N;
             const size_t g = ((size_t)min(e0 + e, a.ne - 1) * 5 * N2 + row) * N;
             double u0[N] = {}, ac[N] = {};
-            if constexpr (F64) {
+            if constexpr (F64 && !GE) {
                 if (need_u0) load_row<N>(io.U0(a) + g, u0);
                 if (need_acc) load_row<N>(io.acc(a) + g, ac);
             }
@@ -549,7 +591,7 @@ struct Column {
             // lifts: faces 4 / 2 at the row's ends, 1 / 3 and 0 / 5 along it
             const T* Lv = sL + e * L::LF + v * N2;
             const T* sg = sSgn + e * 6;
-            if constexpr (F64) {
+            if constexpr (F64 && !GE) {
                 const double l4 = sg[4] * Lv[4 * 5 * N2 + byz], l2 = sg[2] * Lv[2 * 5 * N2 + byz];
                 const double c1 = sg[1] * sM[by], c3 = sg[3] * sM[N + by], c0 = sg[0] * sM[bz], c5 = sg[5] * sM[N + bz];
                 const double* L1 = Lv + 1 * 5 * N2 + bz * N;
@@ -603,6 +645,11 @@ struct Column {
                     continue;
                 }
                 double* res = sRes + e * L::RES + v * VS;
+                if constexpr (GE) {
+#pragma unroll
+                    for (int j = 0; j < N; ++j) res[bz * SZ + by * SY + j] = t[j];
+                    continue;
+                }
 #pragma unroll
                 for (int j = 0; j < N; ++j) {
                     double s = 0.0;
@@ -610,6 +657,12 @@ struct Column {
                     for (int k = 0; k < N; ++k) s += Mi[j * N + k] * t[k];
                     res[bz * SZ + by * SY + j] = s;
                 }
+            }
+        }
+        if constexpr (GE) {
+            if (io.mode(a) != kModeResidual) {
+                sync();
+                dense_inverse_mass(a, e0);
             }
         }
         if constexpr (!F64) {
@@ -667,12 +720,12 @@ struct Column {
     }
 };
 
-template <int P, int E, int NT, typename T, int MB>
+template <int P, int E, int NT, typename T, int MB, bool GE = false>
 __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ StageArgs a)
 {
     extern __shared__ double csm[];
     constexpr int NB = ColLay<P, T>::NB;
-    Column<P, E, NT, T, StageIO, CtaSync<NT>> c(a, StageIO(), CtaSync<NT>(), threadIdx.x, csm);
+    Column<P, E, NT, T, StageIO, CtaSync<NT>, GE> c(a, StageIO(), CtaSync<NT>(), threadIdx.x, csm);
     const int tid = threadIdx.x;
     const int stride = gridDim.x * E;
     int e0 = a.e_begin + blockIdx.x * E;
@@ -686,10 +739,13 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
         }
         c.lifts(a, e0);
         c.interp_x(a);
-        c.columns(a);
+        c.columns(a, e0);
         // the next batch's rows and records, in flight during the contractions (past
         // the end the last element's: a condition would keep the old rows alive)
         c.fetch(a, e0 + stride);
+        // the element's inverse mass matrix, towards L2 (p = 3, 18^3: 107 -> 100 us a stage)
+        if constexpr (GE)
+            if (tid == 0) prefetch_l2(a.gimm + (size_t)e0 * NB * NB, NB * NB);
         c.contract_y(a);
         cp_async_wait_all();  // the lifts have landed
         cta_sync<NT>();
@@ -787,7 +843,9 @@ struct FacePhases {
         }
     }
 
-    // the flux at the listed side's face points, over that side's trace
+    // the flux at the listed side's face points, over that side's trace (GEO: with the
+    // normal data of each point)
+    template <bool GEO = false>
     static __device__ __forceinline__ void flux(const StageArgs& a, const FaceDesc* sD, int nf, T* sTr, unsigned& status, int tid)
     {
         const T* __restrict__ Wt = TabSel<T>::W(a.tab);
@@ -806,7 +864,11 @@ struct FacePhases {
                 UL[v] = isL ? uo : un;
                 UR[v] = isL ? un : uo;
             }
-            const T nd[4] = {T(fd.n[0]), T(fd.n[1]), T(fd.n[2]), T(fd.nmag)};
+            T nd[4] = {T(fd.n[0]), T(fd.n[1]), T(fd.n[2]), T(fd.nmag)};
+            if constexpr (GEO) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) nd[k] = T(a.gnrm[((size_t)fd.side * 4 + k) * NF + c]);
+            }
             const double eref = kShift ? a.geo[fd.cls].eref : 0.0;
             if (!kShift && a.flux == 0) dgp::flux_lax_friedrichs_sq(T(a.gamma), UL, UR, nd, nd[3], Fo);
             else numerical_flux<T, kShift>(a.flux, a.gamma, UL, UR, nd, eref, Fo, status);
@@ -845,7 +907,7 @@ struct FacePhases {
     }
 };
 
-template <int P, typename T, int FB, int NT, int MB>
+template <int P, typename T, int FB, int NT, int MB, bool GEO = false>
 __global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant__ StageArgs a)
 {
     using L = FaceLay<P, T, FB>;
@@ -891,7 +953,7 @@ __global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant
         cta_sync<NT>();
         gather(f0 + fstep, next);
         cp_async_commit();
-        F::flux(a, sD, nf, sTr, status, tid);
+        F::template flux<GEO>(a, sD, nf, sTr, status, tid);
         cta_sync<NT>();
         F::lift(a, f0, nf, sTr, tid);
         slot = next;
@@ -900,38 +962,38 @@ __global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant
     if (status) atomicOr(a.status, status);
 }
 
-template <int P, int E, int NT, typename T, int MB>
+template <int P, int E, int NT, typename T, int MB, bool GE>
 cudaError_t launch_column(const StageArgs& a, int grid, cudaStream_t s)
 {
-    column_kernel<P, E, NT, T, MB><<<grid, NT, ColLay<P, T>::bytes(E), s>>>(a);
+    column_kernel<P, E, NT, T, MB, GE><<<grid, NT, ColLay<P, T, GE>::bytes(E), s>>>(a);
     return cudaGetLastError();
 }
-template <int P, typename T, int FB, int NT, int MB>
+template <int P, typename T, int FB, int NT, int MB, bool GE>
 cudaError_t launch_face_lift(const StageArgs& a, int grid, cudaStream_t s)
 {
-    face_lift_kernel<P, T, FB, NT, MB><<<grid, NT, FaceLay<P, T, FB>::bytes, s>>>(a);
+    face_lift_kernel<P, T, FB, NT, MB, GE><<<grid, NT, FaceLay<P, T, FB>::bytes, s>>>(a);
     return cudaGetLastError();
 }
 
 // E elements and NT threads per CTA, at least MB resident CTAs per SM asked of the
-// compiler; the default from min_per_sm elements per SM on (below, the stage
-// kernel's many threads per element finish sooner than one warp per element)
+// compiler; the default from min_per_sm elements per SM on.
 // The face kernel's batch FB on FNT threads (FMB resident CTAs asked of the
 // compiler) is the measured best of batches of 2 .. 20 faces on 32 .. 256 threads:
 // small CTAs, whose barriers hold few warps, as long as one round of threads
-// covers most of the slices and points.
-template <int P, int E, int NT, typename T, int MB, int FB, int FNT, int FMB>
+// covers most of the slices and points. GE: general geometry.
+template <int P, int E, int NT, typename T, int MB, int FB, int FNT, int FMB, bool GE = false>
 StageVariant make_column_variant(int min_per_sm)
 {
-    static_assert(ColLay<P, T>::bytes(E) <= 227 * 1024, "column kernel shared memory exceeds 227 KB");
+    using CL = ColLay<P, T, GE>;
+    static_assert(CL::bytes(E) <= 227 * 1024, "column kernel shared memory exceeds 227 KB");
     static_assert(FaceLay<P, T, FB>::bytes <= 227 * 1024, "face kernel shared memory exceeds 227 KB");
-    StageVariant v{E, NT, 1, sizeof(T) == 4 ? 1 : 0, kSB | kFX | kCF, ColLay<P, T>::bytes(E),
-                   (const void*)column_kernel<P, E, NT, T, MB>, launch_column<P, E, NT, T, MB>};
+    StageVariant v{E, NT, 1, sizeof(T) == 4 ? 1 : 0, kSB | kFX | kCF | (GE ? kGE : 0), CL::bytes(E),
+                   (const void*)column_kernel<P, E, NT, T, MB, GE>, launch_column<P, E, NT, T, MB, GE>};
     v.min_per_sm = min_per_sm;
-    v.face_func = (const void*)face_lift_kernel<P, T, FB, FNT, FMB>;
+    v.face_func = (const void*)face_lift_kernel<P, T, FB, FNT, FMB, GE>;
     v.face_smem = FaceLay<P, T, FB>::bytes;
     v.face_threads = FNT;
-    v.face_launch = launch_face_lift<P, T, FB, FNT, FMB>;
+    v.face_launch = launch_face_lift<P, T, FB, FNT, FMB, GE>;
     v.face_batch = FB;
     return v;
 }

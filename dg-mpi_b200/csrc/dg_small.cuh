@@ -141,7 +141,7 @@ small_steps_kernel(const __grid_constant__ SmallArgs s)
                     c.fetch(s.a, e0);
                     c.classes();
                     c.interp_x(s.a);
-                    c.columns(s.a);
+                    c.columns(s.a, e0);
                     c.contract_y(s.a);
                 }
                 target += nb;

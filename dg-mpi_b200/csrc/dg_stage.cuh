@@ -116,7 +116,7 @@ struct FaceDesc {
     unsigned strides;
     int info;
     int cls;
-    int pad;
+    int side;  // listed element * 6 + face
 };
 static_assert(sizeof(FaceDesc) == 64, "FaceDesc is four 16-byte words");
 
@@ -394,6 +394,14 @@ __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.w
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 // all but the most recent group complete
 __device__ __forceinline__ void cp_async_wait_older() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+
+// starts fetching n doubles at p into L2 (whole 16-byte pieces of them)
+__device__ __forceinline__ void prefetch_l2(const double* p, int n)
+{
+    const unsigned long long g = __cvta_generic_to_global(p);
+    const unsigned bytes = (static_cast<unsigned>(n) * 8u) & ~15u;
+    if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(g & ~15ull), "r"(bytes) : "memory");
+}
 
 // queue the face records of batch e0 into dst [E][6]
 template <int E, int NT>
@@ -1605,6 +1613,13 @@ StageVariant make_variant()
         v.face_launch = launch_face_kernel<P, T, geo>;
         v.face_batch = face_batch<P, T>();
     }
+    return v;
+}
+
+// v, the untuned default from n elements per SM on
+inline StageVariant from_per_sm(StageVariant v, int n)
+{
+    v.min_per_sm = n;
     return v;
 }
 

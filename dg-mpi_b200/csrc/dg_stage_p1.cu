@@ -5,7 +5,8 @@
 // the face kernel, face lifts added in the inverse mass's first pass; then the minimum
 // of resident CTAs per SM asked of the compiler).  Contexts on non-affine meshes use the
 // general-geometry (kGE) entries only, the others never do.  The
-// first variant of each precision is the default (the measured best); dg_tune_stage may pick another.
+// first variant of each precision whose threshold of elements per SM the mesh reaches is
+// the default (the measured best); dg_tune_stage may pick another.
 #include "dg_stage.cuh"
 #include "dg_small.cuh"
 
@@ -25,7 +26,10 @@ static const StageVariant kVariants1[] = {
     make_variant<1, 8, 128, 1, float>(),
     make_variant<1, 4, 64, 1, float>(),
     make_variant<1, 2, 64, 1, float>(),
-    // general (trilinear) geometry: the variants of non-affine meshes
+    // general (trilinear) geometry: the variants of non-affine meshes.  FP64 RK
+    // stage at 24^3 bent elements 54 -> 49 us in column form; below 16 elements per SM
+    // the one-launch kernel stays ahead (12^3: 9.3 against 10.3 us, 14^3: 14.4 against 13.9)
+    make_column_variant<1, 1, 32, double, 12, 3, 32, 20, true>(16),
     make_variant<1, 2, 64, 1, double, kUF | kGE>(),
     make_variant<1, 2, 64, 1, float, kUF | kGE>(),
 };

@@ -5,7 +5,8 @@
 // the face kernel, face lifts added in the inverse mass's first pass; then the minimum
 // of resident CTAs per SM asked of the compiler).  Contexts on non-affine meshes use the
 // general-geometry (kGE) entries only, the others never do.  The
-// first variant of each precision is the default (the measured best); dg_tune_stage may pick another.
+// first variant of each precision whose threshold of elements per SM the mesh reaches is
+// the default (the measured best); dg_tune_stage may pick another.
 #include "dg_stage.cuh"
 #include "dg_small.cuh"
 
@@ -37,12 +38,16 @@ static const StageVariant kVariants4[] = {
     make_variant<4, 1, 128, 1, float, kUF | kRS | kSB>(),
     make_variant<4, 1, 128, 2, float, kPZ>(),
     make_variant<4, 1, 64, 1, float>(),
-    // general (trilinear) geometry: the variants of non-affine meshes
+    // general (trilinear) geometry: the variants of non-affine meshes.  In
+    // mixed precision with the face kernel 119 -> 96 us per RK stage at 13^3 bent
+    // elements, from 3 elements per SM (8^3: 32.5 -> 26.5, 6^3: 16.4 against 18.5).  The
+    // FP64 column form is slower here (131 against 118 us: four CTAs per SM for want of
+    // registers do not cover the 125 KB matrix of each element)
     make_variant<4, 1, 128, 1, double, kUF | kRS | kSB | kK1 | kGE>(),
+    from_per_sm(make_variant<4, 1, 128, 1, float, kUF | kSB | kGE | kFX>(), 3),
     make_variant<4, 1, 128, 1, float, kUF | kSB | kGE>(),
     make_variant<4, 1, 96, 1, double, kUF | kRS | kSB | kK1 | kGE>(),
     make_variant<4, 1, 128, 1, double, kUF | kRS | kSB | kGE | kFX>(),
-    make_variant<4, 1, 128, 1, float, kUF | kSB | kGE | kFX>(),
 };
 
 int stage_variants_p4(const StageVariant** out)

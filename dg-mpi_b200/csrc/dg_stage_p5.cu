@@ -5,7 +5,8 @@
 // the face kernel, face lifts added in the inverse mass's first pass; then the minimum
 // of resident CTAs per SM asked of the compiler).  Contexts on non-affine meshes use the
 // general-geometry (kGE) entries only, the others never do.  The
-// first variant of each precision is the default (the measured best); dg_tune_stage may pick another.
+// first variant of each precision whose threshold of elements per SM the mesh reaches is
+// the default (the measured best); dg_tune_stage may pick another.
 #include "dg_stage.cuh"
 #include "dg_small.cuh"
 
@@ -35,12 +36,16 @@ static const StageVariant kVariants5[] = {
     make_variant<5, 1, 128, 1, float, kUF | kRS | kSB | kK1>(),
     make_variant<5, 1, 128, 2, float, kSB>(),
     make_variant<5, 1, 64, 2, float>(),
-    // general (trilinear) geometry: the variants of non-affine meshes
+    // general (trilinear) geometry: the variants of non-affine meshes.  With
+    // the face kernel 137 -> 126 us per RK stage at 10^3 bent elements in FP64 (8^3:
+    // 70.7 against 71.2), from 4 elements per SM; in mixed precision 153 -> 143, left to
+    // dg_tune_stage because its FP32 sums round differently from the default's (1e-9 of
+    // the state after a few steps).  The FP64 column form takes 168 us
+    from_per_sm(make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kGE | kFX, 2>(), 4),
     make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kK1 | kGE, 2>(),
     make_variant<5, 1, 128, 1, float, kUF | kRS | kSB | kK1 | kGE>(),
     make_variant<5, 1, 128, 1, double, kUF | kRS | kSB | kK1 | kGE>(),
     make_variant<5, 1, 256, 1, float, kUF | kRS | kSB | kK1 | kGE, 3>(),
-    make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kGE | kFX, 2>(),
     make_variant<5, 1, 256, 1, float, kUF | kRS | kSB | kGE | kFX, 3>(),
 };
 
