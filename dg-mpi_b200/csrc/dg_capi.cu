@@ -252,6 +252,10 @@ int launch_stage(dg_ctx* c, int mode, const double* Us, const double* U0, double
         a.face_begin = f0;
         a.nface = f1;
         const int fb = sv.face_batch;
+        // unpartitioned stages follow one another with nothing on another stream between
+        const bool alone = e_begin == 0 && e_end == c->ne && c->nslices == 0;
+        a.face_overlaps = alone && (mode == dgk::kModeRK2 || mode == dgk::kModeRK3 || mode == dgk::kModeRK4);
+        a.column_overlaps = alone && f1 > f0;
         if (f1 > f0) DG_CUDA(c, sv.face_launch(a, std::min(c->variant_face_grid[c->variant], (f1 - f0 + fb - 1) / fb), c->stream));
     }
     const int batches = (e_end - e_begin + sv.E - 1) / sv.E;

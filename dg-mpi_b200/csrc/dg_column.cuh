@@ -125,6 +125,38 @@ __device__ __forceinline__ void store_row(double* p, const double (&x)[N])
     }
 }
 
+// Dependent launch: a kernel launched with overlap may start when the CTAs of the
+// kernel before it on the stream have ended, without waiting for that kernel's own
+// completion, which it does in wait_prerequisites (all writes visible); only
+// data that no kernel writes is read before.  Without overlap that call does nothing.
+// FP64 RK stage: p = 1, 14^3 9.3 -> 8.8 us, p = 3, 9^3 12.9 -> 11.8, 16^3 34.3 -> 34.0;
+// nothing from some 20^3 on.  An earlier start (griddepcontrol.launch_dependents at
+// the kernels' beginning) places the CTAs unevenly: 9^3 15.8 us, 24^3 100 -> 110.
+__device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// the column kernel of FP64 p = 5 is at its register limit and loses 3 % to the wait
+template <int P, typename T>
+constexpr bool column_overlaps()
+{
+    return !(sizeof(T) == 8 && P >= 5);
+}
+
+inline cudaError_t launch_after(void (*kernel)(StageArgs), const StageArgs& a, int overlap, int grid, int threads,
+                                size_t smem, cudaStream_t s)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
 // x, in a way the compiler does not see through: index arithmetic on it is redone
 // in every iteration of the batch loop instead of being kept in registers across
 // the column phase, which needs them
@@ -729,6 +761,7 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
     const int tid = threadIdx.x;
     const int stride = gridDim.x * E;
     int e0 = a.e_begin + blockIdx.x * E;
+    if constexpr (column_overlaps<P, T>()) wait_prerequisites();  // the face kernel's lifts, and through it the stage before
     if (e0 < a.ne) c.fetch(a, e0);
     for (; e0 < a.ne; e0 += stride) {
         // this batch's RK operands (read by the last pass) and the next batch's rows on
@@ -938,6 +971,9 @@ __global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant
         cp_async_commit();
         cp_async_wait_all();
         cta_sync<NT>();
+    }
+    wait_prerequisites();  // the descriptors do not change, the state does
+    if (f0 < a.nface) {
         gather(f0, 0);
         cp_async_commit();
     }
@@ -965,14 +1001,13 @@ __global__ void __launch_bounds__(NT, MB) face_lift_kernel(const __grid_constant
 template <int P, int E, int NT, typename T, int MB, bool GE>
 cudaError_t launch_column(const StageArgs& a, int grid, cudaStream_t s)
 {
-    column_kernel<P, E, NT, T, MB, GE><<<grid, NT, ColLay<P, T, GE>::bytes(E), s>>>(a);
-    return cudaGetLastError();
+    return launch_after(column_kernel<P, E, NT, T, MB, GE>, a, column_overlaps<P, T>() && a.column_overlaps, grid, NT,
+                        ColLay<P, T, GE>::bytes(E), s);
 }
 template <int P, typename T, int FB, int NT, int MB, bool GE>
 cudaError_t launch_face_lift(const StageArgs& a, int grid, cudaStream_t s)
 {
-    face_lift_kernel<P, T, FB, NT, MB, GE><<<grid, NT, FaceLay<P, T, FB>::bytes, s>>>(a);
-    return cudaGetLastError();
+    return launch_after(face_lift_kernel<P, T, FB, NT, MB, GE>, a, a.face_overlaps, grid, NT, FaceLay<P, T, FB>::bytes, s);
 }
 
 // E elements and NT threads per CTA, at least MB resident CTAs per SM asked of the

@@ -182,6 +182,7 @@ struct StageArgs {
     double gamma;
     double dt;
     StageTables tab;
+    int face_overlaps, column_overlaps;  // column form: the kernel may start before the one ahead of it ends
 };
 
 __host__ __device__ constexpr int odd(int x) { return x | 1; }
