@@ -416,14 +416,20 @@ struct ReduceCfg {
     static constexpr int N = P + 1, NB = N * N * N, ME = KIND == 0 ? (P > 1 ? 2 * P + 2 : 4) : P + 2;
     static constexpr int NV = KIND == 0 ? 5 : 4;  // the kinetic energy needs no energy
     static constexpr int E = ME * ME >= 128 ? 1 : 128 / (ME * ME), NT = (E * ME * ME + 31) / 32 * 32;
-    static constexpr size_t smem = sizeof(double) * E * NV * (NB + N * N * ME + N * ME * ME);
+    static constexpr int A = NB > N * ME * ME ? NB : N * ME * ME;  // coefficients, later the x-y interpolated values
+    static constexpr int LD = (E * NV * NB + NT - 1) / NT;         // coefficients a thread fetches for a batch
+    static constexpr size_t smem = sizeof(double) * E * NV * (A + N * N * ME);
 };
 
 // Interpolation by three 1D passes (x and y through shared memory, z in the
 // column's thread); the dense sum over the (p+1)^3 basis functions per point
 // that this replaces was bound by its 5 (N^3 + N^2 + N) multiply-adds and its
-// divergent constant-memory indices.  Calls, 48^3, p = 4: kinetic energy 4.04 -> 0.47 ms, x-y vortex
-// error 18.1 -> 2.7 ms; 32^3, p = 3: error 9.37 -> 0.37 ms.  Each interpolated
+// divergent constant-memory indices.  The y pass writes over the coefficients (seven CTAs
+// per SM in place of five at p = 3 and 4), whose next batch waits in registers meanwhile
+// (the error up to p = 3, bound by the exact solution's evaluation, is faster
+// without: 64^3, p = 2, 1.57 against 1.70 ms).  Calls, 48^3, p = 4: kinetic energy
+// 4.04 -> 0.28 ms (0.47 with its own buffer for each pass and no prefetch), x-y vortex
+// error 18.1 -> 2.3 ms; 32^3, p = 3: error 9.37 -> 0.33 ms.  Each interpolated
 // value is the same sum in the same order.
 template <int P, int KIND>
 __global__ void __launch_bounds__(ReduceCfg<P, KIND>::NT) reduce_kernel(ReduceArgs a)
@@ -431,21 +437,34 @@ __global__ void __launch_bounds__(ReduceCfg<P, KIND>::NT) reduce_kernel(ReduceAr
     using C = ReduceCfg<P, KIND>;
     constexpr int N = C::N, NB = C::NB, N2 = N * N, ME = C::ME, M2 = ME * ME, E = C::E, NT = C::NT, NV = C::NV;
     extern __shared__ double rsm[];
-    double* sU = rsm;                   // [E][NV][bz][by][bx]
-    double* s1 = sU + E * NV * NB;      // [E][NV][bz][by][i]
-    double* s2 = s1 + E * NV * N2 * ME; // [E][NV][bz][j][i]
+    double* sU = rsm;                  // [E][NV][bz][by][bx]
+    double* s2 = rsm;                  // [E][NV][bz][j][i], over the coefficients
+    double* s1 = rsm + E * NV * C::A;  // [E][NV][bz][by][i]
     const double* Bq = KIND == 0 ? cBe[P] : cVB[P];
     const double* Wq = KIND == 0 ? cWe[P] : cVW[P];
     const double* Xq = KIND == 0 ? cXe[P] : cXq[P];
     const int tid = threadIdx.x;
     double acc[5] = {0, 0, 0, 0, 0};
+    double next[C::LD];  // a batch's coefficients, in flight during the batch before
+    auto fetch = [&](int e0) {
+        const int n = min(E, a.ne - e0) * NV * NB;
+#pragma unroll
+        for (int l = 0; l < C::LD; ++l) {
+            const int i = tid + l * NT, e = i / (NV * NB);
+            if (i < n) next[l] = a.U[(size_t)(e0 + e) * 5 * NB + (i - e * (NV * NB))];
+        }
+    };
+    constexpr bool kAhead = KIND == 1 || P >= 4;  // see above
+    if (kAhead) fetch(blockIdx.x * E);
     for (int e0 = blockIdx.x * E; e0 < a.ne; e0 += gridDim.x * E) {
         const int en = min(E, a.ne - e0);
-        for (int i = tid; i < en * NV * NB; i += NT) {
-            const int e = i / (NV * NB), r = i - e * (NV * NB);
-            sU[i] = a.U[(size_t)(e0 + e) * 5 * NB + r];
-        }
+        if (!kAhead) fetch(e0);
+        __syncthreads();  // the batch before is done with s2
+#pragma unroll
+        for (int l = 0; l < C::LD; ++l)
+            if (tid + l * NT < en * NV * NB) sU[tid + l * NT] = next[l];
         __syncthreads();
+        if (kAhead) fetch(e0 + gridDim.x * E);
         for (int t = tid; t < en * NV * N2; t += NT) {  // x: rows (e, v, bz, by)
             double u[N];
 #pragma unroll
@@ -547,7 +566,18 @@ cudaError_t launch_reduce(const dg_ctx* c, const ReduceArgs& a, int* grid)
             cudaFuncSetAttribute(reduce_kernel<P, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem);
         if (e != cudaSuccess) return e;
     }
-    *grid = std::max(1, std::min(c->red_grid, (a.ne + C::E - 1) / C::E));
+    // more batches than red_grid CTAs (eight per SM) are shared evenly among the CTAs that
+    // fit at once: 32^3, p = 3, kinetic energy 0.081 ms with red_grid CTAs, 0.063 ms so
+    const int batches = (a.ne + C::E - 1) / C::E;
+    *grid = std::max(1, std::min(c->red_grid, batches));
+    if (batches > c->red_grid) {
+        int per_sm = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reduce_kernel<P, KIND>, C::NT, C::smem);
+        if (e != cudaSuccess) return e;
+        const int resident = std::max(1, std::min(c->red_grid, c->red_grid / 8 * per_sm));
+        const int rounds = (batches + resident - 1) / resident;
+        *grid = (batches + rounds - 1) / rounds;
+    }
     reduce_kernel<P, KIND><<<*grid, C::NT, C::smem, c->stream>>>(a);
     return cudaGetLastError();
 }
