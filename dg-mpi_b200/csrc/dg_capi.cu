@@ -1027,7 +1027,7 @@ int unit_pressure_residual(dg_ctx* c)
     dgk::stage_variants(c->p, &vs);
     int v64 = -1;
     for (int v = 0; v < nv && v64 < 0; ++v)
-        if (!vs[v].fp32 && (vs[v].flags & dgk::kGE)) v64 = v;
+        if (!vs[v].fp32 && (vs[v].flags & dgk::kGE) && (!(vs[v].flags & dgk::kFX) || c->d_fflux)) v64 = v;
     if (v64 < 0) return fail(c, DG_ERR_UNSUPPORTED, "no FP64 general-geometry stage kernel for this order");
     const size_t nstate = static_cast<size_t>(c->ne) * c->nb * 5;
     std::vector<double> U(nstate, 0.0);

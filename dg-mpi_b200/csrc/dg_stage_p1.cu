@@ -16,15 +16,11 @@ static const StageVariant kVariants1[] = {
     make_small_variant<1, 1, 32, 8, 4, 3, double>(make_column_variant<1, 3, 32, double, 16, 3, 32, 20>(0)),
     make_column_variant<1, 3, 32, double, 16, 3, 32, 20>(0),
     make_variant<1, 8, 128, 1, double>(),
-    make_variant<1, 4, 64, 1, double>(),
     make_variant<1, 2, 64, 1, double>(),
     make_variant<1, 1, 32, 1, double>(),
     make_small_variant<1, 1, 32, 8, 4, 3, float>(make_column_variant<1, 3, 32, float, 20, 12, 128, 1>(0)),
     make_column_variant<1, 3, 32, float, 20, 12, 128, 1>(0),
     make_variant<1, 8, 128, 1, float, kUF | kSB | kFX>(),
-    make_variant<1, 4, 64, 1, float, kUF | kSB | kFX>(),
-    make_variant<1, 8, 128, 1, float>(),
-    make_variant<1, 4, 64, 1, float>(),
     make_variant<1, 2, 64, 1, float>(),
     // general (trilinear) geometry: the variants of non-affine meshes.  FP64 RK
     // stage at 24^3 bent elements 54 -> 49 us in column form; below 16 elements per SM

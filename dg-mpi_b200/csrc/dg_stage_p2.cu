@@ -17,25 +17,16 @@ static const StageVariant kVariants2[] = {
     make_small_variant<2, 1, 32, 6, 6, 2, double>(make_column_variant<2, 2, 32, double, 11, 6, 32, 1>(0)),
     make_column_variant<2, 2, 32, double, 11, 6, 32, 1>(0),
     make_variant<2, 1, 32, 1, double, kUF | kSB | kFX | kMG>(),
-    make_variant<2, 2, 64, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<2, 1, 32, 1, double, kUF | kSB | kFX>(),
-    make_variant<2, 2, 64, 1, double, kUF | kSB | kFX>(),
     make_variant<2, 1, 64, 1, double, kUF | kRS | kSB | kFX>(),
     make_variant<2, 1, 32, 1, double, kUF>(),
-    make_variant<2, 2, 64, 1, double, kUF | kRS | kSB>(),
-    make_variant<2, 1, 32, 1, double>(),
-    make_variant<2, 2, 64, 1, double>(),
     make_small_variant<2, 1, 64, 3, 6, 2, float>(make_column_variant<2, 2, 32, float, 16, 8, 128, 1>(0)),
     make_small_variant<2, 1, 32, 6, 6, 2, float>(make_column_variant<2, 2, 32, float, 16, 8, 128, 1>(0)),
     make_column_variant<2, 2, 32, float, 16, 8, 128, 1>(0),
     make_variant<2, 1, 32, 1, float, kUF | kSB | kFX | kMG>(),
-    make_variant<2, 2, 64, 1, float, kUF | kSB | kFX | kMG>(),
     make_variant<2, 1, 32, 1, float, kUF | kSB | kFX>(),
-    make_variant<2, 2, 64, 1, float, kUF | kSB | kFX>(),
     make_variant<2, 1, 64, 1, float, kUF | kRS | kSB | kFX>(),
     make_variant<2, 1, 32, 1, float, kUF>(),
-    make_variant<2, 2, 64, 1, float, kUF | kSB>(),
-    make_variant<2, 4, 128, 1, float>(),
     make_variant<2, 1, 32, 1, float>(),
     // general (trilinear) geometry: the variants of non-affine meshes.  RK
     // stage at 22^3 bent elements 90 -> 74 us in FP64 (column form), 95 -> 79 us in

@@ -16,36 +16,18 @@ namespace dgk {
 static const StageVariant kVariants3[] = {
     make_small_variant<3, 1, 64, 4, 4, 3, double>(make_column_variant<3, 1, 32, double, 12, 3, 32, 1>(0)),
     make_column_variant<3, 1, 32, double, 12, 3, 32, 1>(0),
-    make_variant<3, 1, 96, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<3, 1, 128, 1, double, kUF | kSB | kFX | kMG>(),
-    make_variant<3, 1, 128, 1, double, kUF | kRS | kSB | kFX | kMG>(),
     make_variant<3, 1, 128, 1, double, kUF | kSB | kFX>(),
     make_variant<3, 1, 128, 1, double, kUF | kRS | kSB | kFX>(),
-    make_variant<3, 1, 128, 1, double, kUF | kRS | kSB | kFX, 8>(),
-    make_variant<3, 1, 96, 1, double, kUF | kRS | kSB | kFX>(),
-    make_variant<3, 1, 96, 1, double, kUF | kSB | kFX>(),
-    make_variant<3, 1, 64, 1, double, kUF | kRS | kSB | kFX>(),
-    make_variant<3, 2, 128, 1, double, kUF | kRS | kSB | kFX>(),
-    make_variant<3, 1, 32, 1, double, kUF | kSB | kFX>(),
     make_variant<3, 1, 64, 1, double, kUF | kRS | kSB | kK1>(),
-    make_variant<3, 1, 64, 1, double, kUF | kSB | kK1>(),
     make_variant<3, 1, 32, 2, double, kSB>(),
     make_variant<3, 2, 64, 2, double>(),
     make_small_variant<3, 1, 64, 4, 8, 1, float>(make_column_variant<3, 1, 32, float, 16, 5, 64, 1>(0)),
     make_column_variant<3, 1, 32, float, 16, 5, 64, 1>(0),
     make_variant<3, 1, 128, 1, float, kUF | kSB | kFX | kMG>(),
-    make_variant<3, 1, 128, 1, float, kUF | kRS | kSB | kFX | kMG>(),
-    make_variant<3, 1, 64, 1, float, kUF | kSB | kFX | kMG>(),
-    make_variant<3, 1, 64, 1, float, kUF | kSB | kFX>(),
     make_variant<3, 1, 128, 1, float, kUF | kRS | kSB | kFX>(),
-    make_variant<3, 1, 64, 1, float, kUF | kRS | kSB | kFX>(),
-    make_variant<3, 1, 32, 1, float, kUF | kSB | kFX>(),
     make_variant<3, 1, 128, 1, float, kUF | kSB | kFX>(),
     make_variant<3, 1, 32, 1, float, kUF | kSB | kK1>(),
-    make_variant<3, 1, 32, 1, float, kUF | kSB>(),
-    make_variant<3, 2, 64, 1, float, kUF | kSB | kK1>(),
-    make_variant<3, 1, 32, 1, float, kSB>(),
-    make_variant<3, 1, 32, 1, float>(),
     // general (trilinear) geometry: the variants of non-affine meshes.  RK
     // stage at 18^3 bent elements 118 -> 88 us in FP64: column form, the element's
     // matrix fetched into L2 during its contractions (107 without) and eight CTAs per

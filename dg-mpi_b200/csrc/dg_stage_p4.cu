@@ -16,28 +16,17 @@ static const StageVariant kVariants4[] = {
     make_small_variant<4, 1, 64, 2, 4, 1, double>(make_column_variant<4, 1, 64, double, 4, 5, 64, 1>(0)),
     make_column_variant<4, 1, 64, double, 4, 5, 64, 1>(0),
     make_variant<4, 1, 128, 1, double, kUF | kSB | kFX | kMG, 4>(),
-    make_variant<4, 1, 96, 1, double, kUF | kSB | kFX | kMG>(),
     make_variant<4, 1, 128, 1, double, kUF | kSB | kFX, 4>(),
-    make_variant<4, 1, 96, 1, double, kUF | kSB | kFX>(),
-    make_variant<4, 1, 96, 1, double, kUF | kRS | kSB | kFX>(),
-    make_variant<4, 1, 128, 1, double, kUF | kRS | kSB | kFX>(),
-    make_variant<4, 1, 128, 1, double, kUF | kRS | kSB | kFX, 4>(),
-    make_variant<4, 1, 64, 1, double, kUF | kSB | kFX>(),
     make_variant<4, 1, 128, 1, double, kUF | kRS | kSB | kK1, 4>(),
     make_variant<4, 1, 128, 1, double, kUF | kRS | kSB | kK1>(),
-    make_variant<4, 1, 96, 1, double, kUF | kRS | kSB | kK1>(),
     make_variant<4, 1, 64, 2, double>(),
     make_small_variant<4, 1, 64, 3, 6, 1, float>(make_column_variant<4, 1, 64, float, 8, 5, 64, 1>(0)),
     make_column_variant<4, 1, 64, float, 8, 5, 64, 1>(0),
     make_variant<4, 1, 128, 1, float, kUF | kSB | kFX | kMG>(),
-    make_variant<4, 1, 128, 1, float, kUF | kRS | kSB | kFX | kMG>(),
     make_variant<4, 1, 128, 1, float, kUF | kSB | kFX>(),
-    make_variant<4, 1, 128, 1, float, kUF | kRS | kSB | kFX>(),
-    make_variant<4, 1, 64, 1, float, kUF | kSB | kFX>(),
     make_variant<4, 1, 128, 1, float, kUF | kSB>(),
     make_variant<4, 1, 128, 1, float, kUF | kRS | kSB>(),
     make_variant<4, 1, 128, 2, float, kPZ>(),
-    make_variant<4, 1, 64, 1, float>(),
     // general (trilinear) geometry: the variants of non-affine meshes.  In
     // mixed precision with the face kernel 119 -> 96 us per RK stage at 13^3 bent
     // elements, from 3 elements per SM (8^3: 32.5 -> 26.5, 6^3: 16.4 against 18.5).  The

@@ -17,23 +17,17 @@ static const StageVariant kVariants5[] = {
     make_small_variant<5, 1, 64, 2, 4, 1, double>(make_column_variant<5, 1, 64, double, 4, 5, 64, 1>(0)),
     make_column_variant<5, 1, 64, double, 4, 5, 64, 1>(0),
     make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kFX | kMG, 2>(),
-    make_variant<5, 1, 192, 1, double, kUF | kRS | kSB | kFX | kMG>(),
     make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kFX, 2>(),
-    make_variant<5, 1, 192, 1, double, kUF | kRS | kSB | kFX>(),
     make_variant<5, 1, 128, 1, double, kUF | kRS | kSB | kFX>(),
     make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kK1, 2>(),
-    make_variant<5, 1, 128, 1, double, kUF | kRS | kSB | kK1>(),
     make_variant<5, 1, 128, 3, double>(),
     make_small_variant<5, 1, 96, 2, 6, 1, float>(make_column_variant<5, 1, 64, float, 6, 8, 128, 1>(0)),
     make_small_variant<5, 1, 64, 3, 6, 1, float>(make_column_variant<5, 1, 64, float, 6, 8, 128, 1>(0)),
     make_column_variant<5, 1, 64, float, 6, 8, 128, 1>(0),
     make_variant<5, 1, 256, 1, float, kUF | kSB | kFX | kMG, 3>(),
-    make_variant<5, 1, 256, 1, float, kUF | kRS | kSB | kFX | kMG, 3>(),
-    make_variant<5, 1, 256, 1, float, kUF | kRS | kSB | kFX, 3>(),
     make_variant<5, 1, 128, 1, float, kUF | kRS | kSB | kFX>(),
     make_variant<5, 1, 256, 1, float, kUF | kSB | kFX, 3>(),
     make_variant<5, 1, 256, 1, float, kUF | kRS | kSB | kK1, 3>(),
-    make_variant<5, 1, 128, 1, float, kUF | kRS | kSB | kK1>(),
     make_variant<5, 1, 128, 2, float, kSB>(),
     make_variant<5, 1, 64, 2, float>(),
     // general (trilinear) geometry: the variants of non-affine meshes.  With

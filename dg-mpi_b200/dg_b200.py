@@ -535,8 +535,9 @@ class Case:
         "k1" (one face-flux point per thread), "ge" (general trilinear geometry: the variants that
         non-affine meshes run), "fx" (each face's flux once, from a face kernel launched before the
         stage kernel), "tc" (the tensor-core kernel: split products on tcgen05 for the volume
-        integral), "mg" (the face lifts added inside the inverse mass's first pass), and "mb<n>"
-        when the variant asks the compiler for n resident CTAs per SM."""
+        integral), "mg" (the face lifts added inside the inverse mass's first pass), "cf" (column form:
+        lifted fluxes from the face kernel, quadrature columns in registers), "sm" (RK4 steps of
+        small meshes in one launch), and "mb<n>" when the variant asks the compiler for n resident CTAs per SM."""
         out = []
         for v in range(self._lib.dg_num_stage_variants(self.order)):
             E, NT, G, pr, fl = (ctypes.c_int() for _ in range(5))
