@@ -507,12 +507,14 @@ def main():
         # (every face's flux once) and the stage kernel
         face_split = "fx" in variants[best][4].split("+")
         launches_per_stage = 2 if face_split else 1
-        kernels = (f"dgk::face_flux_kernel<{ORDER}> + dgk::stage_kernel<{ORDER}> (one RK stage)" if face_split
+        column = "cf" in variants[best][4].split("+")
+        kernels = (f"dgk::face_lift_kernel<{ORDER}> + dgk::column_kernel<{ORDER}> (one RK stage)" if column
+                   else f"dgk::face_flux_kernel<{ORDER}> + dgk::stage_kernel<{ORDER}> (one RK stage)" if face_split
                    else f"dgk::stage_kernel<{ORDER}>")
         launch_s = device_ms / 1e3 / (4 * K)
         achieved = BYTES_PER_DOF_STAGE * dof / launch_s / 1e9
         flops = algorithmic_flops_per_dof(ORDER) * dof / launch_s / 1e12
-        traffic = profile_traffic()
+        traffic = profile_traffic("column_kernels_p3_40cubed.md") if column else profile_traffic()
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": K, "warmup": W,
             "ms_per_step": device_ms / K, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
