@@ -649,7 +649,7 @@ int dg_batch_tune(dg_batch* b, int reps)
     for (auto& g : b->groups) {
         const int keep = g.ctx->variant;
         int best = keep;
-        rc = dg_tune_stage(g.ctx, reps, &best, nullptr);
+        rc = dgi::tune_ctx(g.ctx, reps, true, &best, nullptr);
         if (rc) return gfail(b, rc, g);
         g.own_variant = best;
         if (best != keep) drop_graph(b);

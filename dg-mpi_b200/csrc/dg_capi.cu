@@ -129,6 +129,17 @@ bool variant_matches(const dg_ctx* c, int v)
            (!(vs[v].flags & dgk::kTC) || c->d_tcop) && (!(vs[v].flags & dgk::kSM) || small_mesh(c, vs[v]));
 }
 
+// the untuned variant of single stages beside variant v
+int single_variant(const dg_ctx* c, int v)
+{
+    const dgk::StageVariant* vs = nullptr;
+    const int nv = dgk::stage_variants(c->p, &vs);
+    if (vs[v].flags & dgk::kSM)
+        for (int w = 0; w < nv; ++w)
+            if (vs[w].beside_small && variant_matches(c, w)) return w;
+    return v;
+}
+
 // Sets the variant's shared-memory attribute and its persistent grid size
 // (SM count x resident CTAs per SM, capped by the number of batches).
 int prepare_variant(dg_ctx* c, int v)
@@ -1413,6 +1424,7 @@ int dgi::create_ctx(const dg_case_desc* cd, const dg_mesh_desc* md, const int* e
                 break;
             }
     }
+    c->single = single_variant(c, c->variant);
     std::vector<int2> hs(c->nslices), hr(c->nslices);
     for (int i = 0; i < c->nslices; ++i) {
         hs[i] = make_int2(plan.send_elem[i], plan.send_face[i]);
@@ -1663,12 +1675,26 @@ int dg_get_state(dg_ctx* c, double* Uc)
     return download_host_layout(c, c->d_U0, Uc);
 }
 
+namespace {
+
+// a forward-Euler update or residual of the whole context, by its variant of single stages
+int launch_single(dg_ctx* c, int mode, double* out, double dt)
+{
+    const int keep = c->variant;
+    c->variant = c->single;
+    const int rc = launch_stage(c, mode, c->d_U0, c->d_U0, out, dt);
+    c->variant = keep;
+    return rc;
+}
+
+}  // namespace
+
 int dg_residual(dg_ctx* c, double* res)
 {
     dgi::NvtxRange nvtx_("dg_residual");
     if (!c || !res) return fail(c, DG_ERR_ARG, "dg_residual: null argument");
     DG_CUDA(c, cudaSetDevice(c->device));
-    int rc = launch_stage(c, dgk::kModeResidual, c->d_U0, c->d_U0, c->d_acc, 0.0);
+    int rc = launch_single(c, dgk::kModeResidual, c->d_acc, 0.0);
     if (rc) return rc;
     rc = download_host_layout(c, c->d_acc, res);
     if (rc) return rc;
@@ -1680,7 +1706,7 @@ int dg_mass_inverse_residual(dg_ctx* c, double dt, double* dU)
     dgi::NvtxRange nvtx_("dg_mass_inverse_residual");
     if (!c || !dU || !std::isfinite(dt)) return fail(c, DG_ERR_ARG, "dg_mass_inverse_residual: bad argument");
     DG_CUDA(c, cudaSetDevice(c->device));
-    int rc = launch_stage(c, dgk::kModeMassInv, c->d_U0, c->d_U0, c->d_acc, dt);
+    int rc = launch_single(c, dgk::kModeMassInv, c->d_acc, dt);
     if (rc) return rc;
     rc = download_host_layout(c, c->d_acc, dU);
     if (rc) return rc;
@@ -1864,6 +1890,7 @@ int dg_set_stage_variant(dg_ctx* c, int v)
         if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
         if (c->graph) { cudaGraphDestroy(c->graph); c->graph = nullptr; }
     }
+    c->single = single_variant(c, v);
     return DG_OK;
 }
 
@@ -1897,52 +1924,7 @@ int dg_tune_stage(dg_ctx* c, int reps, int* best, double* ms_per_variant)
 {
     dgi::NvtxRange nvtx_("dg_tune_stage");
     if (!c || reps < 1) return fail(c, DG_ERR_ARG, "dg_tune_stage: bad argument");
-    DG_CUDA(c, cudaSetDevice(c->device));
-    const int nv = dg_num_stage_variants(c->p);
-    const int keep = c->variant;
-    int winner = keep;
-    double best_ms = 1e300;
-    cudaEvent_t ev[2];
-    DG_CUDA(c, cudaEventCreate(&ev[0]));
-    if (cudaEventCreate(&ev[1]) != cudaSuccess) { cudaEventDestroy(ev[0]); return fail(c, DG_ERR_CUDA, "cudaEventCreate"); }
-    int rc = DG_OK;
-    for (int v = 0; v < nv && rc == DG_OK; ++v) {
-        if (!variant_matches(c, v)) {
-            if (ms_per_variant) ms_per_variant[v] = -1.0;
-            continue;
-        }
-        c->variant = v;
-        // one untimed launch, then `reps` timed ones of an RK2 stage (reads the
-        // stage state, U0 and the accumulator, writes the accumulator and an
-        // output): the traffic of a real stage.  The output goes to scratch and
-        // the accumulator is dead between steps, so the state is unchanged.
-        rc = launch_stage(c, dgk::kModeRK2, c->d_U0, c->d_U0, c->d_out, 1e-3);
-        if (rc) break;
-        cudaEventRecord(ev[0], c->stream);
-        for (int r = 0; r < reps && rc == DG_OK; ++r) rc = launch_stage(c, dgk::kModeRK2, c->d_U0, c->d_U0, c->d_out, 1e-3);
-        cudaEventRecord(ev[1], c->stream);
-        if (cudaEventSynchronize(ev[1]) != cudaSuccess) { rc = fail(c, DG_ERR_CUDA, "tuning launch failed"); break; }
-        float ms = 0.0f;
-        cudaEventElapsedTime(&ms, ev[0], ev[1]);
-        const double per = ms / reps;
-        if (ms_per_variant) ms_per_variant[v] = per;
-        if (per < best_ms) { best_ms = per; winner = v; }
-    }
-    cudaEventDestroy(ev[0]);
-    cudaEventDestroy(ev[1]);
-    c->variant = keep;
-    if (rc) return rc;
-    // the small-mesh forms run other variants' stage launches here; where one
-    // matches, its steps are the fastest (every element has its own threads)
-    const dgk::StageVariant* vs = nullptr;
-    dgk::stage_variants(c->p, &vs);
-    if (c->chunks == 1)
-        for (int v = nv - 1; v >= 0; --v)
-            if ((vs[v].flags & dgk::kSM) && variant_matches(c, v)) winner = v;
-    rc = dg_set_stage_variant(c, winner);
-    if (rc) return rc;
-    if (best) *best = winner;
-    return DG_OK;
+    return dgi::tune_ctx(c, reps, false, best, ms_per_variant);
 }
 
 int dg_rk4_steps(dg_ctx* c, double dt, int nsteps)
@@ -1968,7 +1950,7 @@ int dg_fe_steps(dg_ctx* c, double dt, int nsteps)
     if (!c || nsteps < 0 || !std::isfinite(dt)) return fail(c, DG_ERR_ARG, "dg_fe_steps: bad argument");
     DG_CUDA(c, cudaSetDevice(c->device));
     for (int s = 0; s < nsteps; ++s) {
-        int rc = launch_stage(c, dgk::kModeFE, c->d_U0, c->d_U0, c->d_Ua, dt);
+        int rc = launch_single(c, dgk::kModeFE, c->d_Ua, dt);
         if (rc) return rc;
         std::swap(c->d_U0, c->d_Ua);
     }
@@ -2262,3 +2244,76 @@ int dg_cfl_time_step(dg_ctx* c, const double* Uc, double cfl, double* dt)
 }
 
 }  // extern "C"
+
+// Per variant, after an untimed run, the device time of `reps` RK2 stages (an RK2 stage
+// reads the stage state, U0 and the accumulator, writes the accumulator and an output: the
+// traffic of a real stage; the output goes to scratch and the accumulator is dead between
+// steps, so the state is unchanged) -- or, where the variant's RK4 steps run in one launch,
+// a quarter of that of `reps` steps, with a time step of zero on a state that is put back
+// (a negative zero would come back positive).  Beside a column form the variant of
+// single stages is picked by forward-Euler updates, whose kernels do not overlap the stage
+// before (p = 1, mixed, HLLC, 4^3: column form 8.0 us as an RK stage, 10.4 as an update; 9.0
+// and 8.4 for the one-launch kernel).
+int dgi::tune_ctx(dg_ctx* c, int reps, bool single_only, int* best, double* ms_per_variant)
+{
+    DG_CUDA(c, cudaSetDevice(c->device));
+    const dgk::StageVariant* vs = nullptr;
+    const int nv = dgk::stage_variants(c->p, &vs);
+    const int keep = c->variant;
+    const size_t state_bytes = static_cast<size_t>(c->ne_alloc) * c->nb * 5 * sizeof(double);
+    int winner = keep, single = keep;  // the fastest RK stage, the fastest update
+    double best_ms = 1e300, single_ms = 1e300;
+    cudaEvent_t ev[2];
+    DG_CUDA(c, cudaEventCreate(&ev[0]));
+    if (cudaEventCreate(&ev[1]) != cudaSuccess) { cudaEventDestroy(ev[0]); return fail(c, DG_ERR_CUDA, "cudaEventCreate"); }
+    int rc = DG_OK;
+    // the time of one of `reps` runs of the selected variant
+    auto timed = [&](auto&& run) {
+        rc = run(1);
+        if (rc) return 0.0;
+        cudaEventRecord(ev[0], c->stream);
+        rc = run(reps);
+        cudaEventRecord(ev[1], c->stream);
+        float ms = 0.0f;
+        if (cudaEventSynchronize(ev[1]) != cudaSuccess || cudaEventElapsedTime(&ms, ev[0], ev[1]) != cudaSuccess)
+            rc = rc ? rc : fail(c, DG_ERR_CUDA, "tuning launch failed");
+        return static_cast<double>(ms) / reps;
+    };
+    auto stages = [&](int mode) {
+        return timed([&, mode](int n) {
+            int r = DG_OK;
+            for (int i = 0; i < n && r == DG_OK; ++i) r = launch_stage(c, mode, c->d_U0, c->d_U0, c->d_out, 1e-3);
+            return r;
+        });
+    };
+    for (int v = 0; v < nv && rc == DG_OK; ++v) {
+        if (!variant_matches(c, v) || (single_only && (vs[v].flags & dgk::kSM))) {
+            if (ms_per_variant) ms_per_variant[v] = -1.0;
+            continue;
+        }
+        c->variant = v;
+        double per = 0.0;
+        if (runs_small(c)) {
+            cudaMemcpyAsync(c->d_out, c->d_U0, state_bytes, cudaMemcpyDeviceToDevice, c->stream);
+            per = timed([&](int n) { return launch_small_steps(c, 0.0, n); }) / 4;
+            cudaMemcpyAsync(c->d_U0, c->d_out, state_bytes, cudaMemcpyDeviceToDevice, c->stream);
+        } else {
+            per = stages(dgk::kModeRK2);
+            const double update = !single_only && rc == DG_OK ? stages(dgk::kModeFE) : per;
+            if (rc == DG_OK && update < single_ms) { single_ms = update; single = v; }
+        }
+        if (rc) break;
+        if (ms_per_variant) ms_per_variant[v] = per;
+        if (per < best_ms) { best_ms = per; winner = v; }
+    }
+    cudaEventDestroy(ev[0]);
+    cudaEventDestroy(ev[1]);
+    c->variant = keep;
+    if (rc == DG_OK && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = fail(c, DG_ERR_CUDA, "tuning launch failed");
+    if (rc) return rc;
+    rc = dg_set_stage_variant(c, winner);
+    if (rc) return rc;
+    if (vs[winner].flags & dgk::kCF) c->single = single;
+    if (best) *best = winner;
+    return DG_OK;
+}

@@ -82,6 +82,9 @@ struct dg_ctx {
     int red_grid = 0;
     int sms = 0;  // multiprocessors of the device
     int variant = 0;                                // index into dgk::stage_variants(p)
+    // the variant of forward Euler and residuals: single stages, which a small-mesh variant
+    // would run as two launches and a column form without overlap; mostly `variant`
+    int single = 0;
     int variant_grid[dgi::kMaxVariants] = {};       // persistent grid per variant, 0 = not prepared
     dgk::StageTables stage_tab{};
     cudaGraph_t graph = nullptr;
@@ -124,6 +127,9 @@ void stage_args(const dg_ctx* c, int mode, const double* Us, const double* U0, d
 // stage launch over the owned elements [e_begin, e_end) (e_end < 0: all)
 int launch_stage(dg_ctx* c, int mode, const double* Us, const double* U0, double* out, double dt, int e_begin = 0,
                  int e_end = -1);
+// dg_tune_stage's timing and choice; single_only: among the variants that run single
+// stages (the groups of a batch never take the one-launch form)
+int tune_ctx(dg_ctx* c, int reps, bool single_only, int* best, double* ms_per_variant);
 // waits for the stream and turns the status word into a return code; handed: the
 // queued work copies the word to c->h_status itself
 int check_status(dg_ctx* c, bool handed = false);

@@ -1559,6 +1559,7 @@ struct StageVariant {
     cudaError_t (*face_launch)(const StageArgs&, int grid, cudaStream_t);
     int face_batch;      // faces per CTA batch of the face kernel
     int min_per_sm;      // elements per SM from which the variant may be the untuned default
+    int beside_small;    // 1: the untuned form of single stages beside a small-mesh variant
     // small-mesh variants (kSM, dg_small.cuh): RK4 steps in one cooperative launch
     // of up to one block per SM while the mesh has at most small_elems elements per SM
     const void* small_func;
@@ -1621,6 +1622,14 @@ StageVariant make_variant()
 inline StageVariant from_per_sm(StageVariant v, int n)
 {
     v.min_per_sm = n;
+    return v;
+}
+
+// v, the untuned form of forward Euler and residuals (see dg_ctx::single) beside a
+// small-mesh variant
+inline StageVariant beside_small(StageVariant v)
+{
+    v.beside_small = 1;
     return v;
 }
 

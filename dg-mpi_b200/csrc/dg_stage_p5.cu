@@ -19,7 +19,10 @@ static const StageVariant kVariants5[] = {
     make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kFX | kMG, 2>(),
     make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kFX, 2>(),
     make_variant<5, 1, 128, 1, double, kUF | kRS | kSB | kFX>(),
-    make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kK1, 2>(),
+    // forward Euler and residuals beside the one-launch RK4 steps: one launch, ahead of
+    // the column form's two up to the largest such mesh (an update, 3^3 elements 18.8 ->
+    // 12.7 us, 6^3 22.7 -> 18.4; p <= 4: column form ahead or equal)
+    beside_small(make_variant<5, 1, 256, 1, double, kUF | kRS | kSB | kK1, 2>()),
     make_variant<5, 1, 128, 3, double>(),
     make_small_variant<5, 1, 96, 2, 6, 1, float>(make_column_variant<5, 1, 64, float, 6, 8, 128, 1>(0)),
     make_small_variant<5, 1, 64, 3, 6, 1, float>(make_column_variant<5, 1, 64, float, 6, 8, 128, 1>(0)),
