@@ -240,7 +240,8 @@ void stage_args(const dg_ctx* c, int mode, const double* Us, const double* U0, d
     }
 }
 
-int launch_stage(dg_ctx* c, int mode, const double* Us, const double* U0, double* out, double dt, int e_begin, int e_end)
+int launch_stage(dg_ctx* c, int mode, const double* Us, const double* U0, double* out, double dt, int e_begin, int e_end,
+                 bool follows)
 {
     if (e_end < 0) e_end = c->ne;
     if (e_begin < 0 || e_end > c->ne || e_begin > e_end) return fail(c, DG_ERR_ARG, "stage element range out of bounds");
@@ -265,7 +266,7 @@ int launch_stage(dg_ctx* c, int mode, const double* Us, const double* U0, double
         const int fb = sv.face_batch;
         // unpartitioned stages follow one another with nothing on another stream between
         const bool alone = e_begin == 0 && e_end == c->ne && c->nslices == 0;
-        a.face_overlaps = alone && (mode == dgk::kModeRK2 || mode == dgk::kModeRK3 || mode == dgk::kModeRK4);
+        a.face_overlaps = alone && (follows || mode == dgk::kModeRK2 || mode == dgk::kModeRK3 || mode == dgk::kModeRK4);
         a.column_overlaps = alone && f1 > f0;
         if (f1 > f0) DG_CUDA(c, sv.face_launch(a, std::min(c->variant_face_grid[c->variant], (f1 - f0 + fb - 1) / fb), c->stream));
     }
@@ -1678,11 +1679,11 @@ int dg_get_state(dg_ctx* c, double* Uc)
 namespace {
 
 // a forward-Euler update or residual of the whole context, by its variant of single stages
-int launch_single(dg_ctx* c, int mode, double* out, double dt)
+int launch_single(dg_ctx* c, int mode, double* out, double dt, bool follows = false)
 {
     const int keep = c->variant;
     c->variant = c->single;
-    const int rc = launch_stage(c, mode, c->d_U0, c->d_U0, out, dt);
+    const int rc = launch_stage(c, mode, c->d_U0, c->d_U0, out, dt, 0, -1, follows);
     c->variant = keep;
     return rc;
 }
@@ -1950,7 +1951,7 @@ int dg_fe_steps(dg_ctx* c, double dt, int nsteps)
     if (!c || nsteps < 0 || !std::isfinite(dt)) return fail(c, DG_ERR_ARG, "dg_fe_steps: bad argument");
     DG_CUDA(c, cudaSetDevice(c->device));
     for (int s = 0; s < nsteps; ++s) {
-        int rc = launch_single(c, dgk::kModeFE, c->d_Ua, dt);
+        int rc = launch_single(c, dgk::kModeFE, c->d_Ua, dt, s > 0);
         if (rc) return rc;
         std::swap(c->d_U0, c->d_Ua);
     }
@@ -2251,9 +2252,7 @@ int dg_cfl_time_step(dg_ctx* c, const double* Uc, double cfl, double* dt)
 // steps, so the state is unchanged) -- or, where the variant's RK4 steps run in one launch,
 // a quarter of that of `reps` steps, with a time step of zero on a state that is put back
 // (a negative zero would come back positive).  Beside a column form the variant of
-// single stages is picked by forward-Euler updates, whose kernels do not overlap the stage
-// before (p = 1, mixed, HLLC, 4^3: column form 8.0 us as an RK stage, 10.4 as an update; 9.0
-// and 8.4 for the one-launch kernel).
+// single stages is picked by forward-Euler updates.
 int dgi::tune_ctx(dg_ctx* c, int reps, bool single_only, int* best, double* ms_per_variant)
 {
     DG_CUDA(c, cudaSetDevice(c->device));
@@ -2282,7 +2281,7 @@ int dgi::tune_ctx(dg_ctx* c, int reps, bool single_only, int* best, double* ms_p
     auto stages = [&](int mode) {
         return timed([&, mode](int n) {
             int r = DG_OK;
-            for (int i = 0; i < n && r == DG_OK; ++i) r = launch_stage(c, mode, c->d_U0, c->d_U0, c->d_out, 1e-3);
+            for (int i = 0; i < n && r == DG_OK; ++i) r = launch_stage(c, mode, c->d_U0, c->d_U0, c->d_out, 1e-3, 0, -1, i > 0);
             return r;
         });
     };

@@ -83,7 +83,7 @@ struct dg_ctx {
     int sms = 0;  // multiprocessors of the device
     int variant = 0;                                // index into dgk::stage_variants(p)
     // the variant of forward Euler and residuals: single stages, which a small-mesh variant
-    // would run as two launches and a column form without overlap; mostly `variant`
+    // would run as two launches; mostly `variant`
     int single = 0;
     int variant_grid[dgi::kMaxVariants] = {};       // persistent grid per variant, 0 = not prepared
     dgk::StageTables stage_tab{};
@@ -124,9 +124,10 @@ bool variant_matches(const dg_ctx* c, int v);
 // the stage kernels' arguments for elements [e_begin, e_end) with the context's variant
 void stage_args(const dg_ctx* c, int mode, const double* Us, const double* U0, double* out, double dt, int e_begin,
                 int e_end, dgk::StageArgs& a);
-// stage launch over the owned elements [e_begin, e_end) (e_end < 0: all)
+// stage launch over the owned elements [e_begin, e_end) (e_end < 0: all); follows: the
+// launch before it on the stream is a stage's too (RK2 .. RK4 always follow one)
 int launch_stage(dg_ctx* c, int mode, const double* Us, const double* U0, double* out, double dt, int e_begin = 0,
-                 int e_end = -1);
+                 int e_end = -1, bool follows = false);
 // dg_tune_stage's timing and choice; single_only: among the variants that run single
 // stages (the groups of a batch never take the one-launch form)
 int tune_ctx(dg_ctx* c, int reps, bool single_only, int* best, double* ms_per_variant);
