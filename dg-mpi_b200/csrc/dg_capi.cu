@@ -422,12 +422,14 @@ struct ReduceArgs {
 
 // Points per direction (the error's rule of 2 max(p,1) + 2, the kinetic
 // energy's volume rule), elements and threads per CTA: one thread per (x, y)
-// point column of an element, whole elements to a CTA of about 128 threads.
-template <int P, int KIND>
+// point column of an element, whole elements to a CTA of about 128 threads. With SPREAD
+// one element to a CTA and KS threads to a column, each taking every KS-th point.
+template <int P, int KIND, bool SPREAD>
 struct ReduceCfg {
     static constexpr int N = P + 1, NB = N * N * N, ME = KIND == 0 ? (P > 1 ? 2 * P + 2 : 4) : P + 2;
     static constexpr int NV = KIND == 0 ? 5 : 4;  // the kinetic energy needs no energy
-    static constexpr int E = ME * ME >= 128 ? 1 : 128 / (ME * ME), NT = (E * ME * ME + 31) / 32 * 32;
+    static constexpr int KS = !SPREAD ? 1 : P == 2 ? 6 : P == 3 ? 4 : 5;
+    static constexpr int E = SPREAD || ME * ME >= 128 ? 1 : 128 / (ME * ME), NT = (E * ME * ME * KS + 31) / 32 * 32;
     static constexpr int A = NB > N * ME * ME ? NB : N * ME * ME;  // coefficients, later the x-y interpolated values
     static constexpr int LD = (E * NV * NB + NT - 1) / NT;         // coefficients a thread fetches for a batch
     static constexpr size_t smem = sizeof(double) * E * NV * (A + N * N * ME);
@@ -443,10 +445,10 @@ struct ReduceCfg {
 // 4.04 -> 0.28 ms (0.47 with its own buffer for each pass and no prefetch), x-y vortex
 // error 18.1 -> 2.3 ms; 32^3, p = 3: error 9.37 -> 0.33 ms.  Each interpolated
 // value is the same sum in the same order.
-template <int P, int KIND>
-__global__ void __launch_bounds__(ReduceCfg<P, KIND>::NT) reduce_kernel(ReduceArgs a)
+template <int P, int KIND, bool SPREAD>
+__global__ void __launch_bounds__(ReduceCfg<P, KIND, SPREAD>::NT) reduce_kernel(ReduceArgs a)
 {
-    using C = ReduceCfg<P, KIND>;
+    using C = ReduceCfg<P, KIND, SPREAD>;
     constexpr int N = C::N, NB = C::NB, N2 = N * N, ME = C::ME, M2 = ME * ME, E = C::E, NT = C::NT, NV = C::NV;
     extern __shared__ double rsm[];
     double* sU = rsm;                  // [E][NV][bz][by][bx]
@@ -504,8 +506,9 @@ __global__ void __launch_bounds__(ReduceCfg<P, KIND>::NT) reduce_kernel(ReduceAr
             }
         }
         __syncthreads();
-        if (tid < en * M2) {  // z and the integrand, column (i, j) of element e
-            const int e = tid / M2, ij = tid - e * M2, i = ij % ME, j = ij / ME, ge = e0 + e;
+        if (tid < en * M2 * C::KS) {  // z and the integrand, column (i, j) of element e
+            const int ks = tid / (E * M2), col = tid - ks * (E * M2);
+            const int e = col / M2, ij = col - e * M2, i = ij % ME, j = ij / ME, ge = e0 + e;
             double u[NV][N];
 #pragma unroll
             for (int v = 0; v < NV; ++v)
@@ -518,7 +521,7 @@ __global__ void __launch_bounds__(ReduceCfg<P, KIND>::NT) reduce_kernel(ReduceAr
             const bool same = KIND == 0 && a.ic_type == DG_IC_VORTEX_XY && !a.gnodes && J[2] == 0.0 && J[5] == 0.0;
             double Ue[5];
 #pragma unroll 1
-            for (int k = 0; k < ME; ++k) {
+            for (int k = ks; k < ME; k += C::KS) {
                 double Uq[NV];
 #pragma unroll
                 for (int v = 0; v < NV; ++v) {
@@ -538,7 +541,7 @@ __global__ void __launch_bounds__(ReduceCfg<P, KIND>::NT) reduce_kernel(ReduceAr
                 }
                 const double w = (Wq[i] * Wq[j]) * Wq[k] * dj;
                 if constexpr (KIND == 0) {
-                    if (k == 0 || !same) dgp::initial_state(a.ic_type, a.data, a.gamma, a.R, x, a.t, Ue);
+                    if (k == ks || !same) dgp::initial_state(a.ic_type, a.data, a.gamma, a.R, x, a.t, Ue);
 #pragma unroll
                     for (int v = 0; v < 5; ++v) {
                         const double d = Uq[v] - Ue[v];
@@ -569,13 +572,14 @@ __global__ void __launch_bounds__(ReduceCfg<P, KIND>::NT) reduce_kernel(ReduceAr
 }
 
 // launches the reduction of ne elements on at most c->red_grid CTAs; *grid gets their number
-template <int P, int KIND>
-cudaError_t launch_reduce(const dg_ctx* c, const ReduceArgs& a, int* grid)
+template <int P, int KIND, bool SPREAD>
+cudaError_t launch_reduce_as(const dg_ctx* c, const ReduceArgs& a, int* grid)
 {
-    using C = ReduceCfg<P, KIND>;
+    using C = ReduceCfg<P, KIND, SPREAD>;
+    const auto kernel = reduce_kernel<P, KIND, SPREAD>;
     if (C::smem > 48 * 1024) {
         const cudaError_t e =
-            cudaFuncSetAttribute(reduce_kernel<P, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem);
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem);
         if (e != cudaSuccess) return e;
     }
     // more batches than red_grid CTAs (eight per SM) are shared evenly among the CTAs that
@@ -584,14 +588,26 @@ cudaError_t launch_reduce(const dg_ctx* c, const ReduceArgs& a, int* grid)
     *grid = std::max(1, std::min(c->red_grid, batches));
     if (batches > c->red_grid) {
         int per_sm = 0;
-        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reduce_kernel<P, KIND>, C::NT, C::smem);
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, C::NT, C::smem);
         if (e != cudaSuccess) return e;
         const int resident = std::max(1, std::min(c->red_grid, c->red_grid / 8 * per_sm));
         const int rounds = (batches + resident - 1) / resident;
         *grid = (batches + rounds - 1) / rounds;
     }
-    reduce_kernel<P, KIND><<<*grid, C::NT, C::smem, c->stream>>>(a);
+    kernel<<<*grid, C::NT, C::smem, c->stream>>>(a);
     return cudaGetLastError();
+}
+
+// the error on a mesh of up to one element per SM is spread, as the exact states of a column's
+// points otherwise wait for one another (call, Taylor-Green, 2^3: p = 2 35.8 -> 33.6, p = 3
+// 45.8 -> 32.7, p = 4 46.0 -> 33.7 us; p <= 1 33.6 either way, 35.7 at 5^3; p = 5 with its
+// 432 threads 47.4 -> 45.8 but 33.7 -> 35.8 where a column has one exact state)
+template <int P, int KIND>
+cudaError_t launch_reduce(const dg_ctx* c, const ReduceArgs& a, int* grid)
+{
+    if constexpr (KIND == 0 && P >= 2 && P <= 4)
+        if (a.ne <= c->sms) return launch_reduce_as<P, KIND, true>(c, a, grid);
+    return launch_reduce_as<P, KIND, false>(c, a, grid);
 }
 
 int run_reduce(dg_ctx* c, int kind, int ic_type, const double* data, int ndata, double t, double* out5, int e0, int ne,
