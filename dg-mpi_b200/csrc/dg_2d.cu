@@ -55,7 +55,7 @@ namespace d2 {
 constexpr int kNS = 4;
 constexpr int kMaxN = 6, kMaxM = 7;
 
-constexpr int kSyncWord = 32, kStatusWords = 96;  // the status word, and two counters kSyncWord words on
+constexpr int kSyncWord = 32, kStatusWords = 64;  // the status word, and a counter kSyncWord words on
 
 enum Mode : int { kResidual = 0, kRK1 = 2, kRK2 = 3, kRK3 = 4, kRK4 = 5, kFE = 6 };
 enum Status : unsigned { kRho = 1u, kPressure = 2u, kNaN = 4u, kHLLC = 8u };
@@ -86,6 +86,12 @@ struct Edge {
     int pad;
 };
 
+// an edge of a block's elements in the one-launch steps, and where in the block's shared
+// memory the lift of either side goes (-1: an element of another block)
+struct BlockEdge {
+    int edge, oL, oR;
+};
+
 struct Args {
     const double* Us;
     double* out;
@@ -93,6 +99,9 @@ struct Args {
     double* acc;
     const Geo* geo;
     const Edge* edges;
+    // one-launch steps: block b's edges are block_edges[i], block_first[b] <= i < block_first[b + 1]
+    const BlockEdge* block_edges;
+    const int* block_first;
     double* elift;  // [ne][4 faces][4][n], zero for edges that are no interior ones
     const Tab* tab;
     unsigned* status;
@@ -114,76 +123,82 @@ __device__ __forceinline__ void load_tab(const Args& a, Tab& T)
     __syncthreads();
 }
 
-// the edge of this lane in the batch of edges at i0
+// the flux at this lane's point of edge ed, the N = P + 1 lanes from k N on holding the
+// edge's points, times the point's weight
 template <int P>
-__device__ __forceinline__ Edge edge_of(const Args& a, int i0)
+__device__ __forceinline__ void edge_flux(const Args& a, const double* Us, const Tab& T, const Edge& ed, double (&F)[kNS],
+                                          unsigned& bad)
 {
-    const int k = (threadIdx.x & 31) / (P + 1);
-    return a.edges[k < 32 / (P + 1) && i0 + k < a.nedge ? i0 + k : a.nedge - 1];
+    constexpr int N = P + 1, NB = N * N;
+    const int lane = threadIdx.x & 31, k = lane / N, j = lane - k * N;
+    const int fL = ed.code & 3, fR = (ed.code >> 2) & 3, flip = (ed.code >> 4) & 1, mine = (ed.code >> 5) & 1;
+    // edge node m of face f: basis index o + m s
+    auto node = [](int f, int m) { return (f == 1 ? N - 1 : f == 2 ? (N - 1) * N : 0) + m * (f == 1 || f == 3 ? N : 1); };
+    const int jr = flip ? N - 1 - j : j;           // the right side's point
+    const int q = mine ? N - 1 - j : j;            // the face's quadrature point
+    const double* pL = Us + static_cast<size_t>(ed.eL) * kNS * NB + node(fL, j);
+    const double* pR = Us + static_cast<size_t>(ed.eR) * kNS * NB + node(fR, j);
+    double uL[kNS], uR[kNS], tL[N], tR[N];
+#pragma unroll
+    for (int v = 0; v < kNS; ++v) {
+        uL[v] = pL[v * NB];
+        uR[v] = pR[v * NB];
+    }
+#pragma unroll
+    for (int m = 0; m < N; ++m) {
+        tL[m] = T.FB[(fL * N + j) * N + m];
+        tR[m] = T.FB[(fR * N + jr) * N + m];
+    }
+    constexpr int s3[4] = {0, 1, 2, 4};
+    double UL[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, UR[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int v = 0; v < kNS; ++v) {
+        double sl = 0.0, sr = 0.0;
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            sl += tL[m] * __shfl_sync(0xffffffffu, uL[v], k * N + m);
+            sr += tR[m] * __shfl_sync(0xffffffffu, uR[v], k * N + m);
+        }
+        UL[s3[v]] = sl;
+        UR[s3[v]] = sr;
+    }
+    const double n3[3] = {ed.n[0], ed.n[1], 0.0};
+    double F5[5];
+    bad = 0;
+    if (a.flux == DG_FLUX_HLLC) {
+        if (!dgp::flux_hllc_n(a.gamma, UL, UR, n3, ed.nmag, F5)) bad = kHLLC;
+    } else {
+        dgp::flux_lax_friedrichs_sq(a.gamma, UL, UR, n3, ed.nmag, F5);
+    }
+    const double w = T.fw[q];
+#pragma unroll
+    for (int v = 0; v < kNS; ++v) F[v] = F5[s3[v]] * w;
 }
 
-// the edges of warp `warp` of nwarp, at the state Us; `held`: the warp's only batch
-// of edges, read before
+// the edges of warp `warp` of nwarp, at the state Us
 template <int P>
 __device__ __forceinline__ void edge_phase(const Args& a, const double* Us, int mode, const Tab& T, int warp, int nwarp,
-                                           unsigned& status, const Edge* held = nullptr)
+                                           unsigned& status)
 {
-    constexpr int N = P + 1, NB = N * N, EPW = 32 / N;  // edges per warp
+    constexpr int N = P + 1, EPW = 32 / N;  // edges per warp
     const double* C = mode == kResidual ? T.FB : T.MF;
     const int lane = threadIdx.x & 31, k = lane / N, j = lane - k * N;
     for (int i0 = warp * EPW; i0 < a.nedge; i0 += nwarp * EPW) {
         const bool on = k < EPW && i0 + k < a.nedge;
-        const Edge ed = held ? *held : edge_of<P>(a, i0);
-        const int fL = ed.code & 3, fR = (ed.code >> 2) & 3, flip = (ed.code >> 4) & 1, mine = (ed.code >> 5) & 1;
-        // edge node m of face f: basis index o + m s
-        auto node = [](int f, int m) { return (f == 1 ? N - 1 : f == 2 ? (N - 1) * N : 0) + m * (f == 1 || f == 3 ? N : 1); };
-        const int jr = flip ? N - 1 - j : j;           // the right side's point
-        const int q = mine ? N - 1 - j : j;            // the face's quadrature point
-        const double* pL = Us + static_cast<size_t>(ed.eL) * kNS * NB + node(fL, j);
-        const double* pR = Us + static_cast<size_t>(ed.eR) * kNS * NB + node(fR, j);
-        double uL[kNS], uR[kNS], tL[N], tR[N];
-#pragma unroll
-        for (int v = 0; v < kNS; ++v) {
-            uL[v] = pL[v * NB];
-            uR[v] = pR[v * NB];
-        }
-#pragma unroll
-        for (int m = 0; m < N; ++m) {
-            tL[m] = T.FB[(fL * N + j) * N + m];
-            tR[m] = T.FB[(fR * N + jr) * N + m];
-        }
-        constexpr int s3[4] = {0, 1, 2, 4};
-        double UL[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, UR[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-        for (int v = 0; v < kNS; ++v) {
-            double sl = 0.0, sr = 0.0;
-#pragma unroll
-            for (int m = 0; m < N; ++m) {
-                sl += tL[m] * __shfl_sync(0xffffffffu, uL[v], k * N + m);
-                sr += tR[m] * __shfl_sync(0xffffffffu, uR[v], k * N + m);
-            }
-            UL[s3[v]] = sl;
-            UR[s3[v]] = sr;
-        }
-        const double n3[3] = {ed.n[0], ed.n[1], 0.0};
-        double F5[5];
-        unsigned bad = 0;
-        if (a.flux == DG_FLUX_HLLC) {
-            if (!dgp::flux_hllc_n(a.gamma, UL, UR, n3, ed.nmag, F5)) bad = kHLLC;
-        } else {
-            dgp::flux_lax_friedrichs_sq(a.gamma, UL, UR, n3, ed.nmag, F5);
-        }
+        const Edge ed = a.edges[on ? i0 + k : a.nedge - 1];
+        const int fL = ed.code & 3, fR = (ed.code >> 2) & 3, flip = (ed.code >> 4) & 1;
+        double F[kNS];
+        unsigned bad;
+        edge_flux<P>(a, Us, T, ed, F, bad);
         if (on) status |= bad;
-        const double w = T.fw[q];
         double* oL = a.elift + (static_cast<size_t>(ed.eL) * 4 + fL) * kNS * N + j;
         double* oR = a.elift + (static_cast<size_t>(ed.eR) * 4 + fR) * kNS * N + j;
 #pragma unroll
         for (int v = 0; v < kNS; ++v) {
-            const double F = F5[s3[v]] * w;
             double sl = 0.0, sr = 0.0;
 #pragma unroll
             for (int m = 0; m < N; ++m) {  // point m; node j of either side
-                const double Fm = __shfl_sync(0xffffffffu, F, k * N + m);
+                const double Fm = __shfl_sync(0xffffffffu, F[v], k * N + m);
                 sl += C[(fL * N + m) * N + j] * Fm;
                 sr += C[(fR * N + (flip ? N - 1 - m : m)) * N + j] * Fm;
             }
@@ -217,8 +232,9 @@ struct Cfg {
     static constexpr size_t smem = sizeof(double) * ((static_cast<size_t>(E) * (ES + kL) + 2 * N + 1) / 2 * 2);
 };
 
-// the batches of warp `warp` of nwarp; sm: the warp's shared memory. With LATE the
-// batch's lifts are there only once lifts_ready() has returned true (false: give up).
+// the batches of warp `warp` of nwarp; sm: the warp's shared memory. With LATE other
+// warps put the (only) batch's lifts there, and lifts_ready() returns true (false: give
+// up) once they have.
 template <int P, bool LATE, typename Ready>
 __device__ __forceinline__ void stage_phase(const Args& a, const double* Us, const double* U0, double* out, int mode, double* sm,
                                             int warp, int nwarp, unsigned& status, Ready&& lifts_ready)
@@ -335,12 +351,11 @@ __device__ __forceinline__ void stage_phase(const Args& a, const double* Us, con
         __syncwarp();
         if constexpr (LATE) {
             if (!lifts_ready()) return;
-            get_lifts();
         } else {
             fetch(e0 + stride);  // past the end: the last element again
+            dgk::cp_async_wait_all();
+            __syncwarp();
         }
-        dgk::cp_async_wait_all();
-        __syncwarp();
         // x contraction, the row's edges (bottom 0, right 1, top 2, left 3) and the update
 #pragma unroll 1
         for (int i = lane; i < kRows; i += 32) {
@@ -399,61 +414,123 @@ __global__ void __launch_bounds__(32, MB) stage2d_kernel(const __grid_constant__
     if (status) atomicOr(a.status, status);
 }
 
-// RK4 steps of a small mesh in one cooperative launch, as small_steps_kernel
-// (dg_small.cuh) runs them in 3D: every stage warp keeps one batch of elements and
-// goes up to the y contraction while the edge warps compute the stage's lifts; two
-// counters order them, each wait bounded. Taken while every stage warp has at most
-// one batch, where it beats the two launches by their latency (stage, HLLC: 32^2,
-// p = 1 7.3 -> 6.4, p = 3 8.3 -> 6.7, p = 5 11.4 -> 7.6 us).
+// Steps of a small mesh in one launch.  Every stage warp keeps one batch of elements and
+// goes up to the y contraction while the block's edge warps compute the lifts of its
+// elements into shared memory.  An edge between two blocks is computed by both, so that
+// one wait a stage is left: the edge warps' for the neighbours' states, on a counter in
+// global memory that each block raises after its update.  The wait is bounded, and the
+// launch cooperative (all blocks resident) unless it is of a single stage, which waits for
+// nothing.  A stage's update may overwrite what other blocks' edges read the stage before:
+// they were done with it when their block's update was counted, which this block's edges
+// have waited for.
+// Taken while every stage warp has at most one batch, where it beats the two launches
+// by their latency (RK stage, HLLC, 32^2: p = 1 7.3 -> 5.1, p = 3 8.3 -> 5.9, p = 5 11.4 ->
+// 7.8 us; 6.8, 7.1 and 7.9 with each edge computed once and the lifts handed over
+// between blocks too; forward Euler, 20^2: p = 1 11.6 -> 5.2, p = 3 12.6 -> 5.6 a step).
+// RK: RK4 steps on U0 through Ua and Ub.  Otherwise steps of the one stage `mode`, from
+// U0 to Ua and back: forward Euler, or the residual of U0 into Ua.
 struct StepArgs {
     Args a;
     double *U0, *Ua, *Ub;
-    int nsteps;
-    unsigned* sync;  // [0] arrivals of the stage warps, [32] of the edge warps, one per block and stage
-    unsigned base;   // both values before the launch
+    int nsteps, mode;
+    unsigned* sync;  // arrivals of the stage warps, one per block and stage but the launch's last
+    unsigned base;   // its value before the launch
 };
 constexpr int kStageWarps = 4, kEdgeWarps = 4, kStepThreads = 32 * (kStageWarps + kEdgeWarps);
 
+// the batches of block b: [first_batch(b), first_batch(b + 1)), neighbouring ones, so that
+// many edges have both sides in the block
+__host__ __device__ inline int first_batch(int b, int batches, int nblock)
+{
+    return static_cast<int>(static_cast<long long>(batches) * b / nblock);
+}
+
+// the block's edges [i0, i1) by warp `warp` of nwarp; lifts to the block's shared memory
 template <int P>
+__device__ __forceinline__ void block_edge_phase(const Args& a, const double* Us, int mode, const Tab& T, int warp, int nwarp, int i0,
+                                                 int i1, double* sm, unsigned& status)
+{
+    constexpr int N = P + 1, EPW = 32 / N;
+    const double* C = mode == kResidual ? T.FB : T.MF;
+    const int lane = threadIdx.x & 31, k = lane / N, j = lane - k * N;
+    for (i0 += warp * EPW; i0 < i1; i0 += nwarp * EPW) {
+        const bool on = k < EPW && i0 + k < i1;
+        const BlockEdge be = a.block_edges[on ? i0 + k : i1 - 1];
+        const Edge ed = a.edges[be.edge];
+        const int fL = ed.code & 3, fR = (ed.code >> 2) & 3, flip = (ed.code >> 4) & 1;
+        double F[kNS];
+        unsigned bad;
+        edge_flux<P>(a, Us, T, ed, F, bad);
+        if (on) status |= bad;
+#pragma unroll
+        for (int v = 0; v < kNS; ++v) {
+            double sl = 0.0, sr = 0.0;
+#pragma unroll
+            for (int m = 0; m < N; ++m) {  // point m; node j of either side
+                const double Fm = __shfl_sync(0xffffffffu, F[v], k * N + m);
+                sl += C[(fL * N + m) * N + j] * Fm;
+                sr += C[(fR * N + (flip ? N - 1 - m : m)) * N + j] * Fm;
+            }
+            if (on && be.oL >= 0) sm[be.oL + v * N + j] = -sl;
+            if (on && be.oR >= 0) sm[be.oR + v * N + j] = sr;
+        }
+    }
+}
+
+template <int P, bool RK>
 __global__ void __launch_bounds__(kStepThreads, 1) steps2d_kernel(const __grid_constant__ StepArgs s)
 {
     extern __shared__ __align__(16) double sm[];
     __shared__ Tab T;
-    __shared__ int dead[2];
-    if (threadIdx.x < 2) dead[threadIdx.x] = 0;
+    // the edge warps' wait gave up; the stage (counted through the launch) it was of
+    __shared__ int dead, gave_up;
+    constexpr int kSlot = Cfg<P>::smem / sizeof(double), kL = Cfg<P>::E * Cfg<P>::kL;
+    if (threadIdx.x == 0) {
+        dead = 0;
+        gave_up = 0x7fffffff;
+    }
+    for (int i = threadIdx.x; i < kStageWarps * kL; i += kStepThreads) sm[i / kL * kSlot + i % kL] = 0.0;  // edges that are no interior ones
     load_tab(s.a, T);
-    const int w = threadIdx.x / 32, nb = gridDim.x;
+    const int w = threadIdx.x / 32, nb = gridDim.x, batches = (s.a.ne + Cfg<P>::E - 1) / Cfg<P>::E;
+    const int batch = first_batch(blockIdx.x, batches, nb) + w, end = first_batch(blockIdx.x + 1, batches, nb);
+    const int i0 = s.a.block_first[blockIdx.x], i1 = s.a.block_first[blockIdx.x + 1];
+    // more edges than the edge warps take at once: the stage warps, done up to the y contraction, help
+    const bool share = i1 - i0 > kEdgeWarps * (32 / (P + 1));
+    const int workers = share ? kEdgeWarps + kStageWarps : kEdgeWarps;
     unsigned status = 0, target = s.base;
-    const int ew = (w - kStageWarps) * nb + blockIdx.x, epw = 32 / (P + 1);  // edge warps: index, edges to a batch
-    const bool once = w >= kStageWarps && (ew + nb * kEdgeWarps) * epw >= s.a.nedge && s.a.nedge > 0;
-    const Edge held = once ? edge_of<P>(s.a, ew * epw) : Edge{};
     bool ok = true;
     for (int step = 0; step < s.nsteps && ok; ++step)
 #pragma unroll 1
-        for (int stage = 1; stage <= 4 && ok; ++stage) {
-            const double* Us = stage == 1 ? s.U0 : stage == 3 ? s.Ub : s.Ua;
-            double* out = stage == 4 ? s.U0 : stage == 2 ? s.Ub : s.Ua;
+        for (int stage = 1; stage <= (RK ? 4 : 1) && ok; ++stage) {
+            const int count = RK ? 4 * step + stage : step + 1;
+            const int back = step % 2;
+            const double* Us = !RK ? (back ? s.Ua : s.U0) : stage == 1 ? s.U0 : stage == 3 ? s.Ub : s.Ua;
+            double* out = !RK ? (back ? s.U0 : s.Ua) : stage == 4 ? s.U0 : stage == 2 ? s.Ub : s.Ua;
+            const double* U0 = RK ? s.U0 : Us;
+            const int mode = RK ? kRK1 + stage - 1 : s.mode;
             if (w < kStageWarps) {
-                target += nb;
                 auto ready = [&]() {
-                    return ok = dgk::role_wait<32 * kStageWarps>(s.sync + 32, target, s.a.status, dead, 1, threadIdx.x);
+                    if (share) {
+                        dgk::named_sync<kStepThreads>(4);  // the edge warps' wait is over
+                        block_edge_phase<P>(s.a, Us, mode, T, kEdgeWarps + w, workers, i0, i1, sm, status);
+                    }
+                    dgk::named_sync<kStepThreads>(1);
+                    return ok = *reinterpret_cast<volatile int*>(&gave_up) > count;
                 };
-                const int warp = w * nb + blockIdx.x;
-                if (warp * Cfg<P>::E < s.a.ne)
-                    stage_phase<P, true>(s.a, Us, s.U0, out, kRK1 + stage - 1, sm + w * (Cfg<P>::smem / sizeof(double)), warp,
-                                         nb * kStageWarps, status, ready);
+                if (batch < end)
+                    stage_phase<P, true>(s.a, Us, U0, out, mode, sm + w * kSlot, batch, batches, status, ready);
                 else
                     ready();
-                if (ok) dgk::role_arrive<32 * kStageWarps>(s.sync, 1, threadIdx.x);
+                if (ok && (step + 1 < s.nsteps || (RK && stage < 4))) dgk::role_arrive<32 * kStageWarps>(s.sync, 2, threadIdx.x);
             } else {
-                const int t = threadIdx.x - 32 * kStageWarps;
                 if (step > 0 || stage > 1) {
                     target += nb;
-                    ok = dgk::role_wait<32 * kEdgeWarps>(s.sync, target, s.a.status, dead + 1, 2, t);
-                    if (!ok) break;
+                    ok = dgk::role_wait<32 * kEdgeWarps>(s.sync, target, s.a.status, &dead, 3, threadIdx.x - 32 * kStageWarps);
                 }
-                edge_phase<P>(s.a, Us, kRK1 + stage - 1, T, ew, nb * kEdgeWarps, status, once ? &held : nullptr);
-                dgk::role_arrive<32 * kEdgeWarps>(s.sync + 32, 2, t);
+                if (share) asm volatile("bar.arrive 4, %0;" ::"n"(kStepThreads) : "memory");
+                if (ok) block_edge_phase<P>(s.a, Us, mode, T, w - kStageWarps, workers, i0, i1, sm, status);
+                else gave_up = count;
+                dgk::named_sync<kStepThreads>(1);  // (after a wait that gave up too: the stage warps wait here)
             }
         }
     if (status) atomicOr(s.a.status, status);
@@ -463,13 +540,14 @@ using KernelFn = void (*)(const Args);
 struct Kernels {
     KernelFn edge, stage;
     void (*steps)(const StepArgs);
+    void (*single_steps)(const StepArgs);
     size_t smem;
     int elems, edges_per_warp;
 };
 template <int P, int MB>
 constexpr Kernels kernels()
 {
-    return Kernels{edge2d_kernel<P>, stage2d_kernel<P, MB>, steps2d_kernel<P>, Cfg<P>::smem, Cfg<P>::E, 32 / (P + 1)};
+    return Kernels{edge2d_kernel<P>, stage2d_kernel<P, MB>, steps2d_kernel<P, true>, steps2d_kernel<P, false>, Cfg<P>::smem, Cfg<P>::E, 32 / (P + 1)};
 }
 Kernels kernels_of(int p)
 {
@@ -561,6 +639,7 @@ struct dg_ctx2d {
     double *d_U0 = nullptr, *d_Ua = nullptr, *d_Ub = nullptr, *d_acc = nullptr, *d_res = nullptr;
     d2::Geo* d_geo = nullptr;
     d2::Edge* d_edges = nullptr;
+    int* d_blocks = nullptr;  // d2::Args::block_first, then block_edges
     double* d_elift = nullptr;
     d2::Tab* d_tab = nullptr;
     unsigned* d_status = nullptr;
@@ -570,7 +649,7 @@ struct dg_ctx2d {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int nedge = 0, grid = 1, edge_grid = 1;
     int step_grid = 0;       // blocks of the small-mesh steps, 0: the mesh is too large for them
-    unsigned sync_base = 0;  // their counters' value
+    unsigned sync_base = 0;  // their counter's value
     d2::Args args{};  // tables and geometry of every launch
     dgh::Tables1D t1;
     std::vector<double> coords;  // [nnode][2]
@@ -605,6 +684,7 @@ void release(dg_ctx2d* c)
     cudaFree(c->d_res);
     cudaFree(c->d_geo);
     cudaFree(c->d_edges);
+    cudaFree(c->d_blocks);
     cudaFree(c->d_elift);
     cudaFree(c->d_tab);
     cudaFree(c->d_status);
@@ -613,12 +693,9 @@ void release(dg_ctx2d* c)
     if (c->stream) cudaStreamDestroy(c->stream);
 }
 
-int launch(dg_ctx2d* c, const double* Us, double* out, int mode, double dt)
+d2::Args args_of(const dg_ctx2d* c, int mode, double dt)
 {
     d2::Args a = c->args;
-    a.Us = Us;
-    a.out = out;
-    a.U0 = c->d_U0;
     a.mode = mode;
     a.dt = dt;
     if (mode == d2::kResidual) {  // no inverse mass
@@ -632,6 +709,15 @@ int launch(dg_ctx2d* c, const double* Us, double* out, int mode, double dt)
             a.ME[1][b] = b == n - 1 ? 1.0 : 0.0;
         }
     }
+    return a;
+}
+
+int launch(dg_ctx2d* c, const double* Us, double* out, int mode, double dt)
+{
+    d2::Args a = args_of(c, mode, dt);
+    a.Us = Us;
+    a.out = out;
+    a.U0 = c->d_U0;
     const d2::Kernels k = d2::kernels_of(c->p);
     if (c->nedge > 0) k.edge<<<c->edge_grid, d2::kEdgeThreads, 0, c->stream>>>(a);
     k.stage<<<c->grid, 32, k.smem, c->stream>>>(a);
@@ -720,24 +806,66 @@ void ref_to_phys(const dg_ctx2d* c, int e, double xi, double eta, double& x, dou
     }
 }
 
-// RK4 steps of a small mesh, at most 256 to a launch (queued on the stream)
-int launch_steps(dg_ctx2d* c, double dt, int nsteps)
+// the blocks' edge lists of the one-launch steps: d2::Args::block_first, then block_edges
+std::vector<int> block_edges(const dg_ctx2d* c, const std::vector<d2::Edge>& edges, const d2::Kernels& k)
+{
+    const int nb = c->step_grid, batches = (c->ne + k.elems - 1) / k.elems, n = c->p + 1;
+    std::vector<int> block(c->ne), where(c->ne);  // an element's block, its lifts' place there
+    for (int b = 0; b < nb; ++b) {
+        const int first = d2::first_batch(b, batches, nb);
+        for (int e = first * k.elems; e < std::min(c->ne, d2::first_batch(b + 1, batches, nb) * k.elems); ++e) {
+            block[e] = b;
+            where[e] = (e / k.elems - first) * static_cast<int>(k.smem / sizeof(double)) + e % k.elems * 4 * d2::kNS * n;
+        }
+    }
+    std::vector<int> data(nb + 1, 0);  // the first entries, counted one block on
+    for (const d2::Edge& ed : edges) {
+        ++data[block[ed.eL] + 1];
+        if (block[ed.eR] != block[ed.eL]) ++data[block[ed.eR] + 1];
+    }
+    for (int b = 0; b < nb; ++b) data[b + 1] += data[b];
+    std::vector<int> next(data.begin(), data.end() - 1);
+    data.resize(nb + 1 + 3 * static_cast<size_t>(data[nb]));
+    for (size_t i = 0; i < edges.size(); ++i) {
+        const d2::Edge& ed = edges[i];
+        const int oL = where[ed.eL] + (ed.code & 3) * d2::kNS * n, oR = where[ed.eR] + ((ed.code >> 2) & 3) * d2::kNS * n;
+        const int bL = block[ed.eL], bR = block[ed.eR];
+        auto put = [&](int b, int l, int r) {
+            int* o = &data[nb + 1 + 3 * static_cast<size_t>(next[b]++)];
+            o[0] = static_cast<int>(i);
+            o[1] = l;
+            o[2] = r;
+        };
+        put(bL, oL, bR == bL ? oR : -1);
+        if (bR != bL) put(bR, -1, oR);
+    }
+    return data;
+}
+
+// steps of a small mesh, at most 256 to a launch (queued on the stream): RK4 steps (mode
+// kRK1), or steps of one stage between d_U0 and Ua (see d2::StepArgs)
+int launch_steps(dg_ctx2d* c, int mode, double* Ua, double dt, int nsteps)
 {
     const d2::Kernels k = d2::kernels_of(c->p);
+    const auto kernel = mode == d2::kRK1 ? k.steps : k.single_steps;
     d2::StepArgs s{};
-    s.a = c->args;
-    s.a.dt = dt;
+    s.a = args_of(c, mode, dt);
+    s.mode = mode;
     s.U0 = c->d_U0;
-    s.Ua = c->d_Ua;
+    s.Ua = Ua;
     s.Ub = c->d_Ub;
     s.sync = c->d_status + d2::kSyncWord;
     for (int done = 0; done < nsteps; done += s.nsteps) {
         s.nsteps = std::min(256, nsteps - done);
         s.base = c->sync_base;
         void* args[] = {&s};
-        DG2_CUDA(c, cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k.steps), dim3(c->step_grid), dim3(d2::kStepThreads),
-                                                args, k.smem * d2::kStageWarps, c->stream));
-        c->sync_base += static_cast<unsigned>(c->step_grid) * 4u * s.nsteps;
+        const int stages = (mode == d2::kRK1 ? 4 : 1) * s.nsteps;
+        const void* fn = reinterpret_cast<const void*>(kernel);
+        const dim3 grid(c->step_grid), threads(d2::kStepThreads);
+        const size_t smem = k.smem * d2::kStageWarps;
+        if (stages > 1) DG2_CUDA(c, cudaLaunchCooperativeKernel(fn, grid, threads, args, smem, c->stream));
+        else DG2_CUDA(c, cudaLaunchKernel(fn, grid, threads, args, smem, c->stream));
+        c->sync_base += static_cast<unsigned>(c->step_grid) * (stages - 1u);
     }
     return DG_OK;
 }
@@ -869,9 +997,38 @@ int dg2d_create(const dg_case_desc* cd, const dg_mesh2d_desc* md, dg_ctx2d** out
         if (!d2::make_tab(c->p, c->t1, tab)) return bail(DG_ERR_ARG, "edge trace tables");
 
         if (cudaSetDevice(c->device) != cudaSuccess) return bail(DG_ERR_CUDA, "cudaSetDevice failed");
+        c->nedge = static_cast<int>(edges.size());
+        std::vector<int> blocks;
+        const d2::Kernels k = d2::kernels_of(c->p);
+        int per_sm = 0, edge_per_sm = 0, sms = 0;
+        if (cudaFuncSetAttribute(reinterpret_cast<const void*>(k.stage), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(k.smem)) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(k.stage), 32, k.smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&edge_per_sm, reinterpret_cast<const void*>(k.edge), d2::kEdgeThreads, 0) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess)
+            return bail(DG_ERR_CUDA, "kernel attributes");
+        c->grid = std::max(1, std::min((c->ne + k.elems - 1) / k.elems, std::max(1, per_sm) * std::max(1, sms)));
+        // small meshes: one batch of elements per warp, at most one block per SM
+        const int warps = (c->ne + k.elems - 1) / k.elems;
+        if (warps <= sms * d2::kStageWarps) {
+            int steps_per_sm = 0;
+            const int smem = static_cast<int>(k.smem * d2::kStageWarps);
+            int fits = 1;
+            for (const auto kernel : {k.steps, k.single_steps}) {
+                if (cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&steps_per_sm, reinterpret_cast<const void*>(kernel), d2::kStepThreads, smem) != cudaSuccess)
+                    return bail(DG_ERR_CUDA, "kernel attributes");
+                fits = std::min(fits, steps_per_sm);
+            }
+            if (fits > 0) {
+                c->step_grid = std::min(sms, warps);
+                blocks = block_edges(c, edges, k);
+            }
+        }
+        const int per_cta = k.edges_per_warp * (d2::kEdgeThreads / 32);
+        c->edge_grid = std::max(1, std::min((c->nedge + per_cta - 1) / per_cta, std::max(1, edge_per_sm) * std::max(1, sms)));
         const size_t nstate = static_cast<size_t>(c->ne) * d2::kNS * c->nb * sizeof(double);
         const size_t lift_bytes = static_cast<size_t>(c->ne) * 4 * d2::kNS * (c->p + 1) * sizeof(double);
-        c->nedge = static_cast<int>(edges.size());
         bool ok = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess &&
                   cudaEventCreate(&c->ev0) == cudaSuccess && cudaEventCreate(&c->ev1) == cudaSuccess &&
                   cudaMalloc((void**)&c->d_U0, nstate) == cudaSuccess && cudaMalloc((void**)&c->d_Ua, nstate) == cudaSuccess &&
@@ -879,6 +1036,7 @@ int dg2d_create(const dg_case_desc* cd, const dg_mesh2d_desc* md, dg_ctx2d** out
                   cudaMalloc((void**)&c->d_res, nstate) == cudaSuccess &&
                   cudaMalloc((void**)&c->d_geo, geo.size() * sizeof(d2::Geo)) == cudaSuccess &&
                   cudaMalloc((void**)&c->d_edges, std::max<size_t>(1, edges.size()) * sizeof(d2::Edge)) == cudaSuccess &&
+                  (blocks.empty() || cudaMalloc((void**)&c->d_blocks, blocks.size() * sizeof(int)) == cudaSuccess) &&
                   cudaMalloc((void**)&c->d_elift, lift_bytes) == cudaSuccess &&
                   cudaMalloc((void**)&c->d_tab, sizeof(d2::Tab)) == cudaSuccess &&
                   cudaMalloc((void**)&c->d_status, d2::kStatusWords * sizeof(unsigned)) == cudaSuccess;
@@ -888,6 +1046,7 @@ int dg2d_create(const dg_case_desc* cd, const dg_mesh2d_desc* md, dg_ctx2d** out
         }
         ok = cudaMemcpy(c->d_geo, geo.data(), geo.size() * sizeof(d2::Geo), cudaMemcpyHostToDevice) == cudaSuccess &&
              (edges.empty() || cudaMemcpy(c->d_edges, edges.data(), edges.size() * sizeof(d2::Edge), cudaMemcpyHostToDevice) == cudaSuccess) &&
+             (blocks.empty() || cudaMemcpy(c->d_blocks, blocks.data(), blocks.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess) &&
              cudaMemset(c->d_elift, 0, lift_bytes) == cudaSuccess &&
              cudaMemcpy(c->d_tab, &tab, sizeof(d2::Tab), cudaMemcpyHostToDevice) == cudaSuccess &&
              cudaMemset(c->d_status, 0, d2::kStatusWords * sizeof(unsigned)) == cudaSuccess &&
@@ -899,6 +1058,8 @@ int dg2d_create(const dg_case_desc* cd, const dg_mesh2d_desc* md, dg_ctx2d** out
         a.acc = c->d_acc;
         a.geo = c->d_geo;
         a.edges = c->d_edges;
+        a.block_first = c->d_blocks;
+        a.block_edges = reinterpret_cast<const d2::BlockEdge*>(c->d_blocks + c->step_grid + 1);
         a.elift = c->d_elift;
         a.tab = c->d_tab;
         a.status = c->d_status;
@@ -924,27 +1085,6 @@ int dg2d_create(const dg_case_desc* cd, const dg_mesh2d_desc* md, dg_ctx2d** out
             a.ME[0][b] = c->t1.Minv[b * n];
             a.ME[1][b] = c->t1.Minv[b * n + n - 1];
         }
-        const d2::Kernels k = d2::kernels_of(c->p);
-        int per_sm = 0, edge_per_sm = 0, sms = 0;
-        if (cudaFuncSetAttribute(reinterpret_cast<const void*>(k.stage), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(k.smem)) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(k.stage), 32, k.smem) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&edge_per_sm, reinterpret_cast<const void*>(k.edge), d2::kEdgeThreads, 0) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess)
-            return bail(DG_ERR_CUDA, "kernel attributes");
-        c->grid = std::max(1, std::min((c->ne + k.elems - 1) / k.elems, std::max(1, per_sm) * std::max(1, sms)));
-        // small meshes: one batch of elements per warp, at most one block per SM
-        const int warps = (c->ne + k.elems - 1) / k.elems;
-        if (warps <= sms * d2::kStageWarps) {
-            int steps_per_sm = 0;
-            const int smem = static_cast<int>(k.smem * d2::kStageWarps);
-            if (cudaFuncSetAttribute(reinterpret_cast<const void*>(k.steps), cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&steps_per_sm, reinterpret_cast<const void*>(k.steps), d2::kStepThreads, smem) != cudaSuccess)
-                return bail(DG_ERR_CUDA, "kernel attributes");
-            if (steps_per_sm > 0) c->step_grid = std::min(sms, warps);
-        }
-        const int per_cta = k.edges_per_warp * (d2::kEdgeThreads / 32);
-        c->edge_grid = std::max(1, std::min((c->nedge + per_cta - 1) / per_cta, std::max(1, edge_per_sm) * std::max(1, sms)));
     } catch (const std::bad_alloc&) {
         return bail(DG_ERR_NOMEM, "host allocation failed");
     }
@@ -983,7 +1123,7 @@ int dg2d_residual(dg_ctx2d* c, double* res)
 {
     if (!c || !res) return fail2(c, DG_ERR_ARG, "dg2d_residual: null argument");
     DG2_CUDA(c, cudaSetDevice(c->device));
-    int rc = launch(c, c->d_U0, c->d_res, d2::kResidual, 0.0);
+    int rc = c->step_grid ? launch_steps(c, d2::kResidual, c->d_res, 0.0, 1) : launch(c, c->d_U0, c->d_res, d2::kResidual, 0.0);
     if (rc) return rc;
     if ((rc = check_status(c))) return rc;
     return to_host(c, c->d_res, res, c->d_Ub);
@@ -997,7 +1137,7 @@ int dg2d_rk4_steps_timed(dg_ctx2d* c, double dt, int nsteps, double* device_ms)
     if (rc) return rc;
     DG2_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     if (c->step_grid) {
-        if ((rc = launch_steps(c, dt, nsteps))) return rc;
+        if ((rc = launch_steps(c, d2::kRK1, c->d_Ua, dt, nsteps))) return rc;
     } else {
         for (int s = 0; s < nsteps; ++s) DG2_CUDA(c, cudaGraphLaunch(c->graph_exec, c->stream));
     }
@@ -1017,6 +1157,12 @@ int dg2d_fe_steps(dg_ctx2d* c, double dt, int nsteps)
 {
     if (!c || nsteps < 0 || !(dt > 0.0)) return fail2(c, DG_ERR_ARG, "dg2d_fe_steps: bad argument");
     DG2_CUDA(c, cudaSetDevice(c->device));
+    if (c->step_grid) {
+        const int rc = launch_steps(c, d2::kFE, c->d_Ua, dt, nsteps);
+        if (rc) return rc;
+        if (nsteps % 2) std::swap(c->d_U0, c->d_Ua);
+        return check_status(c);
+    }
     // the update reads its neighbours' stage state, so it writes another buffer
     for (int s = 0; s < nsteps; ++s) {
         int rc = launch(c, c->d_U0, c->d_Ua, d2::kFE, dt);
