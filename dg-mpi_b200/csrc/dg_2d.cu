@@ -48,6 +48,8 @@
 
 namespace dgi {
 int fail(dg_ctx* c, int code, const std::string& msg);
+unsigned* take_status_slot();
+void give_status_slot(unsigned* p);
 }
 
 namespace d2 {
@@ -643,6 +645,7 @@ struct dg_ctx2d {
     double* d_elift = nullptr;
     d2::Tab* d_tab = nullptr;
     unsigned* d_status = nullptr;
+    unsigned* h_status = nullptr;  // its pinned copy on the host (or null: see dgi::take_status_slot)
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     double graph_dt = 0.0;
@@ -691,6 +694,7 @@ void release(dg_ctx2d* c)
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->stream) cudaStreamDestroy(c->stream);
+    dgi::give_status_slot(c->h_status);
 }
 
 d2::Args args_of(const dg_ctx2d* c, int mode, double dt)
@@ -727,9 +731,12 @@ int launch(dg_ctx2d* c, const double* Us, double* out, int mode, double dt)
 
 int check_status(dg_ctx2d* c)
 {
-    unsigned s = 0;
-    DG2_CUDA(c, cudaMemcpyAsync(&s, c->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+    unsigned word = 0;
+    if (!c->h_status) c->h_status = dgi::take_status_slot();
+    unsigned* to = c->h_status ? c->h_status : &word;
+    DG2_CUDA(c, cudaMemcpyAsync(to, c->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     DG2_CUDA(c, cudaStreamSynchronize(c->stream));
+    const unsigned s = *to;
     if (s & dgk::kStatusTimeout) {
         DG2_CUDA(c, cudaMemsetAsync(c->d_status, 0, d2::kStatusWords * sizeof(unsigned), c->stream));
         DG2_CUDA(c, cudaStreamSynchronize(c->stream));
