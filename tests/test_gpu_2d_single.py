@@ -61,3 +61,21 @@ def test_steps_of_a_call_are_single_calls_2d(p):
         step(1e-4, nsteps)
         assert np.array_equal(gpu.get_state(), one_by_one)
         assert gpu.status() == 0
+
+
+@pytest.mark.parametrize("p", [0, 1, 3, 5])
+def test_states_return_whatever_their_size_2d(p):
+    """Set and get return every bit at the sizes around the 16384 values up to which
+    the host transposes a state; a non-physical residual leaves an error, not values."""
+    per = 4 * (p + 1) ** 2
+    rng = np.random.default_rng(p)
+    for ne in (1, 16384 // per, 16384 // per + 1):
+        mesh = dg_b200.periodic_box_2d((ne, 1), (0.0, 0.0), (10.0, 9.0))
+        gpu = dg_b200.Case2D(mesh, p, gas_constant=1.0)
+        U = rng.standard_normal((ne, (p + 1) ** 2, 4))
+        gpu.set_state(U)
+        assert np.array_equal(gpu.get_state(), U)
+        U[:, :, 0] = -1.0
+        gpu.set_state(U)
+        with pytest.raises(dg_b200.DGError, match="NONPHYSICAL"):
+            gpu.residual()
