@@ -903,8 +903,12 @@ struct FacePhases {
                 for (int k = 0; k < 4; ++k) nd[k] = T(a.gnrm[((size_t)fd.side * 4 + k) * NF + c]);
             }
             const double eref = kShift ? a.geo[fd.cls].eref : 0.0;
-            if (!kShift && a.flux == 0) dgp::flux_lax_friedrichs_sq(T(a.gamma), UL, UR, nd, nd[3], Fo);
-            else numerical_flux<T, kShift>(a.flux, a.gamma, UL, UR, nd, eref, Fo, status);
+            bool done = false;
+            if constexpr (!kShift) {
+                done = a.flux == 0;
+                if (done) dgp::flux_lax_friedrichs_sq(a.gamma, UL, UR, nd, nd[3], Fo);
+            }
+            if (!done) numerical_flux<T, kShift>(a.flux, a.gamma, UL, UR, nd, eref, Fo, status);
             const T w = Wt[c % M] * Wt[c / M];
 #pragma unroll
             for (int v = 0; v < 5; ++v) To[v * FS + c] = Fo[v] * w;

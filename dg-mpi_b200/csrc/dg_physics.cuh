@@ -5,6 +5,7 @@
 // rounds like the reference's; citations are relative to the reference root.
 #pragma once
 #include <cmath>
+#include <cstring>
 #include <math.h>
 
 #ifdef __CUDACC__
@@ -124,15 +125,15 @@ DG_HD T interior_flux_r1(T gamma, const T* U, T* F, T hr = T(0))
 }
 
 // One side of a face for the Lax-Friedrichs flux: the normal flux F(U).n_hat
-// = m (m.n_hat)/rho + P n_hat, (rE + P)(m.n_hat)/rho, and the wave speed
-// |m|/rho + sqrt(gamma P / rho) of get_maxwavespeed, with one reciprocal.
+// = m (m.n_hat)/rho + P n_hat, (rE + P)(m.n_hat)/rho, with one reciprocal; m2 = |m|^2,
+// r1 = 1 / rho and c2 = gamma P / rho for the wave speed.
 // SHIFT as for interior_flux_r1, with pref = (gamma-1) E_ref restoring the
-// full pressure in the wave speed.
+// full pressure in c2.
 template <typename T, bool SHIFT = false>
-DG_HD T lf_side(T gamma, const T* U, const T* n_hat, T* Fn, T hr = T(0), T pref = T(0))
+DG_HD void lf_normal_flux(T gamma, const T* U, const T* n_hat, T* Fn, T& m2, T& r1, T& c2, T hr = T(0), T pref = T(0))
 {
-    const T r1 = T(1.) / U[0];
-    const T m2 = U[1] * U[1] + U[2] * U[2] + U[3] * U[3];
+    r1 = T(1.) / U[0];
+    m2 = U[1] * U[1] + U[2] * U[2] + U[3] * U[3];
     const T P = (gamma - T(1.0)) * (U[4] - T(0.5) * (m2 * r1));
     const T mn = U[1] * n_hat[0] + U[2] * n_hat[1] + U[3] * n_hat[2];
     const T vn = mn * r1;
@@ -141,7 +142,16 @@ DG_HD T lf_side(T gamma, const T* U, const T* n_hat, T* Fn, T hr = T(0), T pref 
     Fn[2] = U[2] * vn + P * n_hat[1];
     Fn[3] = U[3] * vn + P * n_hat[2];
     Fn[4] = (SHIFT ? U[4] + P + hr : U[4] + P) * vn;
-    return sqrt(m2) * r1 + sqrt(gamma * (SHIFT ? P + pref : P) * r1);
+    c2 = gamma * (SHIFT ? P + pref : P) * r1;
+}
+
+// ... and the wave speed |m|/rho + sqrt(gamma P / rho) of get_maxwavespeed
+template <typename T, bool SHIFT = false>
+DG_HD T lf_side(T gamma, const T* U, const T* n_hat, T* Fn, T hr = T(0), T pref = T(0))
+{
+    T m2, r1, c2;
+    lf_normal_flux<T, SHIFT>(gamma, U, n_hat, Fn, m2, r1, c2, hr, pref);
+    return sqrt(m2) * r1 + sqrt(c2);
 }
 
 // Lax-Friedrichs of the stage kernel: compute_flux_laxfriedrichs with the
@@ -157,30 +167,40 @@ DG_HD void flux_lax_friedrichs_fast(T gamma, const T* UL, const T* UR, const T* 
     for (int s = 0; s < 5; ++s) F[s] = n_mag * (T(0.5) * (FnL[s] + FnR[s]) - T(0.5) * a * (UR[s] - UL[s]));
 }
 
-// flux_lax_friedrichs_fast in three square roots instead of four: the larger
-// wave speed is picked by its square, (u + c)^2 = u^2 + c^2 + 2 sqrt(u^2 c^2),
-// and rooted once.  FP64 (a square root is 13 of an FP64 lane's multiply-adds).
-template <typename T>
-DG_HD void flux_lax_friedrichs_sq(T gamma, const T* UL, const T* UR, const T* n_hat, T n_mag, T* F)
+// 2^-900 <= x < 2^900: no zero, no negative number, no infinity, no NaN
+DG_HD bool mid_range(double x)
 {
-    T Fn[2][5], a2[2];
-    for (int k = 0; k < 2; ++k) {
-        const T* U = k ? UR : UL;
-        const T r1 = T(1.) / U[0];
-        const T m2 = U[1] * U[1] + U[2] * U[2] + U[3] * U[3];
-        const T P = (gamma - T(1.0)) * (U[4] - T(0.5) * (m2 * r1));
-        const T mn = U[1] * n_hat[0] + U[2] * n_hat[1] + U[3] * n_hat[2];
-        const T vn = mn * r1;
-        Fn[k][0] = mn;
-        Fn[k][1] = U[1] * vn + P * n_hat[0];
-        Fn[k][2] = U[2] * vn + P * n_hat[1];
-        Fn[k][3] = U[3] * vn + P * n_hat[2];
-        Fn[k][4] = (U[4] + P) * vn;
-        const T u2 = m2 * r1 * r1, c2 = gamma * P * r1;
-        a2[k] = u2 + c2 + T(2.0) * sqrt(u2 * c2);
+#ifdef __CUDA_ARCH__
+    const unsigned hi = static_cast<unsigned>(__double2hiint(x));
+#else
+    unsigned long long b;
+    std::memcpy(&b, &x, sizeof(b));
+    const unsigned hi = static_cast<unsigned>(b >> 32);
+#endif
+    return hi - (123u << 20) < (1800u << 20);
+}
+
+// flux_lax_friedrichs_fast in FP64 in three square roots instead of four (one is 13 of
+// an FP64 lane's multiply-adds): the larger wave speed is picked by its square,
+// (u + c)^2 = u^2 + c^2 + 2 sqrt(u^2 c^2), and rooted once.  Where a speed is zero, not a
+// number or beyond the range of its square, or a density negative, by the speeds
+// themselves: u^2 c^2 over- and underflows before they do, and a state at rest with a
+// negative pressure has to give a NaN, which the next stage reports.
+DG_HD void flux_lax_friedrichs_sq(double gamma, const double* UL, const double* UR, const double* n_hat, double n_mag, double* F)
+{
+    double FnL[5], FnR[5], mL, mR, rL, rR, cL, cR;
+    lf_normal_flux(gamma, UL, n_hat, FnL, mL, rL, cL);
+    lf_normal_flux(gamma, UR, n_hat, FnR, mR, rR, cR);
+    const double uL = mL * rL * rL, uR = mR * rR * rR, ucL = uL * cL, ucR = uR * cR;
+    double a;
+    if (mid_range(ucL) && mid_range(ucR) && mid_range(UL[0]) && mid_range(UR[0])) {
+        const double aL = uL + cL + 2.0 * sqrt(ucL), aR = uR + cR + 2.0 * sqrt(ucR);
+        a = sqrt(aR > aL ? aR : aL);
+    } else {
+        const double aL = sqrt(mL) * rL + sqrt(cL), aR = sqrt(mR) * rR + sqrt(cR);
+        a = aR > aL ? aR : aL;
     }
-    const T a = sqrt(a2[1] > a2[0] ? a2[1] : a2[0]);
-    for (int s = 0; s < 5; ++s) F[s] = n_mag * (T(0.5) * (Fn[0][s] + Fn[1][s]) - T(0.5) * a * (UR[s] - UL[s]));
+    for (int s = 0; s < 5; ++s) F[s] = n_mag * (0.5 * (FnL[s] + FnR[s]) - 0.5 * a * (UR[s] - UL[s]));
 }
 
 // Lax-Friedrichs with the face's normal data precomputed (it is constant on a
