@@ -437,6 +437,7 @@ struct StepArgs {
     int nsteps, mode;
     unsigned* sync;  // arrivals of the stage warps, one per block and stage but the launch's last
     unsigned base;   // its value before the launch
+    long long wait_cycles;  // limit of a wait
 };
 constexpr int kStageWarps = 4, kEdgeWarps = 4, kStepThreads = 32 * (kStageWarps + kEdgeWarps);
 
@@ -527,7 +528,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) steps2d_kernel(const __grid_c
             } else {
                 if (step > 0 || stage > 1) {
                     target += nb;
-                    ok = dgk::role_wait<32 * kEdgeWarps>(s.sync, target, s.a.status, &dead, 3, threadIdx.x - 32 * kStageWarps);
+                    ok = dgk::role_wait<32 * kEdgeWarps>(s.sync, target, s.wait_cycles, s.a.status, &dead, 3, threadIdx.x - 32 * kStageWarps);
                 }
                 if (share) asm volatile("bar.arrive 4, %0;" ::"n"(kStepThreads) : "memory");
                 if (ok) block_edge_phase<P>(s.a, Us, mode, T, w - kStageWarps, workers, i0, i1, sm, status);
@@ -877,21 +878,24 @@ std::vector<int> block_edges(const dg_ctx2d* c, const std::vector<d2::Edge>& edg
 }
 
 // steps of a small mesh, at most 256 to a launch (queued on the stream): RK4 steps (mode
-// kRK1), or steps of one stage between d_U0 and Ua (see d2::StepArgs)
-int launch_steps(dg_ctx2d* c, int mode, double* Ua, double dt, int nsteps)
+// kRK1), or steps of one stage between d_U0 and Ua (see d2::StepArgs).  A probe of the waits
+// withholds an arrival: they then run to their limit.
+int launch_steps(dg_ctx2d* c, int mode, double* Ua, double dt, int nsteps, long long wait_cycles = dgk::kSmallWaitCycles,
+                 unsigned withheld = 0)
 {
     const d2::Kernels k = d2::kernels_of(c->p);
     const auto kernel = mode == d2::kRK1 ? k.steps : k.single_steps;
     d2::StepArgs s{};
     s.a = args_of(c, mode, dt);
     s.mode = mode;
+    s.wait_cycles = wait_cycles;
     s.U0 = c->d_U0;
     s.Ua = Ua;
     s.Ub = c->d_Ub;
     s.sync = c->d_status + d2::kSyncWord;
     for (int done = 0; done < nsteps; done += s.nsteps) {
         s.nsteps = std::min(256, nsteps - done);
-        s.base = c->sync_base;
+        s.base = c->sync_base + withheld;
         void* args[] = {&s};
         const int stages = (mode == d2::kRK1 ? 4 : 1) * s.nsteps;
         const void* fn = reinterpret_cast<const void*>(kernel);
@@ -1297,6 +1301,16 @@ int dg2d_l2_error(dg_ctx2d* c, int ic_type, const double* data, int ndata, doubl
     }
     for (int v = 0; v < d2::kNS; ++v) err[v] = std::sqrt(tot[v] / vol);
     return DG_OK;
+}
+
+int dg2d_probe_step_wait(dg_ctx2d* c, long long limit_cycles)
+{
+    if (!c || limit_cycles < 0 || limit_cycles > 4000000000LL)
+        return fail2(c, DG_ERR_ARG, "dg2d_probe_step_wait: limit must be 0 .. 4e9 SM cycles (about 2 s)");
+    if (!c->step_grid) return fail2(c, DG_ERR_UNSUPPORTED, "dg2d_probe_step_wait: steps of this mesh do not wait on the device");
+    DG2_CUDA(c, cudaSetDevice(c->device));
+    const int rc = launch_steps(c, d2::kRK1, c->d_Ua, 0.0, 1, limit_cycles, 1);
+    return rc ? rc : check_status(c);
 }
 
 int dg2d_status(dg_ctx2d* c, unsigned* flags)

@@ -1774,10 +1774,11 @@ int launch_stage_chunked(dg_ctx* c, int stage, int mode, const double* Us, const
 }
 
 // RK4 steps in the small-mesh kernel, at most kSmallSteps to a launch (queued
-// on the context's stream)
+// on the context's stream).  A probe of the kernel's waits withholds an arrival: they
+// then run to their limit.
 constexpr int kSmallSteps = 256;
 
-int launch_small_steps(dg_ctx* c, double dt, int nsteps)
+int launch_small_steps(dg_ctx* c, double dt, int nsteps, long long wait_cycles = dgk::kSmallWaitCycles, unsigned withheld = 0)
 {
     int rc = prepare_variant(c, c->variant);
     if (rc) return rc;
@@ -1791,9 +1792,10 @@ int launch_small_steps(dg_ctx* c, double dt, int nsteps)
     s.Ub = c->d_Ub;
     s.fpt = std::min(sv.small_face_batch, (c->nface + warps - 1) / warps);
     s.sync = c->d_status + kSyncWord;
+    s.wait_cycles = wait_cycles;
     for (int done = 0; done < nsteps; done += s.nsteps) {
         s.nsteps = std::min(kSmallSteps, nsteps - done);
-        s.base = c->sync_base;
+        s.base = c->sync_base + withheld;
         s.done_base = c->done_base;
         s.host_status = done + s.nsteps == nsteps ? c->h_status : nullptr;
         DG_CUDA(c, sv.small_launch(s, grid, c->stream));
@@ -2096,6 +2098,16 @@ int dg_probe_bounded_wait(int device, long long limit_cycles, int arrive, long l
         return fail(nullptr, DG_ERR_TIMEOUT,
                     "dg_probe_bounded_wait: the bounded wait gave up after " + std::to_string(cyc) + " SM cycles");
     return DG_OK;
+}
+
+int dg_probe_step_wait(dg_ctx* c, long long limit_cycles)
+{
+    if (!c || limit_cycles < 0 || limit_cycles > 4000000000LL)
+        return fail(c, DG_ERR_ARG, "dg_probe_step_wait: limit must be 0 .. 4e9 SM cycles (about 2 s)");
+    if (!runs_small(c)) return fail(c, DG_ERR_UNSUPPORTED, "dg_probe_step_wait: steps of this context do not wait on the device");
+    DG_CUDA(c, cudaSetDevice(c->device));
+    const int rc = launch_small_steps(c, 0.0, 1, limit_cycles, 1);
+    return rc ? rc : check_status(c);
 }
 
 int dg_kinetic_energy_noalloc(int order, int nelem, const double* d_state, const double* d_djac, double* d_ke,

@@ -42,6 +42,7 @@ struct SmallArgs {
     unsigned base;        // both counters' value before the launch
     unsigned done_base;   // and that of the finished blocks' counter, sync[64]
     unsigned* host_status;  // pinned copy of the status word, written by the last block (or null)
+    long long wait_cycles;  // limit of a wait
 };
 
 // stage 1 .. 4 of a step
@@ -69,7 +70,7 @@ struct GroupSync {
     __device__ __forceinline__ void operator()() const { named_sync<NT>(id); }
 };
 
-constexpr long long kSmallWaitCycles = 2000000000ll;  // about a second
+constexpr long long kSmallWaitCycles = 2000000000ll;  // about a second, the limit outside of probes
 
 // one arrival for the block by the NT threads of a role, whose writes it publishes
 template <int NT>
@@ -82,14 +83,14 @@ __device__ __forceinline__ void role_arrive(unsigned* count, int id, int tid)
     }
 }
 // waits until the counter has reached target; false (for all threads) when the
-// wait or another block gave up
+// wait, after `limit` SM cycles, or another block gave up
 template <int NT>
-__device__ __forceinline__ bool role_wait(unsigned* count, unsigned target, unsigned* status, int* dead, int id, int tid)
+__device__ __forceinline__ bool role_wait(unsigned* count, unsigned target, long long limit, unsigned* status, int* dead, int id, int tid)
 {
     if (tid == 0) {
         const long long t0 = clock64();
         while (static_cast<int>(*reinterpret_cast<volatile unsigned*>(count) - target) < 0) {
-            if (*reinterpret_cast<volatile unsigned*>(status) & kStatusTimeout || clock64() - t0 > kSmallWaitCycles) {
+            if (*reinterpret_cast<volatile unsigned*>(status) & kStatusTimeout || clock64() - t0 > limit) {
                 atomicOr(status, kStatusTimeout);
                 *dead = 1;
                 break;
@@ -145,7 +146,7 @@ small_steps_kernel(const __grid_constant__ SmallArgs s)
                     c.contract_y(s.a);
                 }
                 target += nb;
-                ok = role_wait<CG * NT>(s.sync + 32, target, s.a.status, dead, 1, threadIdx.x);
+                ok = role_wait<CG * NT>(s.sync + 32, target, s.wait_cycles, s.a.status, dead, 1, threadIdx.x);
                 if (!ok) break;
                 if (active) {
                     c.lifts(s.a, e0);
@@ -183,7 +184,7 @@ small_steps_kernel(const __grid_constant__ SmallArgs s)
             for (int stage = 1; stage <= 4; ++stage) {
                 if (step > 0 || stage > 1) {
                     target += nb;
-                    ok = role_wait<FW * 32>(s.sync, target, s.a.status, dead + 1, 2, ft);
+                    ok = role_wait<FW * 32>(s.sync, target, s.wait_cycles, s.a.status, dead + 1, 2, ft);
                     if (!ok) break;
                 }
                 io.stage = stage;

@@ -162,6 +162,8 @@ def library(path: str | None = None) -> ctypes.CDLL:
         "dg2d_project_ic": (ctypes.c_int, [vp, ctypes.c_int, dp, ctypes.c_int, ctypes.c_double, dp]),
         "dg2d_l2_error": (ctypes.c_int, [vp, ctypes.c_int, dp, ctypes.c_int, ctypes.c_double, dp]),
         "dg2d_status": (ctypes.c_int, [vp, up]),
+        "dg2d_probe_step_wait": (ctypes.c_int, [vp, ctypes.c_longlong]),
+        "dg_probe_step_wait": (ctypes.c_int, [vp, ctypes.c_longlong]),
         "dg_mesh2d_periodic_box": (ctypes.c_int, [ip, dp, dp, ctypes.c_uint, ip, dp, ip, up, ip, up]),
         "dg2d_solution_write_h5": (ctypes.c_int, [ctypes.c_char_p, ctypes.POINTER(_MeshDesc), ctypes.c_int, dp,
                                                   ctypes.c_double]),
@@ -577,6 +579,11 @@ class Case:
         self._check(self._lib.dg_tune_stage(self._ctx, int(reps), ctypes.byref(best), _dptr(ms)))
         return best.value, ms.tolist()
 
+    def probe_step_wait(self, limit_cycles: int):
+        """A step in one launch whose waits give up after that many SM cycles
+        (dg_probe_step_wait): raises DG_ERR_TIMEOUT, the state as before."""
+        self._check(self._lib.dg_probe_step_wait(self._ctx, int(limit_cycles)))
+
 
 class Batch:
     """An ensemble of independent cases advanced together (a dg_batch).
@@ -879,3 +886,7 @@ class Case2D:
         f = ctypes.c_uint()
         self._lib.dg2d_status(self._h, ctypes.byref(f))
         return f.value
+
+    def probe_step_wait(self, limit_cycles: int):
+        """As Case.probe_step_wait (dg2d_probe_step_wait)."""
+        self._check(self._lib.dg2d_probe_step_wait(self._h, int(limit_cycles)))

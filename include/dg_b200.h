@@ -273,6 +273,11 @@ int dg_sync(dg_ctx* ctx);
  * took.  The kernel returns normally either way and leaves nothing in flight,
  * so the device stays usable.  Error text: dg_last_error(NULL). */
 int dg_probe_bounded_wait(int device, long long limit_cycles, int arrive, long long* waited_cycles);
+/* The same of the waits between the blocks of RK4 steps in one launch (small meshes): a
+ * step with an arrival withheld, so that each wait gives up after limit_cycles (0 ..
+ * 4e9) and the launch ends.  DG_ERR_TIMEOUT; the state is as before and the context
+ * steps on.  DG_ERR_UNSUPPORTED where the context's steps are other launches. */
+int dg_probe_step_wait(dg_ctx* ctx, long long limit_cycles);
 
 /* Raw device pointers for callers that keep data resident (benchmarks,
  * multi-GPU exchange).  Layout of the device state: [ne][5][nb]. */
@@ -553,6 +558,8 @@ int dg2d_project_ic(dg_ctx2d* ctx, int ic_type, const double* data, int ndata, d
 int dg2d_l2_error(dg_ctx2d* ctx, int ic_type, const double* data, int ndata, double t, double* err);
 /* the device status word (the 3D bits); DG_ERR_NONPHYSICAL when set */
 int dg2d_status(dg_ctx2d* ctx, unsigned* flags);
+/* dg_probe_step_wait for the 2D steps. */
+int dg2d_probe_step_wait(dg_ctx2d* ctx, long long limit_cycles);
 
 /* Periodic box [x0,x0+L0]x[x1,x1+L1] of n0*n1 quadrilaterals, element id
  * i + n0 j; faces (right, top) of each element in element order; with
