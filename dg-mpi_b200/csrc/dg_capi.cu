@@ -415,13 +415,13 @@ struct ReduceArgs {
     const double* J;        // [nclasses][9]
     const double* gnodes;   // general geometry: element nodes [ne][8][3] (else null)
     double* partials;       // [gridDim.x][5]
-    int ne, ic_type, kind;  // kind 0: L2 error, 1: kinetic energy
+    int ne, ic_type;
     double gamma, R, t;
     double data[16];
 };
 
-// Points per direction (the error's rule of 2 max(p,1) + 2, the kinetic
-// energy's volume rule), elements and threads per CTA: one thread per (x, y)
+// KIND 0: L2 error, 1: kinetic energy.  Points per direction (the error's rule of
+// 2 max(p,1) + 2, the kinetic energy's volume rule), elements and threads per CTA: one thread per (x, y)
 // point column of an element, whole elements to a CTA of about 128 threads. With SPREAD
 // one element to a CTA and KS threads to a column, each taking every KS-th point.
 template <int P, int KIND, bool SPREAD>
@@ -622,7 +622,6 @@ int run_reduce(dg_ctx* c, int kind, int ic_type, const double* data, int ndata, 
     a.partials = c->d_partials;
     a.ne = ne;
     a.ic_type = ic_type;
-    a.kind = kind;
     a.gamma = gamma;
     a.R = R;
     a.t = t;

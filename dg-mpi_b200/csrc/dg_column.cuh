@@ -301,36 +301,30 @@ struct Column {
     // the batch's face lifts on their way into shared memory
     __device__ __forceinline__ void lifts(const StageArgs& a, int e0)
     {
-            const T* gL = reinterpret_cast<const T*>(a.fflux);
-            const int tid = opaque<F64 && P >= 4>(tid0);
+        const T* gL = reinterpret_cast<const T*>(a.fflux);
+        const int tid = opaque<F64 && P >= 4>(tid0);
 #pragma unroll
-            for (int r = 0; r < RL; ++r) {
-                const int i = tid + r * NT;
-                if (i < LT) {
-                    const int c = i % N2, f = (i / N2) % 6, e = i / (6 * N2);
-                    const int ge = min(e0 + e, a.ne - 1);
-                    const int pc = ((fl[r] >> 30) & 1) ? c : a.cmapn[(a.frec[(size_t)ge * 6 + f].info >> 4) * N2 + c];
-                    const T* src = gL + (size_t)(fl[r] & 0x3fffffff) * a.fstride + pc;
-                    T* dst = sL + e * L::LF + f * 5 * N2 + c;
+        for (int r = 0; r < RL; ++r) {
+            const int i = tid + r * NT;
+            if (i < LT) {
+                const int c = i % N2, f = (i / N2) % 6, e = i / (6 * N2);
+                const int ge = min(e0 + e, a.ne - 1);
+                const int pc = ((fl[r] >> 30) & 1) ? c : a.cmapn[(a.frec[(size_t)ge * 6 + f].info >> 4) * N2 + c];
+                const T* src = gL + (size_t)(fl[r] & 0x3fffffff) * a.fstride + pc;
+                T* dst = sL + e * L::LF + f * 5 * N2 + c;
 #pragma unroll
-                    for (int v = 0; v < 5; ++v) cp_async_t(dst + v * N2, src + v * N2);
-                    if (c == 0) sSgn[e * 6 + f] = fl[r] < 0 ? T(-1) : T(1);
-                }
+                for (int v = 0; v < 5; ++v) cp_async_t(dst + v * N2, src + v * N2);
+                if (c == 0) sSgn[e * 6 + f] = fl[r] < 0 ? T(-1) : T(1);
             }
-            classes();
-            cp_async_commit();
+        }
+        classes();
+        cp_async_commit();
     }
 
     // x interpolation of the fetched rows
     __device__ __forceinline__ void interp_x(const StageArgs& a)
     {
         const T* __restrict__ Bt = TabSel<T>::B(a.tab);
-        const T* __restrict__ Wt = TabSel<T>::W(a.tab);
-        const T* __restrict__ Ct = ColTab<T>::B(a.tab);
-        const T* __restrict__ Dt = ColTab<T>::D(a.tab);
-        const double* __restrict__ Mi = a.tab.Minv;
-        const T gamma = T(a.gamma);
-        (void)Bt, (void)Wt, (void)Ct, (void)Dt, (void)Mi, (void)gamma;
         const int tid = opaque<F64 && P >= 4>(tid0);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -360,9 +354,7 @@ struct Column {
         const T* __restrict__ Wt = TabSel<T>::W(a.tab);
         const T* __restrict__ Ct = ColTab<T>::B(a.tab);
         const T* __restrict__ Dt = ColTab<T>::D(a.tab);
-        const double* __restrict__ Mi = a.tab.Minv;
         const T gamma = T(a.gamma);
-        (void)Bt, (void)Wt, (void)Ct, (void)Dt, (void)Mi, (void)gamma;
         const int tid = opaque<F64 && P >= 5>(tid0);
         sync();
         // ---- y interpolation ----
@@ -512,13 +504,8 @@ struct Column {
 
     __device__ __forceinline__ void contract_y(const StageArgs& a)
     {
-        const T* __restrict__ Bt = TabSel<T>::B(a.tab);
-        const T* __restrict__ Wt = TabSel<T>::W(a.tab);
         const T* __restrict__ Ct = ColTab<T>::B(a.tab);
         const T* __restrict__ Dt = ColTab<T>::D(a.tab);
-        const double* __restrict__ Mi = a.tab.Minv;
-        const T gamma = T(a.gamma);
-        (void)Bt, (void)Wt, (void)Ct, (void)Dt, (void)Mi, (void)gamma;
         const int tid = opaque<F64 && P >= 4>(tid0);
         // ---- y contraction: By^T A0 over row 3v, Dy^T A1 + By^T A2 over row 3v+1 ----
 #pragma unroll 1
@@ -591,13 +578,9 @@ struct Column {
     // x contraction, face lifts, inverse mass (FP32 path) and stage update
     __device__ __forceinline__ void finish(const StageArgs& a, int e0)
     {
-        const T* __restrict__ Bt = TabSel<T>::B(a.tab);
-        const T* __restrict__ Wt = TabSel<T>::W(a.tab);
         const T* __restrict__ Ct = ColTab<T>::B(a.tab);
         const T* __restrict__ Dt = ColTab<T>::D(a.tab);
-        const double* __restrict__ Mi = a.tab.Minv;
-        const T gamma = T(a.gamma);
-        (void)Bt, (void)Wt, (void)Ct, (void)Dt, (void)Mi, (void)gamma;
+        [[maybe_unused]] const double* __restrict__ Mi = a.tab.Minv;
         const int tid = opaque<F64 && P >= 4>(tid0);
         // ---- x contraction, face lifts; FP64: the stage update ----
 #pragma unroll 1

@@ -54,7 +54,7 @@ struct dg_ctx {
     // the side whose point order their flux is stored in -- first the nface_inner
     // faces that touch an interior element (computed with the interior
     // elements, before the halo exchange ends), then the others -- and the
-    // face kernel's fluxes [nface][5][(p+2)^2]
+    // face kernel's fluxes [nface][5][(p+2)^2] (column form: lifted, [nface][5][(p+1)^2])
     int nface = 0, nface_inner = 0;
     int2* d_faces = nullptr;
     // the column form's face descriptors and element-to-face records, in d_faces' allocation

@@ -1,8 +1,8 @@
 // dg_physics.cuh -- pointwise 3D Euler physics shared by the host C++ side and
 // the CUDA kernels: pressure, wave speed, interior flux, Lax-Friedrichs and
 // HLLC numerical fluxes, initial conditions / exact solutions.  Operation
-// order follows the reference's functions so that a face flux computed here
-// rounds like the reference's; citations are relative to the reference root.
+// order follows the reference's functions but where a comment says otherwise;
+// citations are relative to the reference root.
 #pragma once
 #include <cmath>
 #include <cstring>
@@ -40,57 +40,10 @@ DG_HD T max_wave_speed(T gamma, const T* U)
     return sqrtrKE + sqrt(gamma * pressure(gamma, U) * rho1);
 }
 
-// EulerFcnType::conv_flux_interior<3>, functions.cpp:64-91; F[j*5+s]
-template <typename T>
-DG_HD void interior_flux(T gamma, const T* U, T* F)
-{
-    const T r1 = T(1.) / U[0];
-    const T ru = U[1], rv = U[2], rw = U[3], rE = U[4];
-    const T P = pressure(gamma, U);
-    F[0] = ru;
-    F[1] = ru * ru * r1 + P;
-    F[2] = ru * rv * r1;
-    F[3] = ru * rw * r1;
-    F[4] = (rE + P) * ru * r1;
-    F[5] = rv;
-    F[6] = rv * ru * r1;
-    F[7] = rv * rv * r1 + P;
-    F[8] = rv * rw * r1;
-    F[9] = (rE + P) * rv * r1;
-    F[10] = rw;
-    F[11] = rw * ru * r1;
-    F[12] = rw * rv * r1;
-    F[13] = rw * rw * r1 + P;
-    F[14] = (rE + P) * rw * r1;
-}
-
-// BaseConvNumFluxType::compute_flux_laxfriedrichs<3>, base/functions.cpp:33-89.
-// N is the unnormalised normal of the left element (its length carries the
-// surface Jacobian).
-template <typename T>
-DG_HD void flux_lax_friedrichs(T gamma, const T* UL, const T* UR, const T* N, T* F)
-{
-    T n_mag = T(0.0);
-    for (int d = 0; d < 3; ++d) n_mag += N[d] * N[d];
-    n_mag = sqrt(n_mag);
-    T n_hat[3];
-    for (int d = 0; d < 3; ++d) n_hat[d] = N[d] / n_mag;
-    T Fq[15], FqL[5] = {T(0), T(0), T(0), T(0), T(0)}, FqR[5] = {T(0), T(0), T(0), T(0), T(0)};
-    interior_flux(gamma, UL, Fq);
-    for (int s = 0; s < 5; ++s)
-        for (int d = 0; d < 3; ++d) FqL[s] += Fq[s + d * 5] * n_hat[d];
-    interior_flux(gamma, UR, Fq);
-    for (int s = 0; s < 5; ++s)
-        for (int d = 0; d < 3; ++d) FqR[s] += Fq[s + d * 5] * n_hat[d];
-    T a = max_wave_speed(gamma, UL);
-    const T aR = max_wave_speed(gamma, UR);
-    if (aR > a) a = aR;
-    for (int s = 0; s < 5; ++s) F[s] = n_mag * (T(0.5) * (FqL[s] + FqR[s]) - T(0.5) * a * (UR[s] - UL[s]));
-}
-
-// The interior flux with one reciprocal of the density: P = (gamma-1)(rE -
-// |m|^2 r1 / 2) instead of the reference's division of |m|^2 by rho (the same
-// quantity, rounded differently); returns P for the positivity check.
+// EulerFcnType::conv_flux_interior<3>, functions.cpp:64-91 (F[j*5+s]), with one
+// reciprocal of the density: P = (gamma-1)(rE - |m|^2 r1 / 2) instead of the
+// reference's division of |m|^2 by rho (the same quantity, rounded differently);
+// returns P for the positivity check.
 //
 // SHIFT: the state's energy is stored relative to a constant E_ref
 // (U[4] = rE - E_ref, so that FP32 keeps its digits for the fluctuation when
@@ -154,8 +107,9 @@ DG_HD T lf_side(T gamma, const T* U, const T* n_hat, T* Fn, T hr = T(0), T pref 
     return sqrt(m2) * r1 + sqrt(c2);
 }
 
-// Lax-Friedrichs of the stage kernel: compute_flux_laxfriedrichs with the
-// face's |N| and N/|N| precomputed and lf_side for each state.
+// BaseConvNumFluxType::compute_flux_laxfriedrichs<3>, base/functions.cpp:33-89, with
+// the face's |N| and N / |N| precomputed (n_mag, n_hat; they are the left element's, and
+// |N| carries the surface Jacobian) and lf_side for each state.
 template <typename T, bool SHIFT = false>
 DG_HD void flux_lax_friedrichs_fast(T gamma, const T* UL, const T* UR, const T* n_hat, T n_mag, T* F, T hr = T(0),
                                     T pref = T(0))
@@ -203,42 +157,9 @@ DG_HD void flux_lax_friedrichs_sq(double gamma, const double* UL, const double* 
     for (int s = 0; s < 5; ++s) F[s] = n_mag * (0.5 * (FnL[s] + FnR[s]) - 0.5 * a * (UR[s] - UL[s]));
 }
 
-// Lax-Friedrichs with the face's normal data precomputed (it is constant on a
-// face of an affine element): n_mag = |N| and n_hat = N / n_mag, evaluated
-// once on the host by the formulas of flux_lax_friedrichs.
-template <typename T>
-DG_HD void flux_lax_friedrichs_n(T gamma, const T* UL, const T* UR, const T* n_hat, T n_mag, T* F)
-{
-    T Fq[15], FqL[5] = {T(0), T(0), T(0), T(0), T(0)}, FqR[5] = {T(0), T(0), T(0), T(0), T(0)};
-    interior_flux(gamma, UL, Fq);
-    for (int s = 0; s < 5; ++s)
-        for (int d = 0; d < 3; ++d) FqL[s] += Fq[s + d * 5] * n_hat[d];
-    interior_flux(gamma, UR, Fq);
-    for (int s = 0; s < 5; ++s)
-        for (int d = 0; d < 3; ++d) FqR[s] += Fq[s + d * 5] * n_hat[d];
-    T a = max_wave_speed(gamma, UL);
-    const T aR = max_wave_speed(gamma, UR);
-    if (aR > a) a = aR;
-    for (int s = 0; s < 5; ++s) F[s] = n_mag * (T(0.5) * (FqL[s] + FqR[s]) - T(0.5) * a * (UR[s] - UL[s]));
-}
-
-// EulerConvNumFluxType::compute_flux_hllc<3>, functions.cpp:298-399.
-// Returns false on the reference's assert branch (no valid wave ordering,
-// e.g. NaN input); F is zeroed then.
-template <typename T>
-DG_HD bool flux_hllc_n(T gam, const T* UL, const T* UR, const T* n, T djac, T* F);
-
-template <typename T>
-DG_HD bool flux_hllc(T gam, const T* UL, const T* UR, const T* N, T* F)
-{
-    const T djac = sqrt(N[0] * N[0] + N[1] * N[1] + N[2] * N[2]);
-    const T djac1 = T(1.) / djac;
-    const T n[3] = {N[0] * djac1, N[1] * djac1, N[2] * djac1};
-    return flux_hllc_n(gam, UL, UR, n, djac, F);
-}
-
-// HLLC with the face's unit normal n = N * (1/|N|) and djac = |N| precomputed
-// by the same operations as in flux_hllc.
+// EulerConvNumFluxType::compute_flux_hllc<3>, functions.cpp:298-399, with the face's unit
+// normal n = N * (1/|N|) and djac = |N| precomputed.  Returns false on the reference's
+// assert branch (no valid wave ordering, e.g. NaN input); F is zeroed then.
 template <typename T>
 DG_HD bool flux_hllc_n(T gam, const T* UL, const T* UR, const T* n, T djac, T* F)
 {

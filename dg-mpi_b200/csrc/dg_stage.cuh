@@ -165,7 +165,7 @@ struct StageArgs {
     // launch option FX: the faces as (element, face) of the side whose point
     // order the flux is stored in [nface], the range [face_begin, nface) one
     // face-kernel launch computes, and the fluxes [nface][5][(p+2)^2] (T
-    // values, weights applied, unsigned)
+    // values, weights applied, unsigned; column form: the lifted ones [nface][5][(p+1)^2])
     const int2* faces;
     const FaceDesc* fdesc;  // [nface], the column form's face list
     const int* lrec;        // [ne][6] face | 1 << 30 where its lift is read in its own node order | 1 << 31 on the left side
@@ -390,8 +390,6 @@ __device__ __forceinline__ void cp_async4(float* smem_dst, const float* gmem_src
 __device__ __forceinline__ void cp_async_t(double* d, const double* g) { cp_async8(d, g); }
 __device__ __forceinline__ void cp_async_t(float* d, const float* g) { cp_async4(d, g); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int G>
-__device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;\n" ::"n"(G) : "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 // all but the most recent group complete
 __device__ __forceinline__ void cp_async_wait_older() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
