@@ -121,18 +121,19 @@ DG_HD void flux_lax_friedrichs_fast(T gamma, const T* UL, const T* UR, const T* 
     for (int s = 0; s < 5; ++s) F[s] = n_mag * (T(0.5) * (FnL[s] + FnR[s]) - T(0.5) * a * (UR[s] - UL[s]));
 }
 
-// 2^-900 <= x < 2^900: no zero, no negative number, no infinity, no NaN
-DG_HD bool mid_range(double x)
+// the upper half of x's bits
+DG_HD unsigned upper_bits(double x)
 {
 #ifdef __CUDA_ARCH__
-    const unsigned hi = static_cast<unsigned>(__double2hiint(x));
+    return static_cast<unsigned>(__double2hiint(x));
 #else
     unsigned long long b;
     std::memcpy(&b, &x, sizeof(b));
-    const unsigned hi = static_cast<unsigned>(b >> 32);
+    return static_cast<unsigned>(b >> 32);
 #endif
-    return hi - (123u << 20) < (1800u << 20);
 }
+// 2^-900 <= x < 2^900: no zero, no negative number, no infinity, no NaN
+DG_HD bool mid_range(double x) { return upper_bits(x) - (123u << 20) < (1800u << 20); }
 
 // flux_lax_friedrichs_fast in FP64 in three square roots instead of four (one is 13 of
 // an FP64 lane's multiply-adds): the larger wave speed is picked by its square,
@@ -147,7 +148,8 @@ DG_HD void flux_lax_friedrichs_sq(double gamma, const double* UL, const double* 
     lf_normal_flux(gamma, UR, n_hat, FnR, mR, rR, cR);
     const double uL = mL * rL * rL, uR = mR * rR * rR, ucL = uL * cL, ucR = uR * cR;
     double a;
-    if (mid_range(ucL) && mid_range(ucR) && mid_range(UL[0]) && mid_range(UR[0])) {
+    const bool positive = static_cast<int>(upper_bits(UL[0]) | upper_bits(UR[0])) >= 0;  // densities
+    if (static_cast<int>(mid_range(ucL)) & static_cast<int>(mid_range(ucR)) & static_cast<int>(positive)) {
         const double aL = uL + cL + 2.0 * sqrt(ucL), aR = uR + cR + 2.0 * sqrt(ucR);
         a = sqrt(aR > aL ? aR : aL);
     } else {
