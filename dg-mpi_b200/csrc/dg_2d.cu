@@ -1,6 +1,6 @@
 // dg_2d.cu -- the 2D quadrilateral path (Solver<2> with LagrangeQuad): the
-// residual and RK stage on periodic meshes of parallelograms, FP64, one warp
-// per element, and its C ABI (dg2d_* in dg_b200.h).
+// residual and RK stage on periodic meshes of parallelograms, FP64, and its C
+// ABI (dg2d_* in dg_b200.h).
 //
 // Reference path replaced (the 2D instantiation of the 3D path's functions,
 // citations relative to the reference root): Solver<2>::get_residual
@@ -12,7 +12,7 @@
 // mult_inv_mass_matrix (tools.cpp:124-139) and the RK4 / FE stage updates
 // (stepper.cpp:23-142).
 //
-// Two launches per stage.
+// Two launches per stage, or all steps of a call in one on small meshes (steps2d_kernel).
 //   edge2d_kernel   every interior edge's numerical flux once: one thread per
 //       (edge, Gauss point), the p + 1 threads of an edge in one warp.  Each holds
 //       one edge node of both sides (the other basis functions vanish on the edge
@@ -32,8 +32,8 @@
 // Why: the kernel this replaces ran one task per value through shared memory, two
 // loads to a multiply-add, and each edge's flux twice (512^2, p = 3: load/store and
 // issue bound at 31 % of the FP64 pipe).  RK stage, HLLC, 256^2: p = 1 108 -> 23, p = 2
-// 141 -> 42, p = 3 179 -> 60, p = 4 319 -> 103, p = 5 463 -> 135 us; 64^2, p = 3 16.5 ->
-// 9.8 us.
+// 141 -> 42, p = 3 179 -> 60, p = 4 319 -> 103, p = 5 463 -> 135 us (both kernels); 64^2,
+// p = 3 16.5 -> 9.8 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>

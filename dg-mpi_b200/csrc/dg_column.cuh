@@ -1,4 +1,5 @@
-// dg_column.cuh -- the column form of the DG stage (affine elements, orders 1..5):
+// dg_column.cuh -- the column form of the DG stage (affine elements, orders 1..5;
+// bent ones in FP64, orders 1..3 the default):
 // face_lift_kernel and column_kernel, one launch each per RK stage.
 //
 // Same scheme as dg_stage.cuh's face kernel and stage kernel, with the work cut
@@ -40,8 +41,8 @@
 // -> column form, GDOF/s: FP64 11.7 -> 24.4 (72^3, p = 1), 24.5 -> 39.0 (60^3,
 // p = 2), 31.9 -> 49.4 (48^3, p = 3), 30.2 -> 41.0 (40^3, p = 4), 31.9 -> 42.6
 // (32^3, p = 5); mixed 19.4 -> 29.6, 33.0 -> 44.6, 39.7 -> 55.2, 44.0 -> 52.3,
-// 41.8 -> 53.4.  The FP32 form is bound by instruction issue (3000 per element at
-// p = 3, 64 % of the issue slots): its lift sums take one y and one z face per row
+// 41.8 -> 53.4.  The FP32 form is bound by instruction issue (3288 per element at
+// p = 3, 68 % of the issue slots): its lift sums take one y and one z face per row
 // and its residual block has constant strides (48^3, p = 3: 0.695 -> 0.641 ms).
 #pragma once
 #include "dg_stage.cuh"
@@ -130,7 +131,8 @@ __device__ __forceinline__ void store_row(double* p, const double (&x)[N])
 // completion, which it does in wait_prerequisites (all writes visible); only
 // data that no kernel writes is read before.  Without overlap that call does nothing.
 // FP64 RK stage: p = 1, 14^3 9.3 -> 8.8 us, p = 3, 9^3 12.9 -> 11.8, 16^3 34.3 -> 34.0;
-// nothing from some 20^3 on.  An earlier start (griddepcontrol.launch_dependents at
+// nothing from some 20^3 on; forward Euler's steps within a call the same way (p = 3, 6^3
+// 12.5 -> 11.4).  An earlier start (griddepcontrol.launch_dependents at
 // the kernels' beginning) places the CTAs unevenly: 9^3 15.8 us, 24^3 100 -> 110.
 __device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -785,8 +787,8 @@ __global__ void __launch_bounds__(NT, MB) column_kernel(const __grid_constant__ 
 // Three buffers of face descriptors: the batch's, the next one's (for its
 // gather) and the one after that in flight.
 //
-// Bound by its FP64 chains at 16-18 warps per SM (FP64 pipe 39 %, `wait` the first
-// stall). One thread per slice used to read its 16 strided coefficients, 32
+// Bound by its FP64 chains and shared-memory wavefronts at 16-18 warps per SM (FP64 pipe
+// 48 %, LSU wavefronts 71 %). One thread per slice used to read its 16 strided coefficients, 32
 // cache lines to a load (79 % of the load pipe): 40^3, p = 3, FP64 0.207 -> 0.172
 // ms with the cooperative gather; descriptors, three square roots and one-warp
 // CTAs bring the RK stage of 48^3 from 0.845 to 0.821 ms.

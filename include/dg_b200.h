@@ -153,7 +153,8 @@ int dg_rk4_steps_timed(dg_ctx* ctx, double dt, int nsteps, double* device_ms);
  * mesh and current state (the state is not modified; the RK accumulator, dead
  * between steps, serves as scratch, so call it between steps) and selects the
  * fastest (entries of the other precision or geometry kind report -1 ms); callers cache the result
- * per (order, precision, GPU) and restore it with dg_set_stage_variant.
+ * per (order, precision, GPU) and build -- the list and its order may change between
+ * builds -- and restore it with dg_set_stage_variant.
  * A variant whose RK4 steps run in one launch (bit 14 of its options) is timed as
  * such; where a column form (bit 13) is the fastest, forward Euler and the residuals
  * run the variant whose forward-Euler update was (after dg_set_stage_variant, the
