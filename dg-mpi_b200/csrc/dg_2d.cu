@@ -659,6 +659,7 @@ struct dg_ctx2d {
     std::vector<double> coords;  // [nnode][2]
     std::vector<unsigned> e2n;   // [ne][4]
     std::vector<double> djac;    // [ne]
+    std::vector<double> host;    // a small state between its layouts (see to_device)
     std::string err;
 };
 
@@ -758,7 +759,7 @@ int to_device(dg_ctx2d* c, const double* h, double* d, double* scratch)
 {
     const int nb = c->nb;
     const long long n = 1LL * c->ne * d2::kNS * nb;
-    double t[kHostValues];
+    double* t = c->host.data();
     const bool on_host = nb > 1 && n <= kHostValues, on_device = nb > 1 && !on_host;
     for (long long e = 0; on_host && e < n; e += d2::kNS * nb)
         for (int b = 0; b < nb; ++b)
@@ -776,7 +777,7 @@ int to_host(dg_ctx2d* c, const double* d, double* h, double* scratch, bool check
 {
     const int nb = c->nb;
     const long long n = 1LL * c->ne * d2::kNS * nb;
-    double t[kHostValues];
+    double* t = c->host.data();
     if (n <= kHostValues) {
         DG2_CUDA(c, cudaMemcpyAsync(t, d, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     } else if (nb > 1) {
@@ -1030,6 +1031,7 @@ int dg2d_create(const dg_case_desc* cd, const dg_mesh2d_desc* md, dg_ctx2d** out
             ed.code = static_cast<int>(fL | fR << 2) | flip << 4 | static_cast<int>(oL) << 5;
             edges.push_back(ed);
         }
+        if (1LL * c->ne * d2::kNS * c->nb <= kHostValues) c->host.resize(static_cast<size_t>(c->ne) * d2::kNS * c->nb);
         c->t1 = dgh::make_tables(c->p);
         d2::Tab tab;
         if (!d2::make_tab(c->p, c->t1, tab)) return bail(DG_ERR_ARG, "edge trace tables");
